@@ -218,6 +218,19 @@ FarConst make_farconst(const OpParams& op, const RuleTable& R, const QuadSel& qs
     k.alpha32[c] = (float)op.alpha[c];
     k.beta32[c] = (float)op.beta[c];
   }
+  // Constant factors of the 3 x 4 rule pair (weights 1/3 and 25/48, 1/(4 pi); bgb_far_pair34.cuh): the
+  // RWG shapes' 1/(2A) cancel the areas (alpha part: 1/4, beta part: 1), the hats carry 1/5 (2/5 for
+  // the integral of G that the hypersingular's curls multiply)
+  {
+    const bool rwg = op.kind == BGB_OP_MAXWELL3D_SL || op.kind == BGB_OP_MAXWELL3D_DL;
+    const double w = 25.0 / 144.0 * BGB_INV_4PI_D;
+    const double fa = rwg ? (op.kind == BGB_OP_MAXWELL3D_DL ? -0.25 : 0.25) * w : 0.2 * w;
+    const double fb = rwg ? w : 0.4 * w;
+    for (int c = 0; c < 2; ++c) {
+      k.far_a[c] = fa * op.alpha[c];
+      k.far_b[c] = fb * op.beta[c];
+    }
+  }
   k.k_hi = (float)op.gamma[1];
   k.k_lo = (float)(op.gamma[1] - (double)k.k_hi);
   k.gre = (float)op.gamma[0];

@@ -93,8 +93,9 @@ int far_target_ctas_per_sm(int precision) {
 }
 
 int rec_stride(int precision, int q, int generic) {
-  const int Q = generic ? BGB_MAXQ : q;
-  return precision == BGB_PREC_MIXED ? farimpl::off32_size(Q) : 13 + 4 * Q;
+  (void)q;
+  if (!generic) return precision == BGB_PREC_MIXED ? kRec34F : kRec34D;
+  return precision == BGB_PREC_MIXED ? farimpl::off32_size(BGB_MAXQ) : 13 + 4 * BGB_MAXQ;
 }
 
 size_t far_smem_bytes(int precision, int op_kind, int qt, int qb, const TilePlan& p) {
@@ -120,19 +121,17 @@ int launch_far_pairs_diag(int precision, const FarConst& k, const void* rt, cons
 
 void launch_prepare_rec(int precision, int side, int q, const Geo64* g, int nt, const RuleTable& rules, int rule,
                         double wscale, void* out, cudaStream_t st) {
-  (void)side;
   if (nt <= 0) return;
   const int blocks = (nt + 127) / 128;
-  const bool gen = (q == BGB_MAXQ);
-  if (precision == BGB_PREC_MIXED) {
-    if (gen) k_prepare_rec32<BGB_MAXQ><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (float*)out);
-    else if (q == 3) k_prepare_rec32<3><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (float*)out);
-    else k_prepare_rec32<4><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (float*)out);
-  } else {
-    if (gen) k_prepare_rec64<BGB_MAXQ><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (double*)out);
-    else if (q == 3) k_prepare_rec64<3><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (double*)out);
-    else k_prepare_rec64<4><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (double*)out);
+  const bool mixed = precision == BGB_PREC_MIXED;
+  if (q != BGB_MAXQ) {  // 3 x 4 rule pair
+    const double scale = side ? -0.4 : 1.0, x2 = side ? 0.16 : 0.25;
+    if (mixed) k_prepare_rec34<float><<<blocks, 128, 0, st>>>(g, nt, scale, x2, (float*)out);
+    else k_prepare_rec34<double><<<blocks, 128, 0, st>>>(g, nt, scale, x2, (double*)out);
+    return;
   }
+  if (mixed) k_prepare_rec32<BGB_MAXQ><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (float*)out);
+  else k_prepare_rec64<BGB_MAXQ><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (double*)out);
 }
 
 }  // namespace bgb

@@ -87,6 +87,13 @@ __device__ __forceinline__ void tri_curls(const T* vo, T inv2a, T c[3][3]) {
     for (int k = 0; k < 3; ++k) c[i][k] = (vo[3 * ((i + 1) % 3) + k] - vo[3 * ((i + 2) % 3) + k]) * inv2a;
 }
 
+}  // namespace farimpl
+}  // namespace bgb
+#include "bgb_far_pair34.cuh"
+namespace bgb {
+namespace farimpl {
+
+// Records of the generic rules (the 3 x 4 rule pair has its own, bgb_far_pair34.cuh).
 // FP32 record of a triangle, in 16-byte groups read with 128-bit shared-memory loads:
 // [CH.xyz CL.x] [CL.yz - -] [x y z w] per quadrature point [VO (9) INV2A - -]; the stride is an odd
 // number of groups, so the records of different triangles start in different bank groups.
@@ -107,7 +114,7 @@ struct PMixed {
   using C = float2;
   static constexpr int kMinBlocks = 3;  // 3 CTAs of 256 threads per SM (<= 85 registers)
   template <int Q>
-  static constexpr int rec() { return Off32<Q>::SIZE; }
+  static constexpr int rec() { return Q <= 4 ? kRec34F : Off32<Q>::SIZE; }
   static __device__ __forceinline__ C mk(double a, double b) { return make_float2((float)a, (float)b); }
 };
 struct PFp64 {
@@ -115,7 +122,7 @@ struct PFp64 {
   using C = double2;
   static constexpr int kMinBlocks = 1;
   template <int Q>
-  static constexpr int rec() { return Off64<Q>::SIZE; }
+  static constexpr int rec() { return Q <= 4 ? kRec34D : Off64<Q>::SIZE; }
   static __device__ __forceinline__ C mk(double a, double b) { return make_double2(a, b); }
 };
 
@@ -195,17 +202,6 @@ __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float 
     // Helmholtz / EFIE: q = s.(2 D_hi + s) with s = a_I - y_J, a_I = D_lo + x_I, split as
     //   q = [c0 + a_I.(a_I + 2 D_hi)] + [y_J.(y_J - 2 D_hi)] - 2 a_I.y_J
     // (per test point, per trial point, per point pair): 5 operations per point pair.
-    // trial points of the pair in registers when the rule is small (shared-memory loads otherwise)
-    constexpr int QY = QB <= 4 ? QB : 1;
-    float MJ[QY];
-    if constexpr (QB <= 4) {
-#pragma unroll
-      for (int J = 0; J < QB; ++J) {
-        if (J >= qb) break;
-        const float4 y = b4[OB::px(J) / 4];
-        MJ[J] = fmaf(y.x, y.x - D2x, fmaf(y.y, y.y - D2y, y.z * (y.z - D2z)));
-      }
-    }
 #pragma unroll
     for (int I = 0; I < QT; ++I) {
       if (I >= qt) break;
@@ -227,9 +223,7 @@ __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float 
         if (J >= qb) break;
         const float4 YJ = b4[OB::px(J) / 4];
         const float yx = YJ.x, yy = YJ.y, yz = YJ.z;
-        float mj;
-        if constexpr (QB <= 4) mj = MJ[J];
-        else mj = fmaf(yx, yx - D2x, fmaf(yy, yy - D2y, yz * (yz - D2z)));
+        const float mj = fmaf(yx, yx - D2x, fmaf(yy, yy - D2y, yz * (yz - D2z)));
         const float dot = fmaf(ax, yx, fmaf(ay, yy, az * yz));
         const float q = fmaf(-2.f, dot, KI + mj);
         const float R2 = R0sq + q;
@@ -721,6 +715,10 @@ __device__ __forceinline__ FarScalars far_scalars(const FarConst& K) {
     S.alpha[c] = K.alpha[c];
     S.beta[c] = K.beta[c];
     S.gamma[c] = K.gamma[c];
+    S.far_a[c] = K.far_a[c];
+    S.far_b[c] = K.far_b[c];
+    S.far_a32[c] = (float)K.far_a[c];
+    S.far_b32[c] = (float)K.far_b[c];
   }
   return S;
 }
@@ -728,7 +726,11 @@ __device__ __forceinline__ FarScalars far_scalars(const FarConst& K) {
 template <class P, int OP, int QT, int QB>
 __device__ __forceinline__ void far_pair(const FarScalars& S, const FarConst& K, const typename P::R* a,
                                          const typename P::R* b, typename P::C L[9]) {
-  if constexpr (sizeof(typename P::R) == 4)
+  if constexpr (QT == 3 && QB == 4 && sizeof(typename P::R) == 4)
+    far_pair34_mixed<OP>(S, a, b, L);
+  else if constexpr (QT == 3 && QB == 4)
+    far_pair34_fp64<OP>(S, K.tay_s, K.tay_c, a, b, L);
+  else if constexpr (sizeof(typename P::R) == 4)
     far_pair_mixed<OP, QT, QB>(S, K.shpT, K.shpB, a, b, L);
   else
     far_pair_fp64<OP, QT, QB>(S, K.shpT64, K.shpB64, K.tay_s, K.tay_c, a, b, L);

@@ -86,6 +86,7 @@ struct FarConst {
   int phase_direct;            // k (r_test + r_trial) <= pi: the point-pair phase needs no reduction
   double alpha[2], beta[2], gamma[2];
   float alpha32[2], beta32[2];
+  double far_a[2], far_b[2];   // 3 x 4 rule pair: alpha and beta times its constant factors
   float k_hi, k_lo, gre;       // gamma_im as double-float, gamma_re
   float shpT[BGB_MAXQ][3], shpB[BGB_MAXQ][3];     // Lagrange hats at rule points
   double shpT64[BGB_MAXQ][3], shpB64[BGB_MAXQ][3];
@@ -103,6 +104,8 @@ struct FarScalars {
   float k_hi, k_lo, gre;
   float alpha32[2], beta32[2];
   double alpha[2], beta[2], gamma[2];
+  double far_a[2], far_b[2];
+  float far_a32[2], far_b32[2];
 };
 
 // Device-side plan of one tiled assembly (all arrays device pointers).
