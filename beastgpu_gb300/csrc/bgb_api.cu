@@ -219,13 +219,14 @@ FarConst make_farconst(const OpParams& op, const RuleTable& R, const QuadSel& qs
     k.beta32[c] = (float)op.beta[c];
   }
   // Constant factors of the 3 x 4 rule pair (weights 1/3 and 25/48, 1/(4 pi); bgb_far_pair34.cuh): the
-  // RWG shapes' 1/(2A) cancel the areas (alpha part: 1/4, beta part: 1), the hats carry 1/5 (2/5 for
-  // the integral of G that the hypersingular's curls multiply)
+  // RWG shapes' 1/(2A) cancel the areas (alpha part: 1/4, beta part: 1).  Hats: the trial records'
+  // areas carry them (kHatScale34), with 1/5 for the alpha part and 2/5 for the integral of G that the
+  // hypersingular's curls multiply
   {
     const bool rwg = op.kind == BGB_OP_MAXWELL3D_SL || op.kind == BGB_OP_MAXWELL3D_DL;
     const double w = 25.0 / 144.0 * BGB_INV_4PI_D;
-    const double fa = rwg ? (op.kind == BGB_OP_MAXWELL3D_DL ? -0.25 : 0.25) * w : 0.2 * w;
-    const double fb = rwg ? w : 0.4 * w;
+    const double fa = rwg ? (op.kind == BGB_OP_MAXWELL3D_DL ? -0.25 : 0.25) * w : 1.0;
+    const double fb = rwg ? w : 2.0;
     for (int c = 0; c < 2; ++c) {
       k.far_a[c] = fa * op.alpha[c];
       k.far_b[c] = fb * op.beta[c];
@@ -247,7 +248,9 @@ FarConst make_farconst(const OpParams& op, const RuleTable& R, const QuadSel& qs
   // plain FP64 kernel: series for exp(-i k (R - R0)) when |k (R - R0)| <= k (r_test + r_trial) is small
   k.tay_n = 0;
   if (test && trial && op.gamma[1] != 0.0) {
-    const double xmax = std::fabs(op.gamma[1]) * (et.max_centroid_radius + eb.max_centroid_radius);
+    // the 3 x 4 rule pair's points lie at 0.5 (test) and 0.4 (trial) of the vertex offsets
+    const bool r34 = k.qt == 3 && k.qb == 4;
+    const double xmax = std::fabs(op.gamma[1]) * ((r34 ? 0.5 : 1.0) * et.max_centroid_radius + (r34 ? 0.4 : 1.0) * eb.max_centroid_radius);
     if (xmax <= 2.0) {
       double fs = 1.0, fc = 1.0;  // (2j+1)!, (2j)!
       int n = 1;
@@ -258,10 +261,11 @@ FarConst make_farconst(const OpParams& op, const RuleTable& R, const QuadSel& qs
         for (int q = 2; q <= 2 * n + 1; ++q) ts *= xmax / q;
         if (tc <= 0x1p-55 && ts <= 0x1p-55) break;
       }
-      // measured on GB300: FP64 sincos of these small arguments costs about as much as 8 series terms
-      // (cube of the reference's benchmark, 4 terms: far stage 16.0 -> 14.4 s; icosphere level 5 at
-      // k = 8 pi, 11 terms: 1.13 -> 1.15 s), so the series is kept for short series only
-      if (n <= 6) {
+      // measured on GB300, other rules: FP64 sincos of these small arguments costs about as much as 8
+      // series terms, so only short series are used (cube of the reference's benchmark, 4 terms: far
+      // stage 16.0 -> 14.4 s; icosphere level 5 at k = 8 pi, 11 terms: 1.13 -> 1.15 s).  3 x 4 points: n
+      // terms cost 2 n + 1 operations per point pair against ~29 for sincos, and 4 for the rotation
+      if (n <= (r34 ? 11 : 6)) {
         k.tay_n = n;
         for (int j = 0; j < n; ++j) {
           if (j > 0) {
@@ -302,6 +306,10 @@ const TileCfg kTileCfgs[] = {
     {24, 24, 8},    // 16
     {60, 64, 5},    // 17: mixed, RWG (~50 test triangles x 5 = one round of 256 pairs per chunk)
     {32, 40, 5},    // 18: Lagrange
+    {48, 48, 5},    // 19: FP64 gather, RWG
+    {32, 32, 5},    // 20
+    {24, 24, 5},    // 21
+    {16, 16, 5},    // 22
 };
 // Preference order when the caller does not pin a tile: the first whose shared memory fits.
 // RWG: 60 x 64 tiles with 5-triangle chunks (C2 mixed far stage 28.6 ms against 31.1 ms for
@@ -322,6 +330,12 @@ const int kNumPrefLagrange = sizeof(kPrefLagrange) / sizeof(int);
 // from full chunks: d = 24 cube 48 x 48 x 4 1,537 ms, 40 x 40 x 4 1,629 ms, 32 x 40 x 5 1,693 ms.
 const int kPrefLagrangeFp64[] = {9, 15, 18, 6, 13, 5, 7};
 const int kNumPrefLagrangeFp64 = sizeof(kPrefLagrangeFp64) / sizeof(int);
+// Output tiles of the FP64 gather (single assemblies; widest first): every pair is computed once
+// whatever the tile, so their width only trades L2 reads at the rims against CTAs per SM.
+const int kPrefGather[] = {19, 20, 21, 22};
+const int kNumPrefGather = sizeof(kPrefGather) / sizeof(int);
+const int kPrefGatherLagrange[] = {18, 21, 22};
+const int kNumPrefGatherLagrange = sizeof(kPrefGatherLagrange) / sizeof(int);
 const int kNumTileCfgs = sizeof(kTileCfgs) / sizeof(kTileCfgs[0]);
 
 // ----------------------------------------------------------------------------------------
@@ -662,7 +676,8 @@ int bgb_destroy(bgb_handle* h) {
   DevBuf* bufs[] = {&h->verts_t, &h->tris_t, &h->verts_b, &h->tris_b, &h->geo_t, &h->geo_b, &h->bnd_t, &h->bnd_b, &h->bnd_c,
                     &h->rec_t, &h->rec_b, &h->cls_count, &h->cls_off, &h->ent_tau, &h->ent_sigma, &h->ent_cls, &h->ent_mask, &h->geodf_t, &h->geodf_b,
                     &h->sing_L, &h->err, &h->df_tab, &h->tplan_i, &h->tplan_l, &h->tplan_d, &h->tplan_f,
-                    &h->diag_a, &h->diag_b, &h->diag_c, &h->diag_d, &h->grp_tri, &h->grp_cnt, &h->grp_off, &h->grp_perm, &h->cls_hist};
+                    &h->diag_a, &h->diag_b, &h->diag_c, &h->diag_d, &h->grp_tri, &h->grp_cnt, &h->grp_off, &h->grp_perm, &h->cls_hist,
+                    &h->prow, &h->pcol[0], &h->pcol[1], &h->panel_L[0], &h->panel_L[1]};
   for (DevBuf* b : bufs) b->release();
   h->curve.release();
   for (int k = 0; k < bgb_handle::kSlots; ++k) {
@@ -920,14 +935,45 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   else if (test->refspace == BGB_REFSPACE_LAGRANGE_C0D1 && precision == BGB_PREC_MIXED)
     prefs.assign(kPrefLagrange, kPrefLagrange + kNumPrefLagrange);
   else if (test->refspace == BGB_REFSPACE_LAGRANGE_C0D1)
-    prefs.assign(kPrefLagrangeFp64, kPrefLagrangeFp64 + kNumPrefLagrangeFp64);
+    prefs.assign(kPrefGatherLagrange, kPrefGatherLagrange + kNumPrefGatherLagrange);
   else if (precision == BGB_PREC_MIXED) prefs.assign(kPrefMixed, kPrefMixed + kNumPrefMixed);
-  else prefs.assign(kPrefFp64, kPrefFp64 + kNumPrefFp64);
+  else prefs.assign(kPrefGather, kPrefGather + kNumPrefGather);
+  // The plain FP64 path computes the pairs of a panel once and gathers the tiles from them
+  // (bgb_gather64.cu); the mixed path computes them inside the tiles.
+  const bool two_phase = precision == BGB_PREC_FP64;
+  // small matrices: narrower tiles until there are two per SM
+  if (two_phase && !pinned_cfg) {
+    auto tiles = [&](int id) {
+      const TileCfg& c = kTileCfgs[id];
+      return ((nrows + c.FM - 1) / c.FM) * ((ncols + c.FN - 1) / c.FN);
+    };
+    while (prefs.size() > 1 && tiles(prefs[0]) < 2 * (int64_t)h->num_sms) prefs.erase(prefs.begin());
+  }
+  // Bytes of one panel's local matrices: up to 2 GiB (a few hundred trial triangles at 20,000 test
+  // triangles, whose rims add 4 - 8% pairs), within the caller's budget and a quarter of free memory.
+  int64_t panel_bytes = 0;
+  if (two_phase) {
+    panel_bytes = (int64_t)2 << 30;
+    if (h->cfg.hbm_budget_bytes > 0) panel_bytes = std::min(panel_bytes, h->cfg.hbm_budget_bytes);
+    const int64_t all = 144 * (int64_t)test->nt * trial->nt;
+    if ((int64_t)h->panel_L[0].cap < std::min(panel_bytes, all)) {
+      size_t freeb = 0, totalb = 0;
+      cudaMemGetInfo(&freeb, &totalb);
+      panel_bytes = std::min(panel_bytes, (int64_t)(freeb + h->panel_L[0].cap + h->panel_L[1].cap) / 4);
+    }
+  }
   int smem_max = 0;
   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+  struct Panel {
+    int bn0, bn1;    // trial tiles [bn0, bn1)
+    int col0, ncol;  // its trial triangles: pcols[col0 .. col0 + ncol)
+  };
   struct Plans {
     HostPlan test;                 // test side, all rows of the window
     std::vector<HostPlan> trial;   // trial side per output block
+    std::vector<int> rows;         // FP64: distinct test triangles, ascending (workspace rows)
+    std::vector<std::vector<Panel>> panels;  // FP64: per output block, runs of trial tiles
+    std::vector<std::vector<int>> pcols;     // and the distinct trial triangles of each, concatenated
     TileCfg tc{};
     int cfg_id = -1;
     size_t smem = 0;
@@ -995,6 +1041,36 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
         probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
         probe.nmax = std::max(probe.nmax, std::max(1, PL.trial[b].nmax));
       }
+      if (two_phase) {
+        // a tile pinned by the caller is one that the fused kernel could run; the gather's two chunk
+        // buffers then take as many triangles as fit (the result does not depend on the chunks)
+        int per_sm = 0;
+        if (pinned_cfg) {
+          smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
+          if (smem > (size_t)smem_max || far_persistent_occupancy(precision, K.op_kind, gen, smem, &per_sm) || per_sm < 1)
+            continue;
+        }
+        for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
+          if (sc != tc.SC) {
+            PL.trial.assign(nblocks, HostPlan());
+            over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
+            probe.SC = sc;
+            probe.gmax = probe.gsmax = 0;
+            for (int b = 0; b < nblocks; ++b) {
+              probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
+              probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
+            }
+          }
+          smem = gather64_smem_bytes(probe);
+          if (gather64_occupancy(smem, &per_sm) == 0 && per_sm >= 1) {
+            PL.cfg_id = id;
+            PL.tc = {tc.FM, tc.FN, sc};
+            PL.smem = smem;
+          }
+        }
+        if (PL.cfg_id >= 0) break;
+        continue;
+      }
       smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
       // Occupancy: when the widest test tile pushes shared memory past what the kernel's
       // CTAs per SM allow, cap the triangles per test tile at the largest count that fits.
@@ -1033,6 +1109,38 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
       snprintf(buf, sizeof buf, "no tile configuration fits in %d B of shared memory (last tried needs %zu B)",
                smem_max, smem);
       PL.err = buf;
+    } else if (two_phase) {
+      PL.rows = PL.test.tb_tris;
+      std::sort(PL.rows.begin(), PL.rows.end());
+      PL.rows.erase(std::unique(PL.rows.begin(), PL.rows.end()), PL.rows.end());
+      const int64_t cap = std::max<int64_t>(1, panel_bytes / (144 * std::max<int64_t>(1, (int64_t)PL.rows.size())));
+      PL.panels.assign(nblocks, {});
+      PL.pcols.assign(nblocks, {});
+      over_blocks([&](int b, int) {
+        const HostPlan& P = PL.trial[b];
+        std::vector<int>& cols = PL.pcols[b];
+        std::vector<int> stamp((size_t)std::max(1, trial->nt), -1);
+        const int nbb = (int)P.bb_off.size() - 1;
+        Panel cur{0, 0, 0, 0};
+        for (int n = 0; n < nbb; ++n) {
+          int fresh = 0;
+          for (int i = P.bb_off[n]; i < P.bb_off[n + 1]; ++i) fresh += stamp[(size_t)P.bb_tris[i]] != cur.bn0;
+          if (n > cur.bn0 && cur.ncol + fresh > cap) {
+            cur.bn1 = n;
+            PL.panels[b].push_back(cur);
+            cur = Panel{n, 0, (int)cols.size(), 0};
+          }
+          for (int i = P.bb_off[n]; i < P.bb_off[n + 1]; ++i) {
+            const int t = P.bb_tris[i];
+            if (stamp[(size_t)t] == cur.bn0) continue;
+            stamp[(size_t)t] = cur.bn0;
+            cols.push_back(t);
+            ++cur.ncol;
+          }
+        }
+        cur.bn1 = nbb;
+        if (nbb > 0) PL.panels[b].push_back(cur);
+      });
     }
     PL.ms = std::chrono::duration<double, std::milli>(clk::now() - t0).count();
   };
@@ -1223,7 +1331,8 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   std::vector<float> TF;
   auto cat_i = [&](std::vector<int>& dst, const std::vector<int>& v) { size_t o = dst.size(); dst.insert(dst.end(), v.begin(), v.end()); return o; };
   const size_t o_tb_off = cat_i(TI, PT.tb_off), o_tb_tris = cat_i(TI, PT.tb_tris), o_tb_fn = cat_i(TI, PT.tb_fn_off),
-               o_fs_off = cat_i(TI, PT.fs_off), o_fs_code = cat_i(TI, PT.fs_code);
+               o_fs_off = cat_i(TI, PT.fs_off), o_fs_code = cat_i(TI, PT.fs_code), o_rows = cat_i(TI, PL.rows);
+  const int nprow = (int)PL.rows.size();
   TF.reserve(PT.fs_coef.size());
   for (double v : PT.fs_coef) TF.push_back((float)v);
   if ((rc = h->tplan_i.ensure(sizeof(int) * std::max<size_t>(1, TI.size()))) ||
@@ -1236,9 +1345,23 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   if ((rc = upload_on(h->stream_up, h->tplan_i, TI)) || (rc = upload_on(h->stream_up, h->tplan_l, PT.rows)) ||
       (rc = upload_on(h->stream_up, h->tplan_d, PT.fs_coef)) || (rc = upload_on(h->stream_up, h->tplan_f, TF)))
     return rc;
+  if (two_phase) {
+    if ((rc = h->prow.ensure(sizeof(int) * std::max(1, test->nt)))) return rc;
+    if ((rc = launch_index_of(h->tplan_i.as<int>() + o_rows, nprow, h->prow.as<int>(), test->nt, h->stream_up))) return rc;
+    ++launches;
+    // one panel workspace per compute stream in use (sized to the largest panel)
+    for (int k = 0; k < std::min(2, nblocks); ++k) {
+      int64_t ncol = 1;
+      for (int b = k; b < nblocks; b += 2)
+        for (const Panel& q : PL.panels[b]) ncol = std::max<int64_t>(ncol, q.ncol);
+      if ((rc = h->pcol[k].ensure(sizeof(int) * std::max(1, trial->nt))) ||
+          (rc = h->panel_L[k].ensure(144 * (size_t)ncol * std::max(1, nprow))))
+        return rc;
+    }
+  }
   BGB_CUDA(cudaEventRecord(h->ev_up[bgb_handle::kSlots], h->stream_up));
   int per_sm = 0;
-  if ((rc = far_persistent_occupancy(precision, K.op_kind, gen, smem, &per_sm))) return rc;
+  if (!two_phase && (rc = far_persistent_occupancy(precision, K.op_kind, gen, smem, &per_sm))) return rc;
   const int ntb = (int)PT.tb_off.size() - 1;
 
   double ms_far = 0, ms_copy = 0;
@@ -1287,13 +1410,14 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     const size_t o_bb_off = cat_i(H.I, PB.bb_off), o_bb_tris = cat_i(H.I, PB.bb_tris), o_bb_fn = cat_i(H.I, PB.bb_fn_off),
                  o_bb_ch = cat_i(H.I, PB.bb_chunk_off), o_ch_grp = cat_i(H.I, PB.ch_grp_off),
                  o_grp_fn = cat_i(H.I, PB.grp_fn), o_grp_sup = cat_i(H.I, PB.grp_sup_off),
-                 o_gs_code = cat_i(H.I, PB.gs_code);
+                 o_gs_code = cat_i(H.I, PB.gs_code), o_pcols = two_phase ? cat_i(H.I, PL.pcols[b]) : 0;
     H.L.reserve(PB.cols.size());
     for (int64_t c : PB.cols) H.L.push_back(c - (host_out ? c0 : 0));  // staging columns start at c0
     H.F.reserve(PB.gs_coef.size());
     for (double v : PB.gs_coef) H.F.push_back((float)v);
     const size_t o_gs_coef = 0;
-    pairs_computed += (int64_t)PT.tb_tris.size() * (int64_t)PB.bb_tris.size();
+    pairs_computed += two_phase ? (int64_t)nprow * (int64_t)PL.pcols[b].size()
+                                : (int64_t)PT.tb_tris.size() * (int64_t)PB.bb_tris.size();
     const int nbb = (int)PB.bb_off.size() - 1;
     // tiles t = bn * ntb + bm (row block fastest: neighbouring rows of a column together); the
     // kernel derives (bm, bn) from t, no item list
@@ -1370,10 +1494,27 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     const int ctas = (int)std::min<int64_t>(ntiles, (int64_t)std::max(1, per_sm) * h->num_sms);
     if (grouped) BGB_CUDA(cudaStreamWaitEvent(cst, h->grp_ev[(size_t)b], 0));  // singular groups 0 .. b
     BGB_CUDA(cudaEventRecord(h->ev2[slot * 4 + 0], cst));
-    if ((rc2 = launch_far_persistent(precision, K.op_kind, gen, dK, dT, nullptr, (int)ntiles, dctr, smem,
-                                     std::max(1, ctas), h->abort_dev, cst)))
-      return rc2;
-    ++launches;
+    if (two_phase) {
+      const int w = b & 1;
+      for (const Panel& q : PL.panels[b]) {
+        const int* cols = bi + o_pcols + q.col0;
+        double2* ws = h->panel_L[w].as<double2>();
+        int* pcol = h->pcol[w].as<int>();
+        if ((rc2 = launch_index_of(cols, q.ncol, pcol, trial->nt, cst)) ||
+            (rc2 = launch_pair64(K.op_kind, gen, dK, T.rec_t, T.rec_b, ti + o_rows, nprow, cols, q.ncol, ws, h->abort_dev, cst)) ||
+            (rc2 = launch_place_special(h->ent_tau.as<int>(), h->ent_sigma.as<int>(), nsing, h->prow.as<int>(), pcol,
+                                        T.sing_L, q.ncol, ws, cst)) ||
+            (rc2 = launch_gather64(dT, ntb * (q.bn1 - q.bn0), q.bn0, h->prow.as<int>(), pcol, ws, q.ncol, smem,
+                                   h->abort_dev, cst)))
+          return rc2;
+        launches += 4;
+      }
+    } else {
+      if ((rc2 = launch_far_persistent(precision, K.op_kind, gen, dK, dT, nullptr, (int)ntiles, dctr, smem,
+                                       std::max(1, ctas), h->abort_dev, cst)))
+        return rc2;
+      ++launches;
+    }
     BGB_CUDA(cudaEventRecord(h->ev2[slot * 4 + 1], cst));
     pending[slot] = true;
     slot_block[slot] = b;

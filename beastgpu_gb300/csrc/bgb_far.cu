@@ -15,6 +15,12 @@ BGB_FAR_EXTERN(PFp64, 2)
 BGB_FAR_EXTERN(PFp64, 3)
 BGB_FAR_EXTERN(PFp64, 4)
 BGB_FAR_EXTERN(PFp64, 5)
+BGB_PAIR64_EXTERN(0)
+BGB_PAIR64_EXTERN(1)
+BGB_PAIR64_EXTERN(2)
+BGB_PAIR64_EXTERN(3)
+BGB_PAIR64_EXTERN(4)
+BGB_PAIR64_EXTERN(5)
 
 template <class P, int QT, int QB>
 static int dispatch_diag(const FarConst& K, const void* rt, const void* rb, const int* tau, const int* sigma,
@@ -86,6 +92,25 @@ int far_persistent_occupancy(int precision, int op_kind, int generic, size_t sme
                  : dispatch_occupancy<PFp64, 3, 4>(op_kind, smem_bytes, per_sm);
 }
 
+int launch_pair64(int op_kind, int generic, const FarConst* K, const void* rt, const void* rb, const int* rows, int nrows,
+                  const int* cols, int ncols, double2* ws, const volatile int* ab, cudaStream_t st) {
+#define BGB_PAIR64_CASE(OP)                                                                            \
+  case OP:                                                                                             \
+    return generic ? launch_pair64_t<OP, BGB_MAXQ, BGB_MAXQ>(K, rt, rb, rows, nrows, cols, ncols, ws, ab, st) \
+                   : launch_pair64_t<OP, 3, 4>(K, rt, rb, rows, nrows, cols, ncols, ws, ab, st)
+  switch (op_kind) {
+    BGB_PAIR64_CASE(BGB_OP_HELMHOLTZ3D_SL);
+    BGB_PAIR64_CASE(BGB_OP_MAXWELL3D_SL);
+    BGB_PAIR64_CASE(BGB_OP_MAXWELL3D_DL);
+    BGB_PAIR64_CASE(BGB_OP_HELMHOLTZ3D_DL);
+    BGB_PAIR64_CASE(BGB_OP_HELMHOLTZ3D_DLT);
+    BGB_PAIR64_CASE(BGB_OP_HELMHOLTZ3D_HS);
+  }
+#undef BGB_PAIR64_CASE
+  set_error("unknown operator kind %d", op_kind);
+  return BGB_ERR_INVALID;
+}
+
 int far_generic_q(int qt, int qb) { return !(qt == 3 && qb == 4); }
 
 int far_target_ctas_per_sm(int precision) {
@@ -125,9 +150,9 @@ void launch_prepare_rec(int precision, int side, int q, const Geo64* g, int nt, 
   const int blocks = (nt + 127) / 128;
   const bool mixed = precision == BGB_PREC_MIXED;
   if (q != BGB_MAXQ) {  // 3 x 4 rule pair
-    const double scale = side ? -0.4 : 1.0, x2 = side ? 0.16 : 0.25;
-    if (mixed) k_prepare_rec34<float><<<blocks, 128, 0, st>>>(g, nt, scale, x2, (float*)out);
-    else k_prepare_rec34<double><<<blocks, 128, 0, st>>>(g, nt, scale, x2, (double*)out);
+    const double scale = side ? -0.4 : 1.0, x2 = side ? 0.16 : 0.25, wa = side ? kHatScale34 : 1.0;
+    if (mixed) k_prepare_rec34<float><<<blocks, 128, 0, st>>>(g, nt, scale, x2, wa, (float*)out);
+    else k_prepare_rec34<double><<<blocks, 128, 0, st>>>(g, nt, scale, x2, wa, (double*)out);
     return;
   }
   if (mixed) k_prepare_rec32<BGB_MAXQ><<<blocks, 128, 0, st>>>(g, nt, rules, rule, wscale, (float*)out);

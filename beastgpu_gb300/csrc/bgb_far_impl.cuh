@@ -1127,6 +1127,66 @@ __global__ void __launch_bounds__(kThreads, P::kMinBlocks) k_far_persistent(cons
 }
 
 // ----------------------------------------------------------------------------------------
+// Plain FP64: the local matrices of a panel, every pair once (the gather is in bgb_gather64.cu).
+//
+// One pair per thread, 16 test x 16 trial triangles per CTA, records in shared memory; the matrix of
+// (row, column) goes to ws[(row * ncols + column) * 9].  Bound by the FP64 pipe: two CTAs per SM
+// (at most 128 registers) keep it fed through the latencies of its 2-lanes-per-clock instructions.
+// ----------------------------------------------------------------------------------------
+constexpr int kPairSide = 16;
+template <int OP, int QT, int QB>
+__global__ void __launch_bounds__(kPairSide * kPairSide, 2) k_pair64(const FarConst* __restrict__ Kp,
+                                                                     const double* __restrict__ rec_t,
+                                                                     const double* __restrict__ rec_b,
+                                                                     const int* __restrict__ rows, int nrows,
+                                                                     const int* __restrict__ cols, int ncols,
+                                                                     double2* __restrict__ ws,
+                                                                     const volatile int* abort_flag) {
+  constexpr int RT = PFp64::rec<QT>(), RB = PFp64::rec<QB>();
+  __shared__ FarConst K;
+  __shared__ double sT[kPairSide * RT], sB[kPairSide * RB];
+  __shared__ int stop;
+  const int tid = threadIdx.x;
+  const int r0 = blockIdx.y * kPairSide, c0 = blockIdx.x * kPairSide;
+  const int nr = min(kPairSide, nrows - r0), nc = min(kPairSide, ncols - c0);
+  for (int i = tid; i < (int)(sizeof(FarConst) / 4); i += kPairSide * kPairSide) ((int*)&K)[i] = ((const int*)Kp)[i];
+  for (int i = tid; i < nr * RT; i += kPairSide * kPairSide) {
+    const int r = i / RT;
+    sT[i] = rec_t[(int64_t)rows[r0 + r] * RT + (i - r * RT)];
+  }
+  for (int i = tid; i < nc * RB; i += kPairSide * kPairSide) {
+    const int r = i / RB;
+    sB[i] = rec_b[(int64_t)cols[c0 + r] * RB + (i - r * RB)];
+  }
+  if (tid == 0) stop = abort_flag && *abort_flag;
+  __syncthreads();
+  if (stop) return;
+  const int ti = tid / kPairSide, si = tid - ti * kPairSide;
+  if (ti >= nr || si >= nc) return;
+  double2 L[9];
+  far_pair<PFp64, OP, QT, QB>(far_scalars(K), K, sT + ti * RT, sB + si * RB, L);
+  double2* o = ws + ((int64_t)(r0 + ti) * ncols + c0 + si) * 9;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) o[k] = L[k];
+}
+
+template <int OP, int QT, int QB>
+int launch_pair64_t(const FarConst* K, const void* rt, const void* rb, const int* rows, int nrows, const int* cols,
+                    int ncols, double2* ws, const volatile int* abort_flag, cudaStream_t st) {
+  if (nrows <= 0 || ncols <= 0) return 0;
+  // rows along y in runs of at most 65535 blocks (a grid's limit)
+  const int step = 65535 * kPairSide;
+  for (int r = 0; r < nrows; r += step) {
+    const int n = std::min(step, nrows - r);
+    const dim3 grid((ncols + kPairSide - 1) / kPairSide, (n + kPairSide - 1) / kPairSide);
+    k_pair64<OP, QT, QB><<<grid, kPairSide * kPairSide, 0, st>>>(K, (const double*)rt, (const double*)rb, rows + r, n,
+                                                                 cols, ncols, ws + (int64_t)r * ncols * 9, abort_flag);
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : cuda_fail(e, "k_pair64 launch");
+}
+
+// ----------------------------------------------------------------------------------------
 // Records
 // ----------------------------------------------------------------------------------------
 template <int Q>
@@ -1276,6 +1336,13 @@ int launch_diag_t(const FarConst& K, const void* rt, const void* rb, const int* 
                                                                      const volatile int*, cudaStream_t);       \
   extern template int occupancy_t<P, OP, 3, 4>(size_t, int*);                                                 \
   extern template int occupancy_t<P, OP, BGB_MAXQ, BGB_MAXQ>(size_t, int*);
+
+#define BGB_PAIR64_EXTERN(OP)                                                                                       \
+  extern template int launch_pair64_t<OP, 3, 4>(const FarConst*, const void*, const void*, const int*, int,        \
+                                                const int*, int, double2*, const volatile int*, cudaStream_t);    \
+  extern template int launch_pair64_t<OP, BGB_MAXQ, BGB_MAXQ>(const FarConst*, const void*, const void*, const int*, \
+                                                              int, const int*, int, double2*, const volatile int*,   \
+                                                              cudaStream_t);
 
 }  // namespace farimpl
 }  // namespace bgb

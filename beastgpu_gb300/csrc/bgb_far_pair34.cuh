@@ -31,6 +31,9 @@ namespace farimpl {
 // on the trial side (an odd number of groups: the records of different triangles start in different banks).
 // FP64 record: centroid, the three offsets, |x_i|^2, area, 1/(2A).
 constexpr int kRec34F = 20, kRec34D = 17;
+// Factor of the trial records' areas: the hats' constants (rule weights, 1/(4 pi), 1/5), in FP64 before
+// the FP32 records are rounded.
+constexpr double kHatScale34 = 0.2 * 25.0 / 144.0 * BGB_INV_4PI_D;
 
 __device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ float ml(float a, float b) { return a * b; }
@@ -480,9 +483,11 @@ __device__ __forceinline__ void far_pair34_fp64(const FarScalars& K, const doubl
 }
 
 // ---- records --------------------------------------------------------------------------------------
-// scale: factor of the vertex offsets (1 test, -0.4 trial); x2: |x_i|^2 = x2 |V_i|^2 (1/4, 0.16).
+// scale: factor of the vertex offsets (1 test, -0.4 trial); x2: |x_i|^2 = x2 |V_i|^2 (1/4, 0.16); warea: factor
+// of the area.
 template <class T>
-__global__ void k_prepare_rec34(const Geo64* __restrict__ g, int nt, double scale, double x2, T* __restrict__ out) {
+__global__ void k_prepare_rec34(const Geo64* __restrict__ g, int nt, double scale, double x2, double warea,
+                                T* __restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const Geo64& S = g[t];
@@ -496,7 +501,7 @@ __global__ void k_prepare_rec34(const Geo64* __restrict__ g, int nt, double scal
     r[k] = (T)c[k];
     if (f32) r[4 + k] = (T)(c[k] - (double)(T)c[k]);
   }
-  r[f32 ? 3 : 15] = (T)S.area;
+  r[f32 ? 3 : 15] = (T)(warea * S.area);
   r[f32 ? 7 : 16] = (T)inv2a;
   for (int i = 0; i < 3; ++i) {
     double s = 0.0;

@@ -73,6 +73,9 @@ struct bgb_handle {
   bgb::DevBuf cls_count, cls_off, ent_tau, ent_sigma, ent_cls, ent_mask, sing_L, err, geodf_t, geodf_b;
   bgb::DevBuf grp_tri, grp_cnt, grp_off, grp_perm;  // singular entries grouped by output block
   bgb::DevBuf cls_hist;                             // entries per class (statistics)
+  // plain FP64 far stage: local matrices of a panel (one per compute stream), workspace row of each test
+  // triangle, column of each trial triangle
+  bgb::DevBuf panel_L[2], prow, pcol[2];
   static constexpr int kSlots = 3;  // output-block slots in flight (staging, plan tables, events)
   bgb::DevBuf plan_i[kSlots], plan_l[kSlots], plan_d[kSlots], plan_f[kSlots], far_const[kSlots], df_tab;
   bgb::DevBuf tplan_i, tplan_l, tplan_d, tplan_f;  // test-side tile tables (shared by all output blocks)
@@ -119,6 +122,10 @@ extern const int kPrefFp64[];
 extern const int kNumPrefFp64;
 extern const int kPrefLagrange[];
 extern const int kNumPrefLagrange;
+extern const int kPrefGather[];
+extern const int kNumPrefGather;
+extern const int kPrefGatherLagrange[];
+extern const int kNumPrefGatherLagrange;
 extern const int kPrefLagrangeFp64[];
 extern const int kNumPrefLagrangeFp64;
 

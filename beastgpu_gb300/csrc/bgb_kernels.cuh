@@ -166,6 +166,20 @@ void launch_prepare_rec(int precision, int side, int q, const Geo64* g, int nt, 
 int far_generic_q(int qt, int qb);  // 1 when the (qt, qb) pair uses the generic instance
 int rec_stride(int precision, int q, int generic);
 
+// Plain FP64 far stage of a single assembly: the local matrices of a panel rows x cols (triangle lists,
+// device), then the output tiles [bn0 * n_tblocks, + ntiles) from them.
+int launch_pair64(int op_kind, int generic, const FarConst* K, const void* rec_t, const void* rec_b, const int* rows,
+                  int nrows, const int* cols, int ncols, double2* ws, const volatile int* abort_flag, cudaStream_t st);
+// ---- bgb_gather64.cu -------------------------------------------------------------------
+// index[list[i]] = i, -1 elsewhere.
+int launch_index_of(const int* list, int n, int* index, int nindex, cudaStream_t st);
+int launch_place_special(const int* tau, const int* sigma, int64_t n, const int* prow, const int* pcol, const double2* L,
+                         int ncols, double2* ws, cudaStream_t st);
+size_t gather64_smem_bytes(const TilePlan& p);
+int gather64_occupancy(size_t smem_bytes, int* per_sm);  // 0 CTAs when it does not fit
+int launch_gather64(const TilePlan* plan, int ntiles, int bn0, const int* prow, const int* pcol, const double2* ws,
+                    int ncols, size_t smem_bytes, const volatile int* abort_flag, cudaStream_t st);
+
 // Diagnostic: far-pair local matrices of explicit pairs with the tile kernels' pair code.
 int launch_far_pairs_diag(int precision, const FarConst& k, const void* rec_t, const void* rec_b, const int* tau,
                           const int* sigma, int64_t n, double2* out, cudaStream_t st);
