@@ -545,7 +545,7 @@ static int check_abort(bgb_handle* h) {
 
 // Classification of all (test, trial) triangle pairs into the non-far CSR; returns the count.
 static int classify_all(bgb_handle* h, const bgb_space* test, const bgb_space* trial, const Geo64* gt,
-                        const Geo64* gb, double k2, int64_t* total) {
+                        const Geo64* gb, double k2, int64_t* total, bool* inexact) {
   int rc;
   const int nt = test->nt, nb = trial->nt;
   if ((rc = h->bnd_t.ensure(sizeof(float4) * std::max(1, nt)))) return rc;
@@ -563,11 +563,12 @@ static int classify_all(bgb_handle* h, const bgb_space* test, const bgb_space* t
                   h->bnd_c.as<float4>());
   launch_scan(h->cls_count.as<int>(), nt, h->cls_off.as<int64_t>(), h->stream);
   int64_t tot = 0;
-  int herr = 0;
+  int herr[2] = {0, 0};
   BGB_CUDA(cudaMemcpyAsync(&tot, h->cls_off.as<int64_t>() + nt, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
-  BGB_CUDA(cudaMemcpyAsync(&herr, h->err.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  BGB_CUDA(cudaMemcpyAsync(herr, h->err.p, sizeof(herr), cudaMemcpyDeviceToHost, h->stream));
   BGB_CUDA(cudaStreamSynchronize(h->stream));
-  if (herr) {
+  *inexact = herr[1] != 0;
+  if (herr[0]) {
     set_error("degenerate geometry: a triangle pair shares more than three vertices");
     return BGB_ERR_INVALID;
   }
@@ -677,7 +678,7 @@ int bgb_destroy(bgb_handle* h) {
                     &h->rec_t, &h->rec_b, &h->cls_count, &h->cls_off, &h->ent_tau, &h->ent_sigma, &h->ent_cls, &h->ent_mask, &h->geodf_t, &h->geodf_b,
                     &h->sing_L, &h->err, &h->df_tab, &h->tplan_i, &h->tplan_l, &h->tplan_d, &h->tplan_f,
                     &h->diag_a, &h->diag_b, &h->diag_c, &h->diag_d, &h->grp_tri, &h->grp_cnt, &h->grp_off, &h->grp_perm, &h->cls_hist,
-                    &h->prow, &h->pcol[0], &h->pcol[1], &h->panel_L[0], &h->panel_L[1]};
+                    &h->ss_pts, &h->near_list, &h->prow, &h->pcol[0], &h->pcol[1], &h->panel_L[0], &h->panel_L[1]};
   for (DevBuf* b : bufs) b->release();
   h->curve.release();
   for (int k = 0; k < bgb_handle::kSlots; ++k) {
@@ -1208,7 +1209,8 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   auto host_ms = [&]() { return std::chrono::duration<double, std::milli>(clk::now() - t_start).count(); };
   double hm[6] = {host_ms(), 0, 0, 0, 0, 0};  // host marks for BGB_TRACE
   int64_t nsing = 0;
-  if ((rc = classify_all(h, test, trial, gt, gb, opp.k2, &nsing))) return rc;
+  bool inexact = false;  // some coincident vertices are not bit-equal
+  if ((rc = classify_all(h, test, trial, gt, gb, opp.k2, &nsing, &inexact))) return rc;
   hm[1] = host_ms();
   launches += 6;  // 2 bounds, 2 classify passes, scan (+1 singular below)
   if (stats) {  // entries per class, published to the mailbox (read after the final synchronisation)
@@ -1220,6 +1222,7 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   cudaEventRecord(h->ev[1], h->stream);
   // 2. singular / near pairs: FP64 kernel (plain path), double-float kernel (mixed path)
   if ((rc = h->sing_L.ensure(sizeof(double2) * 9 * std::max<int64_t>(1, nsing)))) return rc;
+  if ((rc = h->near_list.ensure(sizeof(int) * (size_t)(nsing + 1)))) return rc;
   const bool use_df = precision == BGB_PREC_MIXED && df_singular_ok(opp, ext_t.max_edge, ext_b.max_edge);
   std::vector<float> df_host;  // uploaded asynchronously: lives until the end of the call
   DfTables M{};
@@ -1235,13 +1238,20 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
       // near pairs (singularity extraction: logarithms and arctangents) in FP64
       launch_singular(opp, qsel, R, test->refspace, trial->refspace, gt, gb, h->ent_tau.as<int>(),
                       h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev,
-                      h->num_sms, st, true, perm, range);
+                      h->num_sms, st, true, perm, range, nullptr, h->near_list.as<int>());
       return 2;
     }
+    launch_ss64(opp.kind, opp, nullptr, nullptr, h->ss_tab, h->ss_pts.as<double>(), gt, gb, h->ent_tau.as<int>(),
+                h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), h->ent_mask.as<int16_t>(), nsing,
+                h->sing_L.as<double2>(), h->abort_dev, h->num_sms, st, perm, range);
     launch_singular(opp, qsel, R, test->refspace, trial->refspace, gt, gb, h->ent_tau.as<int>(), h->ent_sigma.as<int>(),
-                    h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev, h->num_sms, st, false, perm,
-                    range);
-    return 1;
+                    h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev, h->num_sms, st, true, perm,
+                    range, nullptr, h->near_list.as<int>());
+    if (inexact)
+      launch_singular(opp, qsel, R, test->refspace, trial->refspace, gt, gb, h->ent_tau.as<int>(),
+                      h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev,
+                      h->num_sms, st, false, perm, range, h->ent_mask.as<int16_t>());
+    return inexact ? 3 : 2;
   };
   // A host output in several blocks integrates its singular entries in groups on a stream of their
   // own: group b holds the entries whose trial triangle first appears in block b, the groups run in
@@ -1284,6 +1294,20 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     dgt = h->geodf_t.as<GeoDf>();
     dgb = same ? dgt : h->geodf_b.as<GeoDf>();
     launches += 1 + (same ? 0 : 1);
+  }
+  if (!use_df) {  // the ray tables of the FP64 kernel depend on the rule orders only
+    bool have = h->ss_pts.p != nullptr;
+    for (int c = 1; c <= 3; ++c) have = have && h->ss_tab.n[c] == qsel.ss[c];
+    if (!have) {
+      std::vector<double> pts;
+      build_ss_tables(qsel, pts, h->ss_tab);
+      if ((rc = h->ss_pts.ensure(sizeof(double) * pts.size()))) {
+        h->ss_tab = SsTab64{};
+        return rc;
+      }
+      BGB_CUDA(cudaMemcpyAsync(h->ss_pts.p, pts.data(), sizeof(double) * pts.size(), cudaMemcpyHostToDevice, h->stream));
+      BGB_CUDA(cudaStreamSynchronize(h->stream));
+    }
   }
   struct SyncOnExit {  // singular groups still in flight when the call returns early
     cudaStream_t st;

@@ -27,6 +27,9 @@ struct bgb_batch {
   bgb::DevBuf cls_count, cls_off, ent_tau, ent_sigma, ent_cls, ent_mask, sing_L, err, geodf_t, geodf_b, opdf;
   bgb::DevBuf plan_i, plan_l, plan_d, plan_f, stage, df_tab;
   bool use_df = false;
+  bgb::SsTab64 ss_tab{};  // FP64 Sauter-Schwab tables (use_df false)
+  bgb::DevBuf ss_pts, near_list;
+  bool inexact = false;   // some coincident vertices are not bit-equal
   bgb::DfTables dfm{};
   int nt_t = 0, nt_b = 0, nv_t = 0, nv_b = 0, nitems = 0;
   bool shared_trial = false;
@@ -48,7 +51,7 @@ struct bgb_batch {
     bgb::DevBuf* bufs[] = {&verts_t, &verts_b, &tris_t, &tris_b, &geo_t, &geo_b, &bnd_t, &bnd_b, &bnd_c, &rec_t, &rec_b,
                            &tri_problem, &prob_trial, &prob_k2, &ops, &Ks, &plans, &items, &counter, &cls_count,
                            &cls_off, &ent_tau, &ent_sigma, &ent_cls, &ent_mask, &sing_L, &err, &geodf_t, &geodf_b, &opdf, &plan_i, &plan_l, &plan_d,
-                           &plan_f, &stage, &df_tab};
+                           &plan_f, &stage, &df_tab, &ss_pts, &near_list};
     for (auto* b : bufs) b->release();
   }
 };
@@ -106,11 +109,19 @@ int enqueue_device_work(bgb_batch* B, cudaStream_t st, bool far_only) {
                          B->ent_mask.as<int16_t>(), B->nsing, B->sing_L.as<double2>(), h->abort_dev, h->num_sms, st);
       launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t, B->ent_tau.as<int>(),
                               B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing, B->sing_L.as<double2>(),
-                              h->abort_dev, h->num_sms, st, true);  // near pairs in FP64
-    } else
+                              h->abort_dev, h->num_sms, st, true, nullptr, B->near_list.as<int>());  // near pairs in FP64
+    } else {
+      launch_ss64(B->op_kind, OpParams{}, B->ops.as<OpParams>(), tp_t, B->ss_tab, B->ss_pts.as<double>(), gt, gb,
+                  B->ent_tau.as<int>(), B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->ent_mask.as<int16_t>(),
+                  B->nsing, B->sing_L.as<double2>(), h->abort_dev, h->num_sms, st);
       launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t, B->ent_tau.as<int>(),
                               B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing, B->sing_L.as<double2>(),
-                              h->abort_dev, h->num_sms, st);
+                              h->abort_dev, h->num_sms, st, true, nullptr, B->near_list.as<int>());
+      if (B->inexact)
+        launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t,
+                                B->ent_tau.as<int>(), B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing,
+                                B->sing_L.as<double2>(), h->abort_dev, h->num_sms, st, false, B->ent_mask.as<int16_t>());
+    }
     const int qt = B->rules.npoints[B->qsel.far_t], qb = B->rules.npoints[B->qsel.far_b];
     launch_prepare_rec(B->precision, 0, B->generic ? BGB_MAXQ : qt, gt, B->nt_t, B->rules, B->qsel.far_t, 1.0,
                        B->rec_t.p, st);
@@ -340,6 +351,12 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
       BGB_CUDA(cudaStreamSynchronize(st));
     }
   }
+  if (!B->use_df) {
+    std::vector<double> pts;
+    build_ss_tables(B->qsel, pts, B->ss_tab);
+    if ((rc = put(st, B->ss_pts, pts))) return fail(rc);
+    BGB_CUDA(cudaStreamSynchronize(st));
+  }
   B->nt_t = (int)(tt.size() / 3);
   B->nv_t = (int)(vt.size() / 3);
   B->nt_b = B->shared_trial ? B->nt_t : (int)(tb.size() / 3);
@@ -387,17 +404,19 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
                           B->prob_trial.as<int2>(), B->prob_k2.as<double>(), B->cls_count.as<int>(), nullptr, nullptr,
                           nullptr, nullptr, B->err.as<int>(), h->num_sms, st, nullptr, B->bnd_c.as<float4>());
   launch_scan(B->cls_count.as<int>(), B->nt_t, B->cls_off.as<int64_t>(), st);
-  int herr = 0;
+  int herr[2] = {0, 0};
   int64_t tot = 0;
   BGB_CUDA(cudaMemcpyAsync(&tot, B->cls_off.as<int64_t>() + B->nt_t, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  BGB_CUDA(cudaMemcpyAsync(&herr, B->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  BGB_CUDA(cudaMemcpyAsync(herr, B->err.p, sizeof(herr), cudaMemcpyDeviceToHost, st));
   BGB_CUDA(cudaStreamSynchronize(st));
-  if (herr) { set_error("degenerate geometry: a triangle pair shares more than three vertices"); return fail(BGB_ERR_INVALID); }
+  B->inexact = herr[1] != 0;
+  if (herr[0]) { set_error("degenerate geometry: a triangle pair shares more than three vertices"); return fail(BGB_ERR_INVALID); }
   B->nsing = tot;
   if ((rc = B->ent_tau.ensure(sizeof(int) * std::max<int64_t>(1, tot))) ||
       (rc = B->ent_sigma.ensure(sizeof(int) * std::max<int64_t>(1, tot))) ||
       (rc = B->ent_cls.ensure(std::max<int64_t>(1, tot))) ||
       (rc = B->ent_mask.ensure(sizeof(int16_t) * std::max<int64_t>(1, tot))) ||
+      (rc = B->near_list.ensure(sizeof(int) * (size_t)(tot + 1))) ||
       (B->use_df && (rc = B->geodf_t.ensure(sizeof(GeoDf) * std::max(1, B->nt_t)))) ||
       (B->use_df && !B->shared_trial && (rc = B->geodf_b.ensure(sizeof(GeoDf) * std::max(1, B->nt_b)))) ||
       (rc = B->sing_L.ensure(sizeof(double2) * 9 * std::max<int64_t>(1, tot))))

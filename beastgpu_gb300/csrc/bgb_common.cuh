@@ -17,6 +17,11 @@
 #define BGB_MAX_SS 16      // largest Gauss-Legendre order for Sauter-Schwab
 #define BGB_TAYLOR_MAX 16  // series terms of the plain FP64 far kernel's point-pair phase
 
+// Vertex-match mask of a pair: bit 3 i + j when test vertex i and trial vertex j coincide; this bit when
+// some coincident pair is not bit-equal (within the tolerance only).
+#define BGB_MASK_INEXACT 512
+#define BGB_SS_SERIES 14   // longest cosine / sine series of the FP64 Sauter-Schwab kernel
+
 namespace bgb {
 
 // ----------------------------------------------------------------------------------------

@@ -26,12 +26,15 @@ void launch_group_entries(const int* sigma, int64_t n, const int* tri_group, int
                           int* perm, int num_sms, cudaStream_t st);
 void launch_classify_dense(const Geo64* tg, const Geo64* bg, int t0, int t1, int s0, int s1, double k2, int8_t* out,
                            int* err, cudaStream_t st);
-// near_only: integrate only the near pairs of the list (the mixed path's double-float kernel skips them).
+// near_only: integrate only the near pairs of the list (the Sauter-Schwab kernels skip them).  inexact_of (the
+// entries' masks): only the pairs whose coincident vertices are not bit-equal.  near_list: scratch of near_only,
+// n + 1 ints.
 // perm (device, optional): integrate only the entries perm[range[0] .. range[1]) (range: device int64[2]).
 void launch_singular(const OpParams& op, const QuadSel& qs, const RuleTable& rules, int rsA, int rsB, const Geo64* tg,
                      const Geo64* bg, const int* et, const int* es, const int8_t* ec, int64_t n, double2* out,
                      const volatile int* abort_flag, int num_sms, cudaStream_t st, bool near_only = false,
-                     const int* perm = nullptr, const int64_t* range = nullptr);
+                     const int* perm = nullptr, const int64_t* range = nullptr, const int16_t* inexact_of = nullptr,
+                     int* near_list = nullptr);
 void launch_local_diag64(const OpParams& op, const QuadSel& qs, const RuleTable& rules, int rsA, int rsB,
                          const Geo64* tg, const Geo64* bg, const int* tau, const int* sigma, int64_t n, int force,
                          double2* out, int8_t* cls, int* err, int num_sms, cudaStream_t st, int16_t* mask = nullptr);
@@ -45,7 +48,24 @@ void launch_classify_batched(bool fill, const float4* tb, const float4* bb, cons
 void launch_singular_batched(int op_kind, const OpParams* ops, const QuadSel& qs, const RuleTable& rules,
                              const Geo64* tg, const Geo64* bg, const int* tri_problem, const int* et, const int* es,
                              const int8_t* ec, int64_t n, double2* out, const volatile int* abort_flag, int num_sms,
-                             cudaStream_t st, bool near_only = false);
+                             cudaStream_t st, bool near_only = false, const int16_t* inexact_of = nullptr,
+                             int* near_list = nullptr);
+
+// ---- bgb_ss64.cu -----------------------------------------------------------------------
+// Tables of the FP64 Sauter-Schwab kernel: ray coordinates and weights of every (eta, region) point
+// (device, five arrays of cnt per class at off), the xi rule, and the series of T_m, m = -1 .. 2 (signed
+// S_(m+n) / n!).
+struct SsTab64 {
+  int off[4], cnt[4], n[4];
+  double gx[4][BGB_MAX_SS], gw[4][BGB_MAX_SS];
+  double ser[4][4][2 * BGB_SS_SERIES];
+};
+void build_ss_tables(const QuadSel& qs, std::vector<double>& pts, SsTab64& M);
+// Singular pairs of the list (near pairs and inexact matches are skipped).  ops / tri_problem non-NULL: batched.
+void launch_ss64(int op_kind, const OpParams& op, const OpParams* ops, const int* tri_problem, const SsTab64& M,
+                 const double* pts, const Geo64* tg, const Geo64* bg, const int* et, const int* es, const int8_t* ec,
+                 const int16_t* emask, int64_t n, double2* out, const volatile int* abort_flag, int num_sms, cudaStream_t st,
+                 const int* perm = nullptr, const int64_t* range = nullptr);
 
 // ---- bgb_singular_df.cu ----------------------------------------------------------------
 // Host-built tables of the double-float singular kernel (one float buffer): Sauter-Schwab

@@ -6,7 +6,8 @@
 //                     test rejects far pairs, the exact FP64 predicate (BEAST quadrule,
 //                     doubleQuadRuleMainCase.jl:187-200) decides the rest; non-far pairs are
 //                     compacted in trial order (ballot/popc), so the list is deterministic.
-//  k_singular<OP>     one warp per non-far pair: Sauter-Schwab CF/CE/CV (SauterSchwab.jl:212-297)
+//  k_singular<OP>     near pairs, and singular pairs outside the ray kernel (bgb_ss64.cu: bit-equal
+//                     shared vertices).  One warp per non-far pair: Sauter-Schwab CF/CE/CV (SauterSchwab.jl:212-297)
 //                     or the near-pair rule with singularity extraction (BEAST's WiltonSERule:
 //                     closed-form inner integrals of 1/R - gamma + gamma^2 R / 2, the smooth rest
 //                     by the near double rule), FP64.  Each point adds a few operator moments
@@ -15,6 +16,8 @@
 //  k_classify_dense   diagnostic: exact class of every pair of a block.
 #include "bgb_kernels.cuh"
 #include "bgb_ss.cuh"
+
+#include <algorithm>
 
 namespace bgb {
 
@@ -99,12 +102,12 @@ __global__ void k_chunk_bounds(const float4* __restrict__ b, int nb, float4* __r
 // Exact FP64 predicate (doubleQuadRuleMainCase.jl:187-200; codes quadrule_determine.jl:76).
 // Rounded like the Julia code: no contraction, IEEE sqrt and division.  *mask (optional)
 // receives the coincident vertex pairs, bit u1 * 3 + u2 (the same test as the reference's
-// vertex matching, pulledback_integrand_gpu.jl:41-51).
+// vertex matching, pulledback_integrand_gpu.jl:41-51), and BGB_MASK_INEXACT.
 // ----------------------------------------------------------------------------------------
 __device__ int classify_exact(const Geo64& a, const Geo64& b, double k2, int* mask = nullptr) {
   const double dtol = 2.220446049250313e-16 * 1.0e3;
   const double xtol2 = 0.2 * 0.2;
-  int hits = 0, m = 0;
+  int hits = 0, m = 0, inexact = 0;
   double dmin2 = 1.7976931348623157e308;  // floatmax(Float64)
 #pragma unroll
   for (int u1 = 0; u1 < 3; ++u1)
@@ -117,9 +120,10 @@ __device__ int classify_exact(const Geo64& a, const Geo64& b, double k2, int* ma
       const bool hit = __dsqrt_rn(d2) < dtol;
       hits += hit;
       m |= (int)hit << (u1 * 3 + u2);
+      inexact |= hit && d2 != 0.0;
       dmin2 = fmin(dmin2, d2);
     }
-  if (mask) *mask = m;
+  if (mask) *mask = m | (inexact ? BGB_MASK_INEXACT : 0);
   if (hits > 3) return -1;
   if (hits > 0) return hits;
   const double mx = fmax(__dmul_rn(dmin2, k2), __ddiv_rn(dmin2, __dmul_rn(16.0, b.area)));
@@ -150,6 +154,8 @@ __device__ __forceinline__ void classify_sweep(int tau, float4 a, const Geo64& A
       if (cls < 0) {
         atomicOr(err, 1);
         cls = 0;
+      } else if (mask & BGB_MASK_INEXACT) {
+        atomicOr(err + 1, 1);
       }
     }
     const unsigned bal = __ballot_sync(0xffffffffu, cls != 0);
@@ -359,11 +365,26 @@ __device__ inline void make_pair_geo(const Geo64& A, const Geo64& B, const Chart
 __device__ inline void exp_tails(double zr, double zi, double2& e2, double2& e3) {
   const double2 mz = make_double2(-zr, -zi);
   const double2 z2h = make_double2(0.5 * (zr * zr - zi * zi), zr * zi);
+  if (zr == 0.0 && zi * zi < 1.0) {
+    // lossless: the even and the odd terms are real series in zi^2, to zi^20 / 20! (the FP64 divisions of the
+    // complex Horner form below were most of a near pair's work)
+    const double y2 = zi * zi;
+    double c = 1.0, s = 1.0;  // y^4 / 24 (1 - y^2 / (5 6) (1 - ...)), y^3 / 6 (1 - y^2 / (4 5) (1 - ...))
+#pragma unroll
+    for (int n = 20; n >= 6; n -= 2) {
+      c = fma(-c * y2, 1.0 / (n * (n - 1)), 1.0);
+      s = fma(-s * y2, 1.0 / ((n - 1) * (n - 2)), 1.0);
+    }
+    e3 = make_double2(y2 * y2 * (1.0 / 24.0) * c, zi * y2 * (1.0 / 6.0) * s);
+    e2 = make_double2(e3.x - 0.5 * y2, e3.y);
+    return;
+  }
   if (zr * zr + zi * zi < 1.0) {
     double2 s = make_double2(1.0, 0.0);
+#pragma unroll
     for (int n = 20; n >= 4; --n) {
       const double2 t = cmul(s, mz);
-      s = make_double2(1.0 + t.x / n, t.y / n);
+      s = make_double2(fma(t.x, 1.0 / n, 1.0), t.y * (1.0 / n));
     }
     const double2 m3 = cmul(cmul(mz, mz), mz);
     e3 = cmul(make_double2(m3.x / 6.0, m3.y / 6.0), s);
@@ -527,7 +548,7 @@ __device__ void singular_part(const Geo64& T, const double x[3], const double ga
     sum_tk1 += t0 * K1;
     for (int c = 0; c < 3; ++c) {
       Jm1[c] += m[c] * K1;
-      J1[c] += m[c] * K3 / 3.0;
+      J1[c] += m[c] * (K3 * (1.0 / 3.0));
       Jm3[c] -= m[c] * f;
     }
   }
@@ -542,7 +563,7 @@ __device__ void singular_part(const Geo64& T, const double x[3], const double ga
   const double den = nq[0] * nq[1] * nq[2] + dot3d(q[0], q[1]) * nq[2] + dot3d(q[0], q[2]) * nq[1] + dot3d(q[1], q[2]) * nq[0];
   const double Om = -2.0 * atan2(trip, den);
   const double Im1 = sum_tf - d * Om;
-  const double I1 = (d * d * Im1 + sum_tk1) / 3.0;
+  const double I1 = (d * d * Im1 + sum_tk1) * (1.0 / 3.0);
   const double i4p = BGB_INV_4PI_D;
   const double g2hr = 0.5 * (gam[0] * gam[0] - gam[1] * gam[1]), g2hi = gam[0] * gam[1];  // gamma^2 / 2
   S.S0 = make_double2((Im1 - gam[0] * T.area + g2hr * I1) * i4p, (-gam[1] * T.area + g2hi * I1) * i4p);
@@ -821,10 +842,10 @@ __device__ void pair_integral64(const OpParams& op, const QuadSel& qs, const Rul
   finalize<OP>(op, A, B, cA, cB, acc, L);
 }
 
-// Singular / near pairs, one warp per entry.  BATCH: the operator constants of the test
-// triangle's problem (ops[tri_problem[tau]]) instead of op1.  Single and batched assemblies
-// share this code, so their values are bit-identical.
-template <int OP, bool BATCH, bool NEAR = false>
+// Singular / near pairs, one warp per entry.  ops (batches): the operator constants of the test
+// triangle's problem (ops[tri_problem[tau]]) instead of op1.  Single and batched assemblies run the
+// same instance, so their values are bit-identical.
+template <int OP, bool NEAR = false>
 __global__ void __launch_bounds__(256, NEAR ? 2 : 1) k_singular(OpParams op1, const OpParams* __restrict__ ops,
                                                   const int* __restrict__ tri_problem,
                                                   const __grid_constant__ QuadSel qs,
@@ -833,7 +854,8 @@ __global__ void __launch_bounds__(256, NEAR ? 2 : 1) k_singular(OpParams op1, co
                                                   const int* __restrict__ ent_tau, const int* __restrict__ ent_sigma,
                                                   const int8_t* __restrict__ ent_cls, int64_t n,
                                                   double2* __restrict__ out, const volatile int* abort_flag,
-                                                  int near_only, const int* __restrict__ perm,
+                                                  const int16_t* __restrict__ inexact_of,
+                                                  const int* __restrict__ near_list, const int* __restrict__ perm,
                                                   const int64_t* __restrict__ range) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -843,7 +865,7 @@ __global__ void __launch_bounds__(256, NEAR ? 2 : 1) k_singular(OpParams op1, co
   auto ent_at = [&](int64_t i) -> int64_t { return perm ? (int64_t)perm[i] : i; };
   auto entry = [&](int64_t e) {
     const int tau = ent_tau[e];
-    const OpParams op = BATCH ? ops[tri_problem[tau]] : op1;
+    const OpParams op = ops ? ops[tri_problem[tau]] : op1;
     const Geo64 A = tg[tau], B = bg[ent_sigma[e]];
     double2 L[3][3];
     pair_integral64<OP, NEAR>(op, qs, rules, ent_cls[e], A, B, L);
@@ -856,24 +878,45 @@ __global__ void __launch_bounds__(256, NEAR ? 2 : 1) k_singular(OpParams op1, co
     }
   };
   if (NEAR) {
-    // near pairs only (the others come from the double-float kernel): a warp reads the classes of
-    // 32 entries at once and integrates the near ones among them
-    for (int64_t b = i0 + warp0 * 32; b < i1; b += warps * 32) {
+    // near pairs only (the others come from the Sauter-Schwab kernels), from the list of k_near_list: near
+    // pairs sit next to each other in the entry list, so warps that scan it for them are unevenly loaded
+    for (int64_t i = warp0; i < near_list[0]; i += warps) {
       if (abort_flag && *abort_flag) return;
-      const int64_t i = b + lane;
-      unsigned near = __ballot_sync(0xffffffffu, i < i1 && ent_cls[ent_at(i)] == BGB_CLASS_NEAR);
-      while (near) {
-        const int l = __ffs(near) - 1;
-        near &= near - 1;
-        entry(ent_at(b + l));
-      }
+      entry(near_list[1 + i]);
     }
     return;
   }
   for (int64_t i = i0 + warp0; i < i1; i += warps) {
     if (abort_flag && *abort_flag) return;
-    entry(ent_at(i));
+    const int64_t e = ent_at(i);
+    if (inexact_of && !(inexact_of[e] & BGB_MASK_INEXACT)) continue;
+    entry(e);
   }
+}
+
+// The near pairs among the entries: list[0] (zeroed by the caller) their number, list[1 ..] the entries, in an
+// order that depends on the atomics (each entry writes only its own local matrix).
+__global__ void k_near_list(const int8_t* __restrict__ cls, int64_t n, const int* __restrict__ perm,
+                            const int64_t* __restrict__ range, int* __restrict__ list) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i0 = perm ? range[0] : 0, i1 = perm ? range[1] : n;
+  for (int64_t b = i0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31); b < i1;
+       b += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = b + lane;
+    const int e = i < i1 ? (perm ? perm[i] : (int)i) : 0;
+    const bool near = i < i1 && cls[e] == BGB_CLASS_NEAR;
+    const unsigned m = __ballot_sync(0xffffffffu, near);
+    if (!m) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(list, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (near) list[1 + at + __popc(m & ((1u << lane) - 1u))] = e;
+  }
+}
+static void launch_near_list(const int8_t* cls, int64_t n, const int* perm, const int64_t* range, int* list, int num_sms,
+                             cudaStream_t st) {
+  cudaMemsetAsync(list, 0, sizeof(int), st);
+  k_near_list<<<(int)std::min<int64_t>((n + 255) / 256, (int64_t)num_sms * 4), 256, 0, st>>>(cls, n, perm, range, list);
 }
 
 // Diagnostic: local matrices of a list of pairs (classified exactly or forced), FP64.
@@ -1014,20 +1057,21 @@ void launch_classify_dense(const Geo64* tg, const Geo64* bg, int t0, int t1, int
 void launch_singular(const OpParams& op, const QuadSel& qs, const RuleTable& rules, int rsA, int rsB, const Geo64* tg,
                      const Geo64* bg, const int* et, const int* es, const int8_t* ec, int64_t n, double2* out,
                      const volatile int* abort_flag, int num_sms, cudaStream_t st, bool near_only, const int* perm,
-                     const int64_t* range) {
+                     const int64_t* range, const int16_t* inexact_of, int* near_list) {
   (void)rsA;
   (void)rsB;
   if (n <= 0) return;
   int64_t blocks = (n + 7) / 8;
-  const int64_t cap = (int64_t)num_sms * (perm ? 2 : 32);  // a group: about one wave beside a far kernel
+  const int64_t cap = (int64_t)num_sms * (perm || near_only ? 2 : 32);  // a group: about one wave beside a far kernel
   if (blocks > cap) blocks = cap;
+  if (near_only) launch_near_list(ec, n, perm, range, near_list, num_sms, st);
 #define BGB_LAUNCH_SING(OPK)                                                                                   \
   if (near_only)                                                                                                 \
-    k_singular<OPK, false, true><<<(int)blocks, 256, 0, st>>>(op, nullptr, nullptr, qs, rules, tg, bg, et, es, ec, n, \
-                                                              out, abort_flag, 1, perm, range);                    \
+    k_singular<OPK, true><<<(int)blocks, 256, 0, st>>>(op, nullptr, nullptr, qs, rules, tg, bg, et, es, ec, n, \
+                                                              out, abort_flag, nullptr, near_list, perm, range);   \
   else                                                                                                           \
-    k_singular<OPK, false><<<(int)blocks, 256, 0, st>>>(op, nullptr, nullptr, qs, rules, tg, bg, et, es, ec, n, out, \
-                                                        abort_flag, 0, perm, range)
+    k_singular<OPK><<<(int)blocks, 256, 0, st>>>(op, nullptr, nullptr, qs, rules, tg, bg, et, es, ec, n, out, \
+                                                        abort_flag, inexact_of, nullptr, perm, range)
   switch (op.kind) {
     case BGB_OP_HELMHOLTZ3D_SL: BGB_LAUNCH_SING(BGB_OP_HELMHOLTZ3D_SL); break;
     case BGB_OP_MAXWELL3D_SL: BGB_LAUNCH_SING(BGB_OP_MAXWELL3D_SL); break;
@@ -1077,17 +1121,18 @@ void launch_classify_batched(bool fill, const float4* tb, const float4* bb, cons
 void launch_singular_batched(int op_kind, const OpParams* ops, const QuadSel& qs, const RuleTable& rules,
                              const Geo64* tg, const Geo64* bg, const int* tri_problem, const int* et, const int* es,
                              const int8_t* ec, int64_t n, double2* out, const volatile int* abort_flag, int num_sms,
-                             cudaStream_t st, bool near_only) {
+                             cudaStream_t st, bool near_only, const int16_t* inexact_of, int* near_list) {
   if (n <= 0) return;
   int64_t blocks = (n + 7) / 8;
-  if (blocks > (int64_t)num_sms * 32) blocks = (int64_t)num_sms * 32;
+  blocks = std::min(blocks, (int64_t)num_sms * (near_only ? 2 : 32));
+  if (near_only) launch_near_list(ec, n, nullptr, nullptr, near_list, num_sms, st);
 #define BGB_LAUNCH_SING(OPK)                                                                                  \
   if (near_only)                                                                                                \
-    k_singular<OPK, true, true><<<(int)blocks, 256, 0, st>>>(OpParams{}, ops, tri_problem, qs, rules, tg, bg, et, es, \
-                                                             ec, n, out, abort_flag, 1, nullptr, nullptr);          \
+    k_singular<OPK, true><<<(int)blocks, 256, 0, st>>>(OpParams{}, ops, tri_problem, qs, rules, tg, bg, et, es, \
+                                                             ec, n, out, abort_flag, nullptr, near_list, nullptr, nullptr); \
   else                                                                                                          \
-    k_singular<OPK, true><<<(int)blocks, 256, 0, st>>>(OpParams{}, ops, tri_problem, qs, rules, tg, bg, et, es, ec, n, \
-                                                       out, abort_flag, 0, nullptr, nullptr)
+    k_singular<OPK><<<(int)blocks, 256, 0, st>>>(OpParams{}, ops, tri_problem, qs, rules, tg, bg, et, es, ec, n, \
+                                                       out, abort_flag, inexact_of, nullptr, nullptr, nullptr)
   switch (op_kind) {
     case BGB_OP_HELMHOLTZ3D_SL: BGB_LAUNCH_SING(BGB_OP_HELMHOLTZ3D_SL); break;
     case BGB_OP_MAXWELL3D_SL: BGB_LAUNCH_SING(BGB_OP_MAXWELL3D_SL); break;

@@ -38,12 +38,13 @@ def test_panels_tiles_and_batch_bit_identical(name, rule):
         Z = bg.assemble_gpu(op, X, X, cfg, quadstrat=qs, out="device")
         np.testing.assert_array_equal(Z.cpu().numpy(), ref)
     # RWG tile 0: chunks of 16 triangles do not fit twice, narrower ones are used
-    for tile in (0, 7, 13, 18, 22) if X.refspace == 1 else (7, 13, 18, 22):
+    for tile in (0, 7, 13, 18, 22) if X.refspace == 1 and rule == (3, 4) else (7, 13, 18, 22):
         Z = bg.assemble_gpu(op, X, X, bg.GPUConfiguration(tile_config=tile), quadstrat=qs)
         np.testing.assert_array_equal(Z, ref)
     b = bg.Batch([(op, X, X)], bg.GPUConfiguration(), quadstrat=qs, autotune=False)
-    np.testing.assert_array_equal(b.outputs[0].cpu().numpy(), ref)
+    got = b.outputs[0].cpu().numpy()
     b.close()
+    np.testing.assert_array_equal(got, ref)
 
 
 @pytest.mark.parametrize("name", ["efie", "hh"])
