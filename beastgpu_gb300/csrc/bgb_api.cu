@@ -809,7 +809,7 @@ int bgb_local_matrices(bgb_handle* h, const bgb_operator* op, const bgb_space* t
   std::vector<float> dftab;
   if (precision == BGB_PREC_MIXED && df_singular_ok(opp, max_edge(test), max_edge(trial))) {
     DfTables M;
-    build_df_tables(qsel, R, dftab, M);
+    build_df_tables(qsel, dftab, M);
     if ((rc = h->df_tab.ensure(sizeof(float) * dftab.size()))) return rc;
     BGB_CUDA(cudaMemcpyAsync(h->df_tab.p, dftab.data(), sizeof(float) * dftab.size(), cudaMemcpyHostToDevice, h->stream));
     if ((rc = h->geodf_t.ensure(sizeof(GeoDf) * std::max(1, test->nt))) ||
@@ -1239,7 +1239,11 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
       launch_singular(opp, qsel, R, test->refspace, trial->refspace, gt, gb, h->ent_tau.as<int>(),
                       h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev,
                       h->num_sms, st, true, perm, range, nullptr, h->near_list.as<int>());
-      return 2;
+      if (inexact)
+        launch_singular(opp, qsel, R, test->refspace, trial->refspace, gt, gb, h->ent_tau.as<int>(),
+                        h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), nsing, h->sing_L.as<double2>(), h->abort_dev,
+                        h->num_sms, st, false, perm, range, h->ent_mask.as<int16_t>());
+      return inexact ? 3 : 2;
     }
     launch_ss64(opp.kind, opp, nullptr, nullptr, h->ss_tab, h->ss_pts.as<double>(), gt, gb, h->ent_tau.as<int>(),
                 h->ent_sigma.as<int>(), h->ent_cls.as<int8_t>(), h->ent_mask.as<int16_t>(), nsing,
@@ -1283,7 +1287,7 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     }
   }
   if (use_df) {
-    build_df_tables(qsel, R, df_host, M);
+    build_df_tables(qsel, df_host, M);
     if ((rc = h->df_tab.ensure(sizeof(float) * df_host.size()))) return rc;
     BGB_CUDA(cudaMemcpyAsync(h->df_tab.p, df_host.data(), sizeof(float) * df_host.size(), cudaMemcpyHostToDevice, h->stream));
     if ((rc = h->geodf_t.ensure(sizeof(GeoDf) * std::max(1, test->nt))) ||

@@ -117,11 +117,11 @@ int enqueue_device_work(bgb_batch* B, cudaStream_t st, bool far_only) {
       launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t, B->ent_tau.as<int>(),
                               B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing, B->sing_L.as<double2>(),
                               h->abort_dev, h->num_sms, st, true, nullptr, B->near_list.as<int>());
-      if (B->inexact)
-        launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t,
-                                B->ent_tau.as<int>(), B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing,
-                                B->sing_L.as<double2>(), h->abort_dev, h->num_sms, st, false, B->ent_mask.as<int16_t>());
     }
+    if (B->inexact)
+      launch_singular_batched(B->op_kind, B->ops.as<OpParams>(), B->qsel, B->rules, gt, gb, tp_t, B->ent_tau.as<int>(),
+                              B->ent_sigma.as<int>(), B->ent_cls.as<int8_t>(), B->nsing, B->sing_L.as<double2>(),
+                              h->abort_dev, h->num_sms, st, false, B->ent_mask.as<int16_t>());
     const int qt = B->rules.npoints[B->qsel.far_t], qb = B->rules.npoints[B->qsel.far_b];
     launch_prepare_rec(B->precision, 0, B->generic ? BGB_MAXQ : qt, gt, B->nt_t, B->rules, B->qsel.far_t, 1.0,
                        B->rec_t.p, st);
@@ -344,7 +344,7 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
       B->use_df &= df_singular_ok(ops[p], max_edge(&problems[p].test), max_edge(&problems[p].trial));
     if (B->use_df) {
       std::vector<float> tab;
-      build_df_tables(B->qsel, B->rules, tab, B->dfm);
+      build_df_tables(B->qsel, tab, B->dfm);
       std::vector<OpDf> od(n);
       for (int p = 0; p < n; ++p) od[p] = make_opdf(ops[p]);
       if ((rc = put(st, B->df_tab, tab)) || (rc = put(st, B->opdf, od))) return fail(rc);

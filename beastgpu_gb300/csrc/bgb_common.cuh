@@ -20,7 +20,7 @@
 // Vertex-match mask of a pair: bit 3 i + j when test vertex i and trial vertex j coincide; this bit when
 // some coincident pair is not bit-equal (within the tolerance only).
 #define BGB_MASK_INEXACT 512
-#define BGB_SS_SERIES 14   // longest cosine / sine series of the FP64 Sauter-Schwab kernel
+#define BGB_SS_SERIES 16   // longest cosine / sine series of the Sauter-Schwab kernels
 
 namespace bgb {
 

@@ -68,16 +68,16 @@ void launch_ss64(int op_kind, const OpParams& op, const OpParams* ops, const int
                  const int* perm = nullptr, const int64_t* range = nullptr);
 
 // ---- bgb_singular_df.cu ----------------------------------------------------------------
-// Host-built tables of the double-float singular kernel (one float buffer): Sauter-Schwab
-// region points (u1, u2, v1, v2, weight as df) per class, near-rule points (u, v, w as df) and
-// the sin / cos table.
+// Tables of the double-float singular kernel: those of SsTab64 as df (ray coordinates and weights in one
+// float buffer, five arrays of cnt pairs per class) and the sin / cos table.
 struct DfTables {
-  int ss_off[4], ss_cnt[4];
-  int near_t_off, near_b_off, near_qt, near_qb;
+  int ss_off[4], cnt[4], n[4];
   int trig_off, total_floats;
   DfTrig trig;
+  dfl gx[4][BGB_MAX_SS], gw[4][BGB_MAX_SS];
+  dfl ser[4][4][2 * BGB_SS_SERIES];
 };
-void build_df_tables(const QuadSel& qs, const RuleTable& R, std::vector<float>& buf, DfTables& M);
+void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M);
 // Per-triangle double-float geometry: vertices (df), area and 1 / area (df).
 struct GeoDf {
   float v[3][3][2];

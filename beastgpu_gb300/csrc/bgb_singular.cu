@@ -120,7 +120,7 @@ __device__ int classify_exact(const Geo64& a, const Geo64& b, double k2, int* ma
       const bool hit = __dsqrt_rn(d2) < dtol;
       hits += hit;
       m |= (int)hit << (u1 * 3 + u2);
-      inexact |= hit && d2 != 0.0;
+      inexact |= hit && __double_as_longlong(d2) != 0;  // an integer compare: the FP64 pipe is the bound
       dmin2 = fmin(dmin2, d2);
     }
   if (mask) *mask = m | (inexact ? BGB_MASK_INEXACT : 0);
@@ -935,6 +935,8 @@ __global__ void __launch_bounds__(256) k_local_diag64(OpParams op, const __grid_
     int mask = 0;
     const int exact = classify_exact(A, B, op.k2, &mask);
     int cls = force >= 0 ? force : exact;
+    // a forced class has no shared vertex to start from: the pair keeps this kernel's value
+    if (force >= 0 && exact != force) mask |= BGB_MASK_INEXACT;
     if (lane == 0 && mask_out) mask_out[e] = (int16_t)mask;
     if (cls < 0) {
       if (lane == 0) atomicOr(err, 1);

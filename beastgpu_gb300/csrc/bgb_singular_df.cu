@@ -1,19 +1,17 @@
-// Singular and near-pair integrals in double-float arithmetic (mixed-precision path).
+// Singular pairs in double-float arithmetic (mixed-precision path).
 //
-// Same rules as k_singular<OP> (Sauter-Schwab CF/CE/CV regions, SauterSchwab.jl:265-297, and
-// the near-pair double quadrature), evaluated with df = float + float values on the FP32
-// pipes instead of native FP64, which runs at 1/62 of the FP32 rate on GB300.  The region
-// points and weights are tabulated on the host in FP64 (the same formulas as ss_region) and
-// stored as df pairs; each point costs ~800 FP32-pipe operations against ~95 FP64 operations
-// (~5900 FP32-equivalents) in k_singular.  Accuracy: ~48-bit operations; local matrices
-// agree with the FP64 kernels and the oracle to ~1e-14 relative.  Operators with a lossy
-// wave number (Re gamma != 0) and angles k R >= 400 use the FP64 kernel.
+// The ray form of the Sauter-Schwab rules of bgb_ss64.cu -- x = P0 + xi X, y = P0 + xi Y from the shared
+// vertex, R = xi |X - Y|, the sum over xi as the series T_m(theta) -- evaluated with df = float + float
+// values on the FP32 pipes instead of native FP64, which runs at 1/62 of the FP32 rate on GB300.  A series
+// step costs 12 operations where its term is above 2^-24 of the leading one (the sum's order is known, so a
+// fast two-sum does) and one beyond; a ray of n = 4 points takes ~1000 FP32-pipe operations, where a
+// sincos and a reciprocal square root per point took ~2800.  Accuracy: ~48-bit operations; local
+// matrices agree with the FP64 kernels and the oracle to ~1e-14 relative.  Operators with a lossy wave
+// number (Re gamma != 0) and angles k R >= 400 use the FP64 kernel; near pairs and pairs whose
+// coincident vertices are not bit-equal stay with k_singular.
 //
-// Points are written relative to the charts' origin vertex: x = o_a + e_a1 u1 + e_a2 u2 and
-// d = x - y = (o_a - o_b) + X - Y, so the difference near the singularity is formed from
-// small terms (o_a = o_b for common faces and edges).  The operator moments are those of
-// k_singular (taken about the chart origins); the per-lane df sums are converted to FP64 for
-// the warp reduction and the 3x3 local matrix.
+// Bound by the FP32 pipe's issue.  One warp per pair; the per-lane sums are reduced through shared
+// memory (15 df additions per lane instead of 80), and nine lanes each form one entry in df.
 #include <cmath>
 #include <vector>
 
@@ -25,268 +23,329 @@ namespace bgb {
 
 namespace {
 
-constexpr int kSsEntryFloats = 10;   // u1, u2, v1, v2, w (df each)
-constexpr int kNearEntryFloats = 6;  // u, v, w (df each)
+constexpr int kWarps = 8;
 
-__device__ __forceinline__ dfl ldf(const float* p) { return dfl{p[0], p[1]}; }
-
+// Moments (complex): hats 9 (p_a q_b, p = (1, alpha xi, beta xi)); EFIE S, Px, Py, P0; MFIE sum H X x Y, sum H (X - Y).
 template <int OP>
-struct DfAcc {
-  static constexpr int N = OP == BGB_OP_HELMHOLTZ3D_SL ? 9 : (OP == BGB_OP_MAXWELL3D_SL ? 8 : 10);
-  dfl re[N], im[N];
+struct DfMoments {
+  static constexpr int N = OP == BGB_OP_HELMHOLTZ3D_SL ? 9 : (OP == BGB_OP_MAXWELL3D_SL ? 8 : 6);
+  static constexpr int M0 = OP == BGB_OP_MAXWELL3D_DL ? -1 : 0;  // lowest T_m used (three of them)
 };
-
-// One point pair: X, Y are the points relative to the chart origins, d = x - y, (bx, by) the
-// barycentric chart coordinates (Helmholtz), w the weight (quadrature weights x Jacobians).
-template <int OP>
-__device__ __forceinline__ void df_point(const dfl X[3], const dfl Y[3], const dfl d[3], dfl bx1, dfl bx2, dfl by1,
-                                         dfl by2, dfl w, dfl kd, bool oscill, const float4* __restrict__ tab,
-                                         const DfTrig& T, DfAcc<OP>& acc) {
-  const dfl R2 = df_add(df_add(df_mul(d[0], d[0]), df_mul(d[1], d[1])), df_mul(d[2], d[2]));
-  const dfl rinv = df_rsqrt(R2);
-  const dfl amp = df_mul(df_mul(w, rinv), T.inv4pi);
-  dfl gr = amp, gi = dfl{0.f, 0.f};
-  if (oscill) {
-    const dfl R = df_mul(R2, rinv);
-    dfl sn, cs;
-    df_sincos(df_mul(kd, R), tab, T, sn, cs);
-    gr = df_mul(amp, cs);
-    gi = df_neg(df_mul(amp, sn));
-  }
-  if (OP == BGB_OP_HELMHOLTZ3D_SL) {
-    const dfl one{1.f, 0.f};
-    const dfl p[3] = {one, bx1, bx2}, q[3] = {one, by1, by2};
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const dfl pq = (a == 0) ? q[b] : (b == 0 ? p[a] : df_mul(p[a], q[b]));
-        acc.re[a * 3 + b] = df_add(acc.re[a * 3 + b], df_mul(gr, pq));
-        acc.im[a * 3 + b] = df_add(acc.im[a * 3 + b], df_mul(gi, pq));
-      }
-  } else if (OP == BGB_OP_MAXWELL3D_SL) {
-    const dfl xy = df_add(df_add(df_mul(X[0], Y[0]), df_mul(X[1], Y[1])), df_mul(X[2], Y[2]));
-    const dfl v[8] = {xy, X[0], X[1], X[2], Y[0], Y[1], Y[2], dfl{1.f, 0.f}};
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      acc.re[k] = df_add(acc.re[k], df_mul(gr, v[k]));
-      acc.im[k] = df_add(acc.im[k], df_mul(gi, v[k]));
-    }
-    acc.re[7] = df_add(acc.re[7], gr);
-    acc.im[7] = df_add(acc.im[7], gi);
-  } else {
-    // H = -(gamma + 1/R) G / R with gamma = i k:  H = -(rinv + i k) (G rinv)
-    const dfl g2r = df_mul(gr, rinv), g2i = df_mul(gi, rinv);
-    const dfl Hr = df_neg(df_sub(df_mul(rinv, g2r), df_mul(kd, g2i)));
-    const dfl Hi = df_neg(df_add(df_mul(rinv, g2i), df_mul(kd, g2r)));
-    const dfl e0 = df_sub(df_mul(d[1], Y[2]), df_mul(d[2], Y[1]));
-    const dfl e1 = df_sub(df_mul(d[2], Y[0]), df_mul(d[0], Y[2]));
-    const dfl e2 = df_sub(df_mul(d[0], Y[1]), df_mul(d[1], Y[0]));
-    const dfl f0 = df_sub(df_mul(X[1], d[2]), df_mul(X[2], d[1]));
-    const dfl f1 = df_sub(df_mul(X[2], d[0]), df_mul(X[0], d[2]));
-    const dfl f2 = df_sub(df_mul(X[0], d[1]), df_mul(X[1], d[0]));
-    const dfl a1 = df_add(df_add(df_mul(X[0], e0), df_mul(X[1], e1)), df_mul(X[2], e2));
-    const dfl v[10] = {a1, e0, e1, e2, f0, f1, f2, d[0], d[1], d[2]};
-#pragma unroll
-    for (int k = 0; k < 10; ++k) {
-      acc.re[k] = df_add(acc.re[k], df_mul(Hr, v[k]));
-      acc.im[k] = df_add(acc.im[k], df_mul(Hi, v[k]));
-    }
-  }
-}
 
 __device__ __forceinline__ dfl gdf(const float* p) { return dfl{p[0], p[1]}; }
 
-// Local matrix entry (i, j) from the reduced moments, in df (moments about the chart origins).
+// a * b, not renormalised (the low part may reach a few units of the high part's last place)
+__device__ __forceinline__ dfl df_mulx(dfl a, dfl b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  return {p, __fmaf_rn(a.lo, b.hi, e)};
+}
+// a * b + c for |c| >= |a b|
+__device__ __forceinline__ dfl df_fma_big(dfl a, dfl b, dfl c) {
+  const dfl p = df_mulx(a, b);
+  float s, e;
+  df_fast_two_sum(c.hi, p.hi, s, e);
+  e = __fadd_rn(e, __fadd_rn(c.lo, p.lo));
+  dfl r;
+  df_fast_two_sum(s, e, r.hi, r.lo);
+  return r;
+}
+// c + a * b
+__device__ __forceinline__ dfl df_macc(dfl c, dfl a, dfl b) { return df_add(c, df_mulx(a, b)); }
+__device__ __forceinline__ dfl df_dot(const dfl a[3], const dfl b[3]) {
+  return df_macc(df_macc(df_mulx(a[0], b[0]), a[1], b[1]), a[2], b[2]);
+}
+// 1 / sqrt(s): hardware estimate y and one cubic step y (1 + r (1/2 + 3 r / 8)), r = 1 - s y^2 kept as two floats
+__device__ __forceinline__ dfl df_rsqrt_step(dfl s) {
+  const float y = rsqrtf(s.hi);
+  const float yy = __fmul_rn(y, y);
+  const dfl q = df_mulx(s, dfl{yy, __fmaf_rn(y, y, -yy)});
+  float rh, rl;
+  df_fast_two_sum(__fsub_rn(1.0f, q.hi), -q.lo, rh, rl);
+  const float h = 0.5f * y, p = __fmul_rn(h, rh);
+  float e = __fmaf_rn(h, rh, -p);
+  e = __fmaf_rn(h, rl, e);
+  e = __fmaf_rn(__fmul_rn(0.75f * h, rh), rh, e);
+  float o, t;
+  df_fast_two_sum(y, p, o, t);
+  dfl r;
+  df_fast_two_sum(o, __fadd_rn(t, e), r.hi, r.lo);
+  return r;
+}
+
+// Entry (i, j) of the local matrix from the reduced moments (re, im of moment q at v[2 q], v[2 q + 1]).
 template <int OP>
-__device__ __forceinline__ double2 df_entry(const OpDf& op, const GeoDf& A, const GeoDf& B, const dfl oa[3],
-                                            const dfl ob[3], const dfl* mr, const dfl* mi, int i, int j) {
+__device__ __forceinline__ double2 df_entry(const OpDf& op, const GeoDf& A, const GeoDf& B, const int I[3], const int J[3],
+                                            const float2* v, dfl inv4pi, int i, int j) {
+  auto m = [&](int q) { return dfl{v[q].x, v[q].y}; };
   const dfl ar = gdf(op.alpha[0]), ai = gdf(op.alpha[1]);
-  dfl tr, ti;
+  dfl tr{0.f, 0.f}, ti{0.f, 0.f};
   if (OP == BGB_OP_HELMHOLTZ3D_SL) {
-    // f = T p with T = [[0,1,0],[0,0,1],[1,-1,-1]]
-    const int Tm[3][3] = {{0, 1, 0}, {0, 0, 1}, {1, -1, -1}};
-    tr = ti = dfl{0.f, 0.f};
+    // hats of the reordered vertices: 1 - p1, p2, p1 - p2
+    const int H[3][3] = {{1, -1, 0}, {0, 0, 1}, {0, 1, -1}};
+    const int r = I[0] == i + 1 ? 0 : (I[1] == i + 1 ? 1 : 2), c = J[0] == j + 1 ? 0 : (J[1] == j + 1 ? 1 : 2);
     for (int a = 0; a < 3; ++a)
       for (int b = 0; b < 3; ++b) {
-        const int t = Tm[i][a] * Tm[j][b];
+        const int t = H[r][a] * H[c][b];
         if (t > 0) {
-          tr = df_add(tr, mr[a * 3 + b]);
-          ti = df_add(ti, mi[a * 3 + b]);
+          tr = df_add(tr, m(2 * (a * 3 + b)));
+          ti = df_add(ti, m(2 * (a * 3 + b) + 1));
         } else if (t < 0) {
-          tr = df_sub(tr, mr[a * 3 + b]);
-          ti = df_sub(ti, mi[a * 3 + b]);
+          tr = df_sub(tr, m(2 * (a * 3 + b)));
+          ti = df_sub(ti, m(2 * (a * 3 + b) + 1));
         }
       }
+    const dfl w = df_mul(df_mulf(df_mul(gdf(A.area), gdf(B.area)), 4.f), inv4pi);
+    tr = df_mul(tr, w);
+    ti = df_mul(ti, w);
     const dfl Lr = df_sub(df_mul(ar, tr), df_mul(ai, ti)), Li = df_add(df_mul(ar, ti), df_mul(ai, tr));
     return make_double2(df_to_double(Lr), df_to_double(Li));
   }
   dfl V[3], W[3];
   for (int c = 0; c < 3; ++c) {
-    V[c] = df_sub(gdf(A.v[i][c]), oa[c]);
-    W[c] = df_sub(gdf(B.v[j][c]), ob[c]);
+    V[c] = df_sub(gdf(A.v[i][c]), gdf(A.v[I[0] - 1][c]));
+    W[c] = df_sub(gdf(B.v[j][c]), gdf(B.v[J[0] - 1][c]));
   }
-  const dfl inv4AA = df_mulf(df_mul(gdf(A.inv_area), gdf(B.inv_area)), 0.25f);
   if (OP == BGB_OP_MAXWELL3D_SL) {
-    tr = mr[0];
-    ti = mi[0];
+    // (1/(4 A A') of the shapes cancels the Jacobians; the divergences leave 4)
+    tr = m(0);
+    ti = m(1);
     for (int c = 0; c < 3; ++c) {
-      tr = df_sub(tr, df_add(df_mul(V[c], mr[4 + c]), df_mul(W[c], mr[1 + c])));
-      ti = df_sub(ti, df_add(df_mul(V[c], mi[4 + c]), df_mul(W[c], mi[1 + c])));
+      tr = df_sub(tr, df_add(df_mul(V[c], m(8 + 2 * c)), df_mul(W[c], m(2 + 2 * c))));
+      ti = df_sub(ti, df_add(df_mul(V[c], m(9 + 2 * c)), df_mul(W[c], m(3 + 2 * c))));
     }
-    const dfl vw = df_add(df_add(df_mul(V[0], W[0]), df_mul(V[1], W[1])), df_mul(V[2], W[2]));
-    tr = df_add(tr, df_mul(vw, mr[7]));
-    ti = df_add(ti, df_mul(vw, mi[7]));
-    const dfl car = df_mul(ar, inv4AA), cai = df_mul(ai, inv4AA);
-    const dfl invAA = df_mulf(inv4AA, 4.f);
-    const dfl cbr = df_mul(gdf(op.beta[0]), invAA), cbi = df_mul(gdf(op.beta[1]), invAA);
-    dfl Lr = df_sub(df_mul(car, tr), df_mul(cai, ti));
-    dfl Li = df_add(df_mul(car, ti), df_mul(cai, tr));
-    Lr = df_add(Lr, df_sub(df_mul(cbr, mr[7]), df_mul(cbi, mi[7])));
-    Li = df_add(Li, df_add(df_mul(cbr, mi[7]), df_mul(cbi, mr[7])));
+    const dfl vw = df_dot(V, W), pr = m(14), pi = m(15);
+    tr = df_mul(df_add(tr, df_mul(vw, pr)), inv4pi);
+    ti = df_mul(df_add(ti, df_mul(vw, pi)), inv4pi);
+    const dfl i4{4.f * inv4pi.hi, 4.f * inv4pi.lo};
+    const dfl br = df_mul(gdf(op.beta[0]), i4), bi = df_mul(gdf(op.beta[1]), i4);
+    dfl Lr = df_sub(df_mul(ar, tr), df_mul(ai, ti)), Li = df_add(df_mul(ar, ti), df_mul(ai, tr));
+    Lr = df_add(Lr, df_sub(df_mul(br, pr), df_mul(bi, pi)));
+    Li = df_add(Li, df_add(df_mul(br, pi), df_mul(bi, pr)));
     return make_double2(df_to_double(Lr), df_to_double(Li));
   }
-  // MFIE: A1 - W.C - V.B + V.(E x W)
-  tr = mr[0];
-  ti = mi[0];
+  // MFIE: (W - V).B + (W x V).E with B = sum H X x Y, E = sum H (X - Y); the sign of H = -(gamma + 1/R) G / R at the end
+  const dfl x[3] = {df_sub(df_mul(W[1], V[2]), df_mul(W[2], V[1])), df_sub(df_mul(W[2], V[0]), df_mul(W[0], V[2])),
+                    df_sub(df_mul(W[0], V[1]), df_mul(W[1], V[0]))};
   for (int c = 0; c < 3; ++c) {
-    tr = df_sub(tr, df_add(df_mul(W[c], mr[4 + c]), df_mul(V[c], mr[1 + c])));
-    ti = df_sub(ti, df_add(df_mul(W[c], mi[4 + c]), df_mul(V[c], mi[1 + c])));
+    const dfl wv = df_sub(W[c], V[c]);
+    tr = df_add(tr, df_add(df_mul(wv, m(2 * c)), df_mul(x[c], m(6 + 2 * c))));
+    ti = df_add(ti, df_add(df_mul(wv, m(2 * c + 1)), df_mul(x[c], m(7 + 2 * c))));
   }
-  const dfl* Er = mr + 7;
-  const dfl* Ei = mi + 7;
-  const dfl xr[3] = {df_sub(df_mul(Er[1], W[2]), df_mul(Er[2], W[1])), df_sub(df_mul(Er[2], W[0]), df_mul(Er[0], W[2])),
-                     df_sub(df_mul(Er[0], W[1]), df_mul(Er[1], W[0]))};
-  const dfl xi[3] = {df_sub(df_mul(Ei[1], W[2]), df_mul(Ei[2], W[1])), df_sub(df_mul(Ei[2], W[0]), df_mul(Ei[0], W[2])),
-                     df_sub(df_mul(Ei[0], W[1]), df_mul(Ei[1], W[0]))};
-  for (int c = 0; c < 3; ++c) {
-    tr = df_add(tr, df_mul(V[c], xr[c]));
-    ti = df_add(ti, df_mul(V[c], xi[c]));
-  }
-  const dfl car = df_mul(ar, inv4AA), cai = df_mul(ai, inv4AA);
-  const dfl Lr = df_sub(df_mul(car, tr), df_mul(cai, ti)), Li = df_add(df_mul(car, ti), df_mul(cai, tr));
+  tr = df_mul(tr, df_neg(inv4pi));
+  ti = df_mul(ti, df_neg(inv4pi));
+  const dfl Lr = df_sub(df_mul(ar, tr), df_mul(ai, ti)), Li = df_add(df_mul(ar, ti), df_mul(ai, tr));
   return make_double2(df_to_double(Lr), df_to_double(Li));
 }
 
-template <int OP, bool BATCH>
-__global__ void __launch_bounds__(256) k_singular_df(OpDf op1, const OpDf* __restrict__ ops,
-                                                     const int* __restrict__ tri_problem, const __grid_constant__ DfTables M,
-                                                     const float* __restrict__ tab, const GeoDf* __restrict__ tg,
-                                                     const GeoDf* __restrict__ bg, const int* __restrict__ ent_tau,
-                                                     const int* __restrict__ ent_sigma, const int8_t* __restrict__ ent_cls,
-                                                     const int16_t* __restrict__ ent_mask, int64_t n,
-                                                     double2* __restrict__ out, const volatile int* abort_flag,
-                                                     const int* __restrict__ perm, const int64_t* __restrict__ range) {
+template <int OP>
+__global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const OpDf* __restrict__ ops,
+                                                                const int* __restrict__ tri_problem,
+                                                                const __grid_constant__ DfTables M,
+                                                                const float* __restrict__ tab, const GeoDf* __restrict__ tg,
+                                                                const GeoDf* __restrict__ bg, const int* __restrict__ ent_tau,
+                                                                const int* __restrict__ ent_sigma,
+                                                                const int8_t* __restrict__ ent_cls,
+                                                                const int16_t* __restrict__ ent_mask, int64_t n,
+                                                                double2* __restrict__ out, const volatile int* abort_flag,
+                                                                const int* __restrict__ perm,
+                                                                const int64_t* __restrict__ range) {
+  constexpr int NA = DfMoments<OP>::N, NV = 2 * NA, M0 = DfMoments<OP>::M0;
+  constexpr int NS = NV <= 16 ? 16 : 32;  // rows of the reduction (two lanes per row when 16 suffice)
   __shared__ float4 trig[128];
+  __shared__ float2 part[kWarps][NV][33];
+  __shared__ float2 red[kWarps][NV];
   for (int i = threadIdx.x; i < 128; i += blockDim.x) trig[i] = ((const float4*)(tab + M.trig_off))[i];
   __syncthreads();
-  constexpr int NA = DfAcc<OP>::N;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   // perm: the entries perm[range[0] .. range[1]) (one output block's group); otherwise 0 .. n
   const int64_t i0 = perm ? range[0] : 0, i1 = perm ? range[1] : n;
-  for (int64_t i = i0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < i1; i += warps) {
+  for (int64_t it = i0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < i1; it += warps) {
     if (abort_flag && *abort_flag) return;
-    const int64_t e = perm ? (int64_t)perm[i] : i;
-    const int cls = ent_cls[e];
-    if (cls == BGB_CLASS_NEAR) continue;  // near pairs stay FP64 (k_singular with near_only)
-    const int tau = ent_tau[e];
-    const OpDf op = BATCH ? ops[tri_problem[tau]] : op1;
-    const GeoDf A = tg[tau], B = bg[ent_sigma[e]];
-    DfAcc<OP> acc;
-#pragma unroll
-    for (int k = 0; k < NA; ++k) acc.re[k] = acc.im[k] = dfl{0.f, 0.f};
-    const dfl kd = gdf(op.k);
-    const bool oscill = op.oscill != 0;
-    dfl oa[3], ob[3];
-    if (cls == BGB_CLASS_NEAR) {
-      dfl ea[2][3], eb[2][3], D0[3];
-      for (int c = 0; c < 3; ++c) {
-        oa[c] = gdf(A.v[2][c]);
-        ob[c] = gdf(B.v[2][c]);
-        ea[0][c] = df_sub(gdf(A.v[0][c]), oa[c]);
-        ea[1][c] = df_sub(gdf(A.v[1][c]), oa[c]);
-        eb[0][c] = df_sub(gdf(B.v[0][c]), ob[c]);
-        eb[1][c] = df_sub(gdf(B.v[1][c]), ob[c]);
-        D0[c] = df_sub(oa[c], ob[c]);
-      }
-      const dfl AB = df_mul(gdf(A.area), gdf(B.area));
-      const float* tt = tab + M.near_t_off;
-      const float* tb = tab + M.near_b_off;
-      for (int idx = lane; idx < M.near_qt * M.near_qb; idx += 32) {
-        const int I = idx / M.near_qb, J = idx - I * M.near_qb;
-        const float* p = tt + I * kNearEntryFloats;
-        const float* q = tb + J * kNearEntryFloats;
-        const dfl u = ldf(p), v = ldf(p + 2), wI = ldf(p + 4);
-        const dfl s = ldf(q), t = ldf(q + 2), wJ = ldf(q + 4);
-        dfl X[3], Y[3], d[3];
-        for (int c = 0; c < 3; ++c) {
-          X[c] = df_add(df_mul(ea[0][c], u), df_mul(ea[1][c], v));
-          Y[c] = df_add(df_mul(eb[0][c], s), df_mul(eb[1][c], t));
-          d[c] = df_sub(df_add(D0[c], X[c]), Y[c]);
-        }
-        df_point<OP>(X, Y, d, u, v, s, t, df_mul(df_mul(wI, wJ), AB), kd, oscill, trig, M.trig, acc);
-      }
-    } else if (!(OP == BGB_OP_MAXWELL3D_DL && cls == BGB_CLASS_CF)) {
-      int I[3], J[3];
-      ss_permutation_mask(cls, ent_mask[e], I, J);
-      for (int k = 0; k < 3; ++k) {  // guard against an inconsistent mask
-        I[k] = I[k] < 1 ? 1 : (I[k] > 3 ? 3 : I[k]);
-        J[k] = J[k] < 1 ? 1 : (J[k] > 3 ? 3 : J[k]);
-      }
-      const int ia0 = I[2] - 1, ia1 = I[0] - 1, ia2 = I[1] - 1;
-      const int ib0 = J[2] - 1, ib1 = J[0] - 1, ib2 = J[1] - 1;
-      dfl ea[2][3], eb[2][3], D0[3];
-      for (int c = 0; c < 3; ++c) {
-        oa[c] = gdf(A.v[ia0][c]);
-        ob[c] = gdf(B.v[ib0][c]);
-        ea[0][c] = df_sub(gdf(A.v[ia1][c]), oa[c]);
-        ea[1][c] = df_sub(gdf(A.v[ia2][c]), oa[c]);
-        eb[0][c] = df_sub(gdf(B.v[ib1][c]), ob[c]);
-        eb[1][c] = df_sub(gdf(B.v[ib2][c]), ob[c]);
-        D0[c] = df_sub(oa[c], ob[c]);
-      }
-      // barycentric chart coordinates b = cv3 + (cv1 - cv3) u1 + (cv2 - cv3) u2 with the
-      // reference-triangle vertices (1,0), (0,1), (0,0) (integer coefficients)
-      const float VX[3] = {1.f, 0.f, 0.f}, VY[3] = {0.f, 1.f, 0.f};
-      const float ba0 = VX[ia0], ba1 = VY[ia0], bb0 = VX[ib0], bb1 = VY[ib0];
-      const float cax1 = VX[ia1] - ba0, cax2 = VX[ia2] - ba0, cay1 = VY[ia1] - ba1, cay2 = VY[ia2] - ba1;
-      const float cbx1 = VX[ib1] - bb0, cbx2 = VX[ib2] - bb0, cby1 = VY[ib1] - bb1, cby2 = VY[ib2] - bb1;
-      const dfl jac = df_mulf(df_mul(gdf(A.area), gdf(B.area)), 4.f);
-      const float* tbl = tab + M.ss_off[cls];
-      const int cnt = M.ss_cnt[cls];
-      for (int idx = lane; idx < cnt; idx += 32) {
-        const float* p = tbl + idx * kSsEntryFloats;
-        const dfl u1 = ldf(p), u2 = ldf(p + 2), v1 = ldf(p + 4), v2 = ldf(p + 6), mul = ldf(p + 8);
-        dfl X[3], Y[3], d[3];
-        for (int c = 0; c < 3; ++c) {
-          X[c] = df_add(df_mul(ea[0][c], u1), df_mul(ea[1][c], u2));
-          Y[c] = df_add(df_mul(eb[0][c], v1), df_mul(eb[1][c], v2));
-          d[c] = df_sub(df_add(D0[c], X[c]), Y[c]);
-        }
-        dfl bx1{0.f, 0.f}, bx2{0.f, 0.f}, by1{0.f, 0.f}, by2{0.f, 0.f};
-        if (OP == BGB_OP_HELMHOLTZ3D_SL) {
-          bx1 = df_addf(df_add(df_mulf(u1, cax1), df_mulf(u2, cax2)), ba0);
-          bx2 = df_addf(df_add(df_mulf(u1, cay1), df_mulf(u2, cay2)), ba1);
-          by1 = df_addf(df_add(df_mulf(v1, cbx1), df_mulf(v2, cbx2)), bb0);
-          by2 = df_addf(df_add(df_mulf(v1, cby1), df_mulf(v2, cby2)), bb1);
-        }
-        df_point<OP>(X, Y, d, bx1, bx2, by1, by2, df_mul(jac, mul), kd, oscill, trig, M.trig, acc);
-      }
-    } else {
-      for (int c = 0; c < 3; ++c) oa[c] = ob[c] = dfl{0.f, 0.f};
+    const int64_t e = perm ? (int64_t)perm[it] : it;
+    const int cls = ent_cls[e], mask = ent_mask[e];
+    if (cls < BGB_CLASS_CV || cls > BGB_CLASS_CF || (mask & BGB_MASK_INEXACT)) continue;  // k_singular
+    if (OP == BGB_OP_MAXWELL3D_DL && cls == BGB_CLASS_CF) {  // vanishes on a flat face
+      if (lane < 9) out[e * 9 + lane] = make_double2(0.0, 0.0);
+      continue;
     }
-    // warp reduction in df
-#pragma unroll
-    for (int k = 0; k < NA; ++k)
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const dfl orr{__shfl_xor_sync(0xffffffffu, acc.re[k].hi, off), __shfl_xor_sync(0xffffffffu, acc.re[k].lo, off)};
-        const dfl oii{__shfl_xor_sync(0xffffffffu, acc.im[k].hi, off), __shfl_xor_sync(0xffffffffu, acc.im[k].lo, off)};
-        acc.re[k] = df_add(acc.re[k], orr);
-        acc.im[k] = df_add(acc.im[k], oii);
+    const int tau = ent_tau[e];
+    const OpDf& op = ops ? ops[tri_problem[tau]] : op1;  // one instance for both: the same bits
+    const GeoDf &A = tg[tau], &B = bg[ent_sigma[e]];
+    int I[3], J[3];
+    ss_permutation_mask(cls, mask, I, J);
+    for (int k = 0; k < 3; ++k) {  // guard against an inconsistent mask
+      I[k] = I[k] < 1 ? 1 : (I[k] > 3 ? 3 : I[k]);
+      J[k] = J[k] < 1 ? 1 : (J[k] > 3 ? 3 : J[k]);
+    }
+    dfl a1[3], a2[3], b1[3], b2[3];
+    float la = 0.f, lb = 0.f, l2 = 0.f, m2 = 0.f;
+    for (int c = 0; c < 3; ++c) {
+      a1[c] = df_sub(gdf(A.v[I[2] - 1][c]), gdf(A.v[I[0] - 1][c]));
+      a2[c] = df_sub(gdf(A.v[I[1] - 1][c]), gdf(A.v[I[2] - 1][c]));
+      b1[c] = df_sub(gdf(B.v[J[2] - 1][c]), gdf(B.v[J[0] - 1][c]));
+      b2[c] = df_sub(gdf(B.v[J[1] - 1][c]), gdf(B.v[J[2] - 1][c]));
+      const float x = a1[c].hi, y = b1[c].hi, z = x + a2[c].hi, w = y + b2[c].hi;
+      la = fmaf(x, x, la);
+      lb = fmaf(y, y, lb);
+      l2 = fmaf(z, z, l2);
+      m2 = fmaf(w, w, m2);
+    }
+    const dfl kd = gdf(op.k);
+    // terms of the series (theta <= k (largest |X| + largest |Y|), on one face k times its edge): nd in df, then float ones to 2^-51
+    int nd = 0, nj = 0;
+    {
+      const float th = 1.0001f * fabsf(kd.hi) * (sqrtf(fmaxf(la, l2)) + (cls == BGB_CLASS_CF ? 0.f : sqrtf(fmaxf(lb, m2))));
+      if (th <= 3.f) {
+        float t = 1.f;
+        do {
+          ++nj;
+          if (t > 6e-8f) nd = nj;
+          t *= th * th / (float)((2 * nj - 1) * (2 * nj));
+        } while (t > 4e-16f && nj < BGB_SS_SERIES);
       }
-    if (lane < 9) out[e * 9 + lane] = df_entry<OP>(op, A, B, oa, ob, acc.re, acc.im, lane / 3, lane % 3);
+    }
+    dfl acc[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = dfl{0.f, 0.f};
+    const int cnt = M.cnt[cls];
+    const float2* __restrict__ pt = (const float2*)(tab + M.ss_off[cls]);
+    for (int idx = lane; idx < cnt; idx += 32) {
+      const float2 p0 = pt[idx], p1 = pt[cnt + idx], p2 = pt[2 * cnt + idx], p3 = pt[3 * cnt + idx], p4 = pt[4 * cnt + idx];
+      const dfl al{p0.x, p0.y}, be{p1.x, p1.y}, ga{p2.x, p2.y}, de{p3.x, p3.y}, om{p4.x, p4.y};
+      dfl X[3], Y[3], d[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        X[c] = df_macc(df_mulx(al, a1[c]), be, a2[c]);
+        Y[c] = df_macc(df_mulx(ga, b1[c]), de, b2[c]);
+        d[c] = df_sub(X[c], Y[c]);
+      }
+      const dfl r2 = df_dot(d, d);
+      const dfl rinv = df_rsqrt_step(r2);
+      const dfl th = df_mul(kd, df_mulx(r2, rinv));
+      dfl C[3], S[3];  // T_m = C - i S, m = M0 .. M0 + 2
+      if (nj > 0) {
+        const dfl th2 = df_mul(th, th);
+        const dfl(*__restrict__ ser)[2 * BGB_SS_SERIES] = M.ser[cls];
+        float c[3], s[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) c[q] = s[q] = 0.f;
+        for (int k = nj - 1; k >= nd; --k) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            c[q] = __fmaf_rn(c[q], th2.hi, ser[q + 1 + M0][2 * k].hi);
+            s[q] = __fmaf_rn(s[q], th2.hi, ser[q + 1 + M0][2 * k + 1].hi);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          C[q] = dfl{c[q], 0.f};
+          S[q] = dfl{s[q], 0.f};
+        }
+        for (int k = nd - 1; k >= 1; --k) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            C[q] = df_fma_big(C[q], th2, ser[q + 1 + M0][2 * k]);
+            S[q] = df_fma_big(S[q], th2, ser[q + 1 + M0][2 * k + 1]);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {  // the first two terms may be of either order
+          C[q] = df_macc(ser[q + 1 + M0][0], C[q], th2);
+          S[q] = df_mul(df_macc(ser[q + 1 + M0][1], S[q], th2), th);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) C[q] = S[q] = dfl{0.f, 0.f};
+        for (int l = 0; l < M.n[cls]; ++l) {
+          dfl sn, cs;
+          const dfl xi = M.gx[cls][l];
+          df_sincos(df_mul(th, xi), trig, M.trig, sn, cs);
+          dfl w = df_mul(M.gw[cls][l], xi);
+          if (M0 == 0) w = df_mul(w, xi);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            C[q] = df_macc(C[q], w, cs);
+            S[q] = df_macc(S[q], w, sn);
+            w = df_mul(w, xi);
+          }
+        }
+      }
+      const dfl g = df_mul(om, rinv);
+      if (OP == BGB_OP_MAXWELL3D_DL) {
+        // (i k + 1/(xi R)) (C - i S): degree 2 (X x Y) from T_1, T_0 / R, degree 1 (X - Y) from T_0, T_-1 / R
+        const dfl f = df_mul(g, rinv);
+        const dfl hr2 = df_mul(f, df_add(df_mulx(kd, S[2]), df_mulx(rinv, C[1])));
+        const dfl hi2 = df_mul(f, df_sub(df_mulx(kd, C[2]), df_mulx(rinv, S[1])));
+        const dfl hr1 = df_mul(f, df_add(df_mulx(kd, S[1]), df_mulx(rinv, C[0])));
+        const dfl hi1 = df_mul(f, df_sub(df_mulx(kd, C[1]), df_mulx(rinv, S[0])));
+        const dfl x[3] = {df_sub(df_mulx(X[1], Y[2]), df_mulx(X[2], Y[1])), df_sub(df_mulx(X[2], Y[0]), df_mulx(X[0], Y[2])),
+                          df_sub(df_mulx(X[0], Y[1]), df_mulx(X[1], Y[0]))};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          acc[2 * c] = df_macc(acc[2 * c], hr2, x[c]);
+          acc[2 * c + 1] = df_macc(acc[2 * c + 1], hi2, x[c]);
+          acc[6 + 2 * c] = df_macc(acc[6 + 2 * c], hr1, d[c]);
+          acc[7 + 2 * c] = df_macc(acc[7 + 2 * c], hi1, d[c]);
+        }
+      } else if (OP == BGB_OP_MAXWELL3D_SL) {
+        const dfl xy = df_mul(g, df_dot(X, Y)), t1r = df_mul(g, C[1]), t1i = df_mul(df_neg(g), S[1]);
+        acc[0] = df_macc(acc[0], xy, C[2]);
+        acc[1] = df_macc(acc[1], xy, df_neg(S[2]));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          acc[2 + 2 * c] = df_macc(acc[2 + 2 * c], t1r, X[c]);
+          acc[3 + 2 * c] = df_macc(acc[3 + 2 * c], t1i, X[c]);
+          acc[8 + 2 * c] = df_macc(acc[8 + 2 * c], t1r, Y[c]);
+          acc[9 + 2 * c] = df_macc(acc[9 + 2 * c], t1i, Y[c]);
+        }
+        acc[14] = df_macc(acc[14], g, C[0]);
+        acc[15] = df_macc(acc[15], g, df_neg(S[0]));
+      } else {
+        dfl tr[3], ti[3];  // kernel sums of degree 0, 1, 2
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          tr[q] = df_mul(g, C[q]);
+          ti[q] = df_mul(df_neg(g), S[q]);
+        }
+        const dfl p[3] = {dfl{1.f, 0.f}, al, be}, q[3] = {dfl{1.f, 0.f}, ga, de};
+        acc[0] = df_add(acc[0], tr[0]);
+        acc[1] = df_add(acc[1], ti[0]);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+          for (int b = 0; b < 3; ++b) {
+            if (a + b == 0) continue;
+            const int deg = (a > 0) + (b > 0);
+            const dfl pq = a == 0 ? q[b] : (b == 0 ? p[a] : df_mul(p[a], q[b]));
+            acc[2 * (3 * a + b)] = df_macc(acc[2 * (3 * a + b)], tr[deg], pq);
+            acc[2 * (3 * a + b) + 1] = df_macc(acc[2 * (3 * a + b) + 1], ti[deg], pq);
+          }
+      }
+    }
+    // reduction: lane v (and v + 16 when 16 rows suffice) sums row v
+#pragma unroll
+    for (int k = 0; k < NV; ++k) part[wid][k][lane] = make_float2(acc[k].hi, acc[k].lo);
+    __syncwarp();
+    {
+      const int v = lane & (NS - 1), h = NS == 16 ? (lane >> 4) * 16 : 0;
+      dfl s{0.f, 0.f};
+      if (v < NV)
+        for (int k = 0; k < (NS == 16 ? 16 : 32); ++k) {
+          const float2 x = part[wid][v][h + k];
+          s = df_add(s, dfl{x.x, x.y});
+        }
+      if (NS == 16) {
+        const dfl o{__shfl_xor_sync(0xffffffffu, s.hi, 16), __shfl_xor_sync(0xffffffffu, s.lo, 16)};
+        s = df_add(s, o);
+      }
+      if (lane < NV) red[wid][lane] = make_float2(s.hi, s.lo);
+    }
+    __syncwarp();
+    if (lane < 9) out[e * 9 + lane] = df_entry<OP>(op, A, B, I, J, red[wid], M.trig.inv4pi, lane / 3, lane % 3);
+    __syncwarp();
   }
 }
 
@@ -322,56 +381,37 @@ void split_ld(long double x, float* out) {
 
 }  // namespace
 
-void build_df_tables(const QuadSel& qs, const RuleTable& R, std::vector<float>& buf, DfTables& M) {
+void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M) {
   buf.clear();
   M = DfTables{};
   auto align4 = [&]() {
     while (buf.size() % 4) buf.push_back(0.f);
   };
+  std::vector<double> pts;
+  SsTab64 T;
+  build_ss_tables(qs, pts, T);
+  auto df = [](double x) {
+    float q[2];
+    split(x, q);
+    return dfl{q[0], q[1]};
+  };
   for (int cls = 1; cls <= 3; ++cls) {
     align4();
     M.ss_off[cls] = (int)buf.size();
-    const int n = qs.ss[cls];
-    const int nreg = cls == BGB_CLASS_CV ? 2 : (cls == BGB_CLASS_CE ? 5 : 6);
-    const double* gx = qs.gl_x[cls];
-    const double* gw = qs.gl_w[cls];
-    int cnt = 0;
-    for (int i = 0; i < n; ++i)
-      for (int j = 0; j < n; ++j)
-        for (int k = 0; k < n; ++k)
-          for (int l = 0; l < n; ++l) {
-            const double wt = gw[i] * gw[j] * gw[k] * gw[l];
-            for (int r = 0; r < nreg; ++r) {
-              double u1, u2, v1, v2, mul;
-              ss_region(cls, r, gx[i], gx[j], gx[k], gx[l], wt, u1, u2, v1, v2, mul);
-              float e[10];
-              split(u1, e);
-              split(u2, e + 2);
-              split(v1, e + 4);
-              split(v2, e + 6);
-              split(mul, e + 8);
-              buf.insert(buf.end(), e, e + 10);
-              ++cnt;
-            }
-          }
-    M.ss_cnt[cls] = cnt;
-  }
-  for (int side = 0; side < 2; ++side) {
-    align4();
-    const int rule = side ? qs.near_b : qs.near_t;
-    if (side) M.near_b_off = (int)buf.size();
-    else M.near_t_off = (int)buf.size();
-    const int q = R.npoints[rule];
-    if (side) M.near_qb = q;
-    else M.near_qt = q;
-    for (int I = 0; I < q; ++I) {
-      const double* p = R.uvw[R.offset[rule] + I];
-      float e[6];
-      split(p[0], e);
-      split(p[1], e + 2);
-      split(p[2], e + 4);  // normalised weight (sum 1); the areas are applied per pair
-      buf.insert(buf.end(), e, e + 6);
+    M.cnt[cls] = T.cnt[cls];
+    M.n[cls] = T.n[cls];
+    for (int i = 0; i < 5 * T.cnt[cls]; ++i) {
+      float q[2];
+      split(pts[(size_t)T.off[cls] + i], q);
+      buf.push_back(q[0]);
+      buf.push_back(q[1]);
     }
+    for (int l = 0; l < T.n[cls]; ++l) {
+      M.gx[cls][l] = df(T.gx[cls][l]);
+      M.gw[cls][l] = df(T.gw[cls][l]);
+    }
+    for (int m = 0; m < 4; ++m)
+      for (int k = 0; k < 2 * BGB_SS_SERIES; ++k) M.ser[cls][m][k] = df(T.ser[cls][m][k]);
   }
   align4();
   M.trig_off = (int)buf.size();
@@ -430,21 +470,17 @@ void launch_singular_df(int op_kind, const OpDf& op, const OpDf* opdf_array, con
   int64_t blocks = (n + 7) / 8;
   const int64_t cap = (int64_t)num_sms * (perm ? 2 : 32);  // a group: about one wave beside a far kernel
   if (blocks > cap) blocks = cap;
-  const bool batch = opdf_array != nullptr;
-#define BGB_LAUNCH_DF(OPK)                                                                                        \
-  if (batch)                                                                                                      \
-    k_singular_df<OPK, true><<<(int)blocks, 256, 0, st>>>(op, opdf_array, tri_problem, M, dtab, tg, bg, et, es, ec, \
-                                                          emask, n, out, abort_flag, perm, range);               \
-  else                                                                                                            \
-    k_singular_df<OPK, false><<<(int)blocks, 256, 0, st>>>(op, opdf_array, tri_problem, M, dtab, tg, bg, et, es, ec, \
-                                                           emask, n, out, abort_flag, perm, range);
-  if (op_kind == BGB_OP_HELMHOLTZ3D_SL) {
-    BGB_LAUNCH_DF(BGB_OP_HELMHOLTZ3D_SL)
-  } else if (op_kind == BGB_OP_MAXWELL3D_SL) {
-    BGB_LAUNCH_DF(BGB_OP_MAXWELL3D_SL)
-  } else if (op_kind == BGB_OP_MAXWELL3D_DL) {
-    BGB_LAUNCH_DF(BGB_OP_MAXWELL3D_DL)
-  }  // other operators take the FP64 singular kernel (df_singular_ok)
+#define BGB_LAUNCH_DF(OPK)                                                                                          \
+  case OPK:                                                                                                         \
+    k_singular_df<OPK><<<(int)blocks, 32 * kWarps, 0, st>>>(op, opdf_array, tri_problem, M, dtab, tg, bg, et, es, ec, \
+                                                            emask, n, out, abort_flag, perm, range);                \
+    break
+  switch (op_kind) {  // other operators take the FP64 kernel (df_singular_ok)
+    BGB_LAUNCH_DF(BGB_OP_HELMHOLTZ3D_SL);
+    BGB_LAUNCH_DF(BGB_OP_MAXWELL3D_SL);
+    BGB_LAUNCH_DF(BGB_OP_MAXWELL3D_DL);
+    default: break;
+  }
 #undef BGB_LAUNCH_DF
 }
 

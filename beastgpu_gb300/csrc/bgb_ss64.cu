@@ -15,7 +15,7 @@
 //
 // Bound by the FP64 pipe.  One warp per pair; the per-lane sums are reduced through shared memory
 // (16 additions per lane instead of five butterfly steps per moment) and nine lanes each form one
-// entry.  theta up to 2 takes the series (its terms stay below 2); beyond, and for lossy wave numbers,
+// entry.  theta up to 3 takes the series (its terms stay below 5); beyond, and for lossy wave numbers,
 // the sum over xi is taken point by point.  Pairs whose coincident vertices are not bit-equal (flagged by
 // the classifier) have no common origin and stay with k_singular.
 #include "bgb_kernels.cuh"
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_ss64(OpParams op1, const OpP
     sub3(B.v[J[1] - 1], B.v[J[2] - 1], b2);
     if (OP == BGB_OP_HELMHOLTZ3D_DL) tri_unit_normal(B, nrm);
     if (OP == BGB_OP_HELMHOLTZ3D_DLT) tri_unit_normal(A, nrm);
-    // terms of the series: theta <= k (largest |X| + largest |Y|), truncation below 2^-56
+    // terms of the series: theta <= k (largest |X| + largest |Y|), on one face k times its edge; truncation below 2^-56
     int nj = 0;
     if (gre == 0.0) {
       float la = 0.f, lb = 0.f, l2 = 0.f, m2 = 0.f;
@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_ss64(OpParams op1, const OpP
         l2 = fmaf(z, z, l2);
         m2 = fmaf(w, w, m2);
       }
-      const float th = 1.0001f * fabsf((float)gim) * (sqrtf(fmaxf(la, l2)) + sqrtf(fmaxf(lb, m2)));
-      if (th <= 2.f) {
+      const float th = 1.0001f * fabsf((float)gim) * (sqrtf(fmaxf(la, l2)) + (cls == BGB_CLASS_CF ? 0.f : sqrtf(fmaxf(lb, m2))));
+      if (th <= 3.f) {
         float t = 1.f;
         do {
           ++nj;
