@@ -310,21 +310,22 @@ const TileCfg kTileCfgs[] = {
     {32, 32, 5},    // 20
     {24, 24, 5},    // 21
     {16, 16, 5},    // 22
+    {60, 80, 5},    // 23: mixed, RWG
 };
-// Preference order when the caller does not pin a tile: the first whose shared memory fits.
-// RWG: 60 x 64 tiles with 5-triangle chunks (C2 mixed far stage 28.6 ms against 31.1 ms for
-// 64 x 64 x 4, whose ~53 test triangles x 4 leave a sixth of the 256 threads idle in each chunk).
-const int kPrefMixed[] = {17, 4, 8, 1, 5, 6, 7};
+// Preference order when the caller does not pin a tile, widest first: the first whose shared memory
+// fits, from the first with at least a tile per CTA slot on (narrow_for_size).
+// RWG: ~50 test triangles x 5 are one round of 256 pairs per chunk; the wider trial side evaluates 1.5%
+// fewer pairs in a fifth fewer tiles (level-5 EFIE far stage: 60 x 80 x 5 20.7 ms, 60 x 64 x 5 21.7, 64 x 64 x 4
+// 23.3, 48 x 96 x 6 21.8).
+const int kPrefMixed[] = {23, 17, 19, 20, 21, 22, 7};
 const int kNumPrefMixed = sizeof(kPrefMixed) / sizeof(int);
 // (60 x 64 x 5 gained 0.4% on the FP64 EFIE and lost 3.5% on the FP64 MFIE: the FP64 pipe, not the
 // idle lanes, bounds the plain kernel)
 const int kPrefFp64[] = {4, 8, 5, 6, 7};
 const int kNumPrefFp64 = sizeof(kPrefFp64) / sizeof(int);
-// Lagrange hats have ~6 supports: small function blocks keep the halo and the gather short
-// (measured on the two-plate Helmholtz case: 32 x 32 tiles 6x faster than 64 x 64).
-// d = 40 cube, mixed: 32 x 40 x 5 330 ms, 40 x 40 x 4 334 ms, 32 x 32 x 4 364 ms (with the FP32
-// Lagrange kernels' per-chunk trial staging).
-const int kPrefLagrange[] = {18, 6, 13, 15, 5, 7};
+// Lagrange hats have ~6 supports: small function blocks keep the halo and the gather short (Helmholtz box of
+// 19,484 triangles: 32 x 40 x 5 18.8 ms, 32 x 48 x 5 19.3, 40 x 40 x 3 19.9, 32 x 32 x 4 21.0).
+const int kPrefLagrange[] = {18, 21, 22, 7};
 const int kNumPrefLagrange = sizeof(kPrefLagrange) / sizeof(int);
 // The plain FP64 kernel (one CTA per SM, FP64-pipe bound) gains from fewer halo pairs more than
 // from full chunks: d = 24 cube 48 x 48 x 4 1,537 ms, 40 x 40 x 4 1,629 ms, 32 x 40 x 5 1,693 ms.
@@ -942,14 +943,10 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   // The plain FP64 path computes the pairs of a panel once and gathers the tiles from them
   // (bgb_gather64.cu); the mixed path computes them inside the tiles.
   const bool two_phase = precision == BGB_PREC_FP64;
-  // small matrices: narrower tiles until there are two per SM
-  if (two_phase && !pinned_cfg) {
-    auto tiles = [&](int id) {
-      const TileCfg& c = kTileCfgs[id];
+  if (!pinned_cfg)
+    narrow_for_size(prefs, (two_phase ? 2 : far_target_ctas_per_sm(precision)) * (int64_t)h->num_sms, [&](const TileCfg& c) {
       return ((nrows + c.FM - 1) / c.FM) * ((ncols + c.FN - 1) / c.FN);
-    };
-    while (prefs.size() > 1 && tiles(prefs[0]) < 2 * (int64_t)h->num_sms) prefs.erase(prefs.begin());
-  }
+    });
   // Bytes of one panel's local matrices: up to 2 GiB (a few hundred trial triangles at 20,000 test
   // triangles, whose rims add 4 - 8% pairs), within the caller's budget and a quarter of free memory.
   int64_t panel_bytes = 0;
@@ -1032,78 +1029,60 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
       }
       PL.test = HostPlan();
       plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth);
-      PL.trial.assign(nblocks, HostPlan());
-      TilePlan probe{};
-      probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = tc.SC; probe.MAXS = PL.test.MAXS;
-      probe.tmax = std::max(1, PL.test.tmax);
-      over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, tc.SC, PL.trial[b], threads); });
-      for (int b = 0; b < nblocks; ++b) {
-        probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
-        probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
-        probe.nmax = std::max(probe.nmax, std::max(1, PL.trial[b].nmax));
-      }
-      if (two_phase) {
-        // a tile pinned by the caller is one that the fused kernel could run; the gather's two chunk
-        // buffers then take as many triangles as fit (the result does not depend on the chunks)
-        int per_sm = 0;
-        if (pinned_cfg) {
-          smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
-          if (smem > (size_t)smem_max || far_persistent_occupancy(precision, K.op_kind, gen, smem, &per_sm) || per_sm < 1)
-            continue;
+      // Chunks of tc.SC trial triangles; a tile pinned by the caller, and the last choice, also with
+      // narrower chunks when the chunk buffers do not fit (the result does not depend on the chunks).
+      for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
+        TilePlan probe{};
+        probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = sc; probe.MAXS = PL.test.MAXS;
+        probe.tmax = std::max(1, PL.test.tmax);
+        PL.trial.assign(nblocks, HostPlan());
+        over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
+        for (int b = 0; b < nblocks; ++b) {
+          probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
+          probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
+          probe.nmax = std::max(probe.nmax, std::max(1, PL.trial[b].nmax));
         }
-        for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
-          if (sc != tc.SC) {
-            PL.trial.assign(nblocks, HostPlan());
-            over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
-            probe.SC = sc;
-            probe.gmax = probe.gsmax = 0;
-            for (int b = 0; b < nblocks; ++b) {
-              probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
-              probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
+        int occ = 0;
+        if (two_phase) {
+          smem = gather64_smem_bytes(probe);
+          if (gather64_occupancy(smem, &occ)) occ = 0;
+        } else {
+          smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
+          // Occupancy: when the widest test tile pushes shared memory past what the kernel's
+          // CTAs per SM allow, cap the triangles per test tile at the largest count that fits.
+          if (smem <= (size_t)smem_max && far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ) == 0 &&
+              occ >= 1 && occ < target_occ) {
+            int cap = -1;
+            for (int t = probe.tmax - 1; t >= std::max(1, PL.test.MAXS); --t) {
+              TilePlan q = probe;
+              q.tmax = t;
+              const size_t sm = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, q);
+              int o = 0;
+              if (far_persistent_occupancy(precision, K.op_kind, gen, sm, &o) == 0 && o >= target_occ) {
+                cap = t;
+                break;
+              }
+            }
+            if (cap > 0) {
+              PL.test = HostPlan();
+              plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth, cap);
+              probe.MAXS = PL.test.MAXS;
+              probe.tmax = std::max(1, PL.test.tmax);
+              smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
             }
           }
-          smem = gather64_smem_bytes(probe);
-          if (gather64_occupancy(smem, &per_sm) == 0 && per_sm >= 1) {
-            PL.cfg_id = id;
-            PL.tc = {tc.FM, tc.FN, sc};
-            PL.smem = smem;
-          }
+          occ = 0;
+          if (smem > (size_t)smem_max || far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ)) occ = 0;
         }
-        if (PL.cfg_id >= 0) break;
-        continue;
-      }
-      smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
-      // Occupancy: when the widest test tile pushes shared memory past what the kernel's
-      // CTAs per SM allow, cap the triangles per test tile at the largest count that fits.
-      int occ = 0;
-      if (smem <= (size_t)smem_max && far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ) == 0 &&
-          occ >= 1 && occ < target_occ) {
-        int cap = -1;
-        for (int t = probe.tmax - 1; t >= std::max(1, PL.test.MAXS); --t) {
-          TilePlan q = probe;
-          q.tmax = t;
-          const size_t sm = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, q);
-          int o = 0;
-          if (far_persistent_occupancy(precision, K.op_kind, gen, sm, &o) == 0 && o >= target_occ) {
-            cap = t;
-            break;
-          }
-        }
-        if (cap > 0) {
-          PL.test = HostPlan();
-          plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth, cap);
-          probe.MAXS = PL.test.MAXS;
-          probe.tmax = std::max(1, PL.test.tmax);
-          smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
+        if (occ >= 1) {
+          PL.cfg_id = id;
+          PL.tc = {tc.FM, tc.FN, sc};
+          PL.smem = smem;
+        } else if (id != prefs.back()) {
+          break;
         }
       }
-      occ = 0;
-      if (smem <= (size_t)smem_max && far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ) == 0 && occ >= 1) {
-        PL.cfg_id = id;
-        PL.tc = tc;
-        PL.smem = smem;
-        break;
-      }
+      if (PL.cfg_id >= 0) break;
     }
     if (PL.cfg_id < 0) {
       char buf[160];

@@ -138,8 +138,8 @@ int enqueue_device_work(bgb_batch* B, cudaStream_t st, bool far_only) {
 int build_plans(bgb_batch* B, const bgb_problem* pr, const std::vector<Supports>& St, const std::vector<Supports>& Sb,
                 const std::vector<std::vector<double>>& cent_t, const std::vector<std::vector<double>>& cent_b,
                 const std::vector<int>& tbase, const std::vector<int>& bbase, int cfg, int schedule, bool upload_all,
-                size_t* smem_out) {
-  const TileCfg tc = kTileCfgs[cfg];
+                bool narrow, size_t* smem_out) {
+  TileCfg tc = kTileCfgs[cfg];
   const int n = B->n;
   std::vector<HostPlan> P(n);
   // one shared-memory layout for the whole launch: the batch-wide maxima
@@ -147,17 +147,33 @@ int build_plans(bgb_batch* B, const bgb_problem* pr, const std::vector<Supports>
   for (int p = 0; p < n; ++p) {
     // function orders in runs of this configuration's tile widths
     plan_test_side(St[p], order_functions(St[p], cent_t[p], 0, pr[p].test.nfun, tc.FM), tc.FM, 0, P[p]);
-    plan_trial_side(Sb[p], order_functions(Sb[p], cent_b[p], 0, pr[p].trial.nfun, tc.FN), tc.FN, tc.SC, P[p]);
+    tmax = std::max(tmax, P[p].tmax); MAXS = std::max(MAXS, P[p].MAXS);
+  }
+  int smem_max = 0;
+  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, B->h->device);
+  for (;; tc.SC /= 2) {  // narrower chunks when the chunk buffer does not fit (the result does not depend on them)
+    nmax = gmax = gsmax = 1;
+    for (int p = 0; p < n; ++p) {
+      HostPlan Q;
+      plan_trial_side(Sb[p], order_functions(Sb[p], cent_b[p], 0, pr[p].trial.nfun, tc.FN), tc.FN, tc.SC, Q);
+      P[p].bb_off.swap(Q.bb_off); P[p].bb_tris.swap(Q.bb_tris); P[p].bb_fn_off.swap(Q.bb_fn_off);
+      P[p].bb_chunk_off.swap(Q.bb_chunk_off); P[p].ch_grp_off.swap(Q.ch_grp_off); P[p].grp_fn.swap(Q.grp_fn);
+      P[p].grp_sup_off.swap(Q.grp_sup_off); P[p].gs_code.swap(Q.gs_code); P[p].gs_coef.swap(Q.gs_coef);
+      P[p].cols.swap(Q.cols);
+      P[p].nmax = Q.nmax; P[p].gmax = Q.gmax; P[p].gsmax = Q.gsmax;
+      nmax = std::max(nmax, Q.nmax); gmax = std::max(gmax, Q.gmax); gsmax = std::max(gsmax, Q.gsmax);
+    }
+    TilePlan probe{};
+    probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = tc.SC; probe.MAXS = MAXS;
+    probe.gmax = gmax; probe.gsmax = gsmax; probe.tmax = tmax; probe.nmax = nmax;
+    *smem_out = far_smem_bytes(B->precision, B->op_kind, B->rules.npoints[B->qsel.far_t],
+                               B->rules.npoints[B->qsel.far_b], probe);
+    if (*smem_out <= (size_t)smem_max || tc.SC == 1 || !narrow) break;
+  }
+  for (int p = 0; p < n; ++p) {
     for (int& t : P[p].tb_tris) t += tbase[p];
     for (int& t : P[p].bb_tris) t += bbase[p];
-    tmax = std::max(tmax, P[p].tmax); nmax = std::max(nmax, P[p].nmax); MAXS = std::max(MAXS, P[p].MAXS);
-    gmax = std::max(gmax, P[p].gmax); gsmax = std::max(gsmax, P[p].gsmax);
   }
-  TilePlan probe{};
-  probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = tc.SC; probe.MAXS = MAXS;
-  probe.gmax = gmax; probe.gsmax = gsmax; probe.tmax = tmax; probe.nmax = nmax;
-  *smem_out = far_smem_bytes(B->precision, B->op_kind, B->rules.npoints[B->qsel.far_t], B->rules.npoints[B->qsel.far_b],
-                             probe);
   if (!upload_all) return 0;
   // concatenate
   std::vector<int> I;
@@ -457,18 +473,26 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
   const int nprefs = lagrange ? (mixed ? kNumPrefLagrange : kNumPrefLagrangeFp64) : mixed ? kNumPrefMixed : kNumPrefFp64;
   std::vector<int> cands;
   if (h->cfg.tile_config >= 0) cands.push_back(h->cfg.tile_config);
-  else
-    for (int i = 0; i < nprefs; ++i) cands.push_back(prefs[i]);
+  else {
+    cands.assign(prefs, prefs + nprefs);
+    if (mixed)  // (the FP64 lists are not in order of width)
+      narrow_for_size(cands, far_target_ctas_per_sm(precision) * (int64_t)h->num_sms, [&](const TileCfg& c) {
+        int64_t t = 0;
+        for (int p = 0; p < n; ++p)
+          t += (int64_t)((problems[p].test.nfun + c.FM - 1) / c.FM) * ((problems[p].trial.nfun + c.FN - 1) / c.FN);
+        return t;
+      });
+  }
   const bool autotune = (flags & 1) && cands.size() > 1;
   // first full run (records + singular) with the first fitting candidate
   int first = -1;
   size_t smem = 0;
   for (int c : cands) {
-    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, 1, false, &smem))) return fail(rc);
+    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, 1, false, c == cands.back(), &smem))) return fail(rc);
     if (smem <= (size_t)smem_max) { first = c; break; }
   }
   if (first < 0) { set_error("bgb_batch_create: no tile shape fits shared memory"); return fail(BGB_ERR_CAPACITY); }
-  if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, first, 1, true, &smem))) return fail(rc);
+  if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, first, 1, true, first == cands.back(), &smem))) return fail(rc);
   auto set_cfg = [&](int cfg, size_t sm) -> int {
     B->cfg_id = cfg;
     B->smem = sm;
@@ -491,9 +515,9 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
     best_ms = 1e30;
     for (int c : cands)
       for (int sched = 0; sched < 2; ++sched) {
-        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, false, &smem))) return fail(rc);
+        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, false, c == cands.back(), &smem))) return fail(rc);
         if (smem > (size_t)smem_max) continue;
-        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, true, &smem)) || (rc = set_cfg(c, smem)))
+        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, true, c == cands.back(), &smem)) || (rc = set_cfg(c, smem)))
           return fail(rc);
         if ((rc = enqueue_device_work(B, st, true))) return fail(rc);  // warm-up
         cudaEventRecord(B->ev[0], st);
@@ -503,7 +527,7 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
         const double ms = event_ms(B->ev[0], B->ev[1]);
         if (ms < best_ms) { best_ms = ms; best_cfg = c; best_sched = sched; }
       }
-    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, best_cfg, best_sched, true, &smem)) ||
+    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, best_cfg, best_sched, true, best_cfg == cands.back(), &smem)) ||
         (rc = set_cfg(best_cfg, smem)))
       return fail(rc);
   }

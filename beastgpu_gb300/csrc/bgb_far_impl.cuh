@@ -37,8 +37,6 @@ constexpr float kPiA = 6.28125f;
 constexpr float kPiB = (float)(kTwoPi - 6.28125);
 constexpr float kPiC = (float)(kTwoPi - 6.28125 - (double)(float)(kTwoPi - 6.28125));
 constexpr float kInv2Pi = (float)(1.0 / kTwoPi);
-constexpr int kThreads = 256;
-
 // Hardware approximations (PTX .approx with flush-to-zero).  Their arguments in the FP32 pair loop
 // are normal numbers (squared distances, sums of distances, phases within a few pi), so the
 // denormal handling that the non-flushing forms add to each call is dead weight there.
@@ -112,7 +110,7 @@ struct Off64 {
 struct PMixed {
   using R = float;
   using C = float2;
-  static constexpr int kMinBlocks = 3;  // 3 CTAs of 256 threads per SM (<= 85 registers)
+  static constexpr int kThreads = 256, kMinBlocks = 3;  // 24 warps per SM (<= 85 registers)
   template <int Q>
   static constexpr int rec() { return Q <= 4 ? kRec34F : Off32<Q>::SIZE; }
   static __device__ __forceinline__ C mk(double a, double b) { return make_float2((float)a, (float)b); }
@@ -120,7 +118,7 @@ struct PMixed {
 struct PFp64 {
   using R = double;
   using C = double2;
-  static constexpr int kMinBlocks = 1;
+  static constexpr int kThreads = 256, kMinBlocks = 1;
   template <int Q>
   static constexpr int rec() { return Q <= 4 ? kRec34D : Off64<Q>::SIZE; }
   static __device__ __forceinline__ C mk(double a, double b) { return make_double2(a, b); }
@@ -752,12 +750,20 @@ __device__ __forceinline__ int64_t find_sigma(const int64_t* __restrict__ off, c
 // ----------------------------------------------------------------------------------------
 // Tile kernel
 // ----------------------------------------------------------------------------------------
+// A support of a trial function in a chunk: its offset in a pair's local matrices, its coefficient.
+template <class R>
+struct Support {
+  int col;
+  R w;
+};
+
 template <class P>
 struct Smem {
   float4* bndT;
   float4* bndB;
   int* triT;
   int* triB;
+  int* row;        // output row of each test function
   typename P::R* recT;
   typename P::R* recB;
   int* fcnt;
@@ -765,22 +771,19 @@ struct Smem {
   typename P::R* fcoef;
   typename P::C* Lbuf;
   typename P::C* Zs;
-  int* grpFn;      // per group of the trial block: local function
-  int* grpOff;     // per group: first support (block-relative), plus one end marker per chunk
+  int2* grp;       // per group of the trial block: offset of its function in Zs, first support << 5 | count
   int* chGrp;      // per chunk: first group (block-relative)
-  int* gsCode;
-  typename P::R* gsCoef;
+  Support<typename P::R>* gs;
 };
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Trial records staged per chunk (two chunk buffers, the next copied in while the current one is
-// computed) instead of per tile: for the FP32 Lagrange kernels, whose ~6-support hats make wide
-// trial blocks, the freed shared memory keeps more test triangles per tile (the d = 40 cube: 3%
-// faster); the RWG kernels keep per-tile staging (3% faster there: no copy per chunk, no spills).
-template <class P, int OP>
+// computed) instead of per tile: for the large records of the generic FP32 rules on Lagrange spaces,
+// whose ~6-support hats make wide trial blocks.
+template <class P, int OP, int QB>
 __host__ __device__ constexpr bool chunk_trial_records() {
-  return sizeof(typename P::R) == 4 && is_lagrange_op(OP);
+  return sizeof(typename P::R) == 4 && is_lagrange_op(OP) && QB > 4;
 }
 
 template <class P>
@@ -799,6 +802,7 @@ __host__ __device__ inline size_t carve(unsigned char* base, int tmax, int nmax,
   p = take(sizeof(float4) * nmax); if (s) s->bndB = (float4*)p;
   p = take(sizeof(int) * tmax); if (s) s->triT = (int*)p;
   p = take(sizeof(int) * nmax); if (s) s->triB = (int*)p;
+  p = take(sizeof(int) * FM); if (s) s->row = (int*)p;
   p = take(sizeof(R) * (size_t)tmax * rt); if (s) s->recT = (R*)p;
   p = take(sizeof(R) * (size_t)(chunk_recb ? 2 * SC : nmax) * rb); if (s) s->recB = (R*)p;
   p = take(sizeof(int) * FM); if (s) s->fcnt = (int*)p;
@@ -807,11 +811,9 @@ __host__ __device__ inline size_t carve(unsigned char* base, int tmax, int nmax,
   p = take(sizeof(C) * 9 * (size_t)tmax * SC); if (s) s->Lbuf = (C*)p;
   p = take(sizeof(C) * (size_t)FM * FN); if (s) s->Zs = (C*)p;
   const int nch = (nmax + SC - 1) / SC;
-  p = take(sizeof(int) * (size_t)gmax); if (s) s->grpFn = (int*)p;
-  p = take(sizeof(int) * (size_t)(gmax + 1)); if (s) s->grpOff = (int*)p;
+  p = take(sizeof(int2) * (size_t)gmax); if (s) s->grp = (int2*)p;
   p = take(sizeof(int) * (size_t)(nch + 1)); if (s) s->chGrp = (int*)p;
-  p = take(sizeof(int) * (size_t)gsmax); if (s) s->gsCode = (int*)p;
-  p = take(sizeof(R) * (size_t)gsmax); if (s) s->gsCoef = (R*)p;
+  p = take(sizeof(Support<R>) * (size_t)gsmax); if (s) s->gs = (Support<R>*)p;
   return off;
 }
 
@@ -831,11 +833,12 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
   using C = typename P::C;
   constexpr int RT = P::template rec<QT>();
   constexpr int RB = P::template rec<QB>();
+  constexpr int kThreads = P::kThreads;
   const int tid = threadIdx.x;
   const FarScalars S = far_scalars(K);  // registers, not shared-memory loads in the pair loop
   const int SC = p.SC, MAXS = p.MAXS;
   Smem<P> s;
-  constexpr bool kChunkB = chunk_trial_records<P, OP>();
+  constexpr bool kChunkB = chunk_trial_records<P, OP, QB>();
   carve<P>(smem, p.tmax, p.nmax, RT, RB, p.FM, p.FN, MAXS, SC, p.gmax, p.gsmax, kChunkB, &s);
 
   const int t0 = p.tb_off[bm], tm = p.tb_off[bm + 1] - t0;
@@ -879,12 +882,13 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
   }
   const bool f32 = sizeof(R) == 4;
   // local matrices of a chunk: entry (i, j) of pair (ti, si) at Lbuf[(i * 3 + j) * LS + ti * SC + si];
-  // supports are staged as their offsets in it (test: (i * 3) * LS + ti * SC, trial: j * LS + slot)
+  // supports are staged as their offsets in it (test: (i * 3) * LS + ti * SC, trial: j * LS + si)
   const int LS = p.tmax * SC;
   for (int m = tid; m < fm; m += kThreads) {
     const int a0 = p.fs_off[f0 + m], a1 = p.fs_off[f0 + m + 1];
     const int cnt = min(a1 - a0, MAXS);
     s.fcnt[m] = cnt;
+    s.row[m] = (int)p.rows[f0 + m];
     for (int k = 0; k < cnt; ++k) {
       const int fc = p.fs_code[a0 + k];  // test triangle << 2 | local
       s.fcode[m * MAXS + k] = (fc & 3) * 3 * LS + (fc >> 2) * SC;
@@ -892,19 +896,18 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
     }
   }
   // the trial block's gather groups (all chunks), block-relative
-  const int c0 = p.bb_chunk_off[bn], c1 = p.bb_chunk_off[bn + 1];
-  const int gb0 = p.ch_grp_off[c0], gb1 = p.ch_grp_off[c1];
+  const int c0 = p.bb_chunk_off[bn], nch = p.bb_chunk_off[bn + 1] - c0;
+  const int gb0 = p.ch_grp_off[c0], gb1 = p.ch_grp_off[c0 + nch];
   const int sb0 = p.grp_sup_off[gb0], sb1 = p.grp_sup_off[gb1];
   for (int i = tid; i < gb1 - gb0; i += kThreads) {
-    s.grpFn[i] = p.grp_fn[gb0 + i];
-    s.grpOff[i] = p.grp_sup_off[gb0 + i] - sb0;
+    const int q0 = p.grp_sup_off[gb0 + i], q1 = p.grp_sup_off[gb0 + i + 1];  // at most SC <= 16 supports
+    s.grp[i] = make_int2(p.grp_fn[gb0 + i] * fm, (q0 - sb0) << 5 | (q1 - q0));
   }
-  if (tid == 0) s.grpOff[gb1 - gb0] = sb1 - sb0;
-  for (int i = tid; i <= c1 - c0; i += kThreads) s.chGrp[i] = p.ch_grp_off[c0 + i] - gb0;
+  for (int i = tid; i <= nch; i += kThreads) s.chGrp[i] = p.ch_grp_off[c0 + i] - gb0;
   for (int i = tid; i < sb1 - sb0; i += kThreads) {
     const int code = p.gs_code[sb0 + i];  // trial slot << 2 | local
-    s.gsCode[i] = (code & 3) * LS + (code >> 2);
-    s.gsCoef[i] = f32 ? (R)p.gs_coef32[sb0 + i] : (R)p.gs_coef[sb0 + i];
+    s.gs[i].col = (code & 3) * LS + (code >> 2) % SC;
+    s.gs[i].w = f32 ? (R)p.gs_coef32[sb0 + i] : (R)p.gs_coef[sb0 + i];
   }
   for (int i = tid; i < fm * fn; i += kThreads) s.Zs[i] = P::mk(0.0, 0.0);
   if (tid == 0) *s_nonfar = 0;
@@ -954,127 +957,139 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
     const float lim = 1.001f * (A.w + B.w) + 1e-5f * mag + 1e-30f;
     blocks_apart = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > lim * lim;  // false for NaN: scan
   }
-  for (int i = tid; i < (blocks_apart ? 0 : tm); i += kThreads) {
-    const int T = s.triT[i];
-    for (int64_t e = p.sing_off[T], e1 = p.sing_off[T + 1]; e < e1; ++e) {
-      const int sg = p.sing_sigma[e];
-      int lo = 0, hi = nbk;  // triB is sorted ascending
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (s.triB[mid] < sg) lo = mid + 1;
-        else hi = mid;
-      }
-      if (lo < nbk && s.triB[lo] == sg) {
-        *s_nonfar = 1;
-        break;
+  bool check = false;
+  if (!blocks_apart) {  // the same in every thread
+    for (int i = tid; i < tm; i += kThreads) {
+      const int T = s.triT[i];
+      for (int64_t e = p.sing_off[T], e1 = p.sing_off[T + 1]; e < e1; ++e) {
+        const int sg = p.sing_sigma[e];
+        int lo = 0, hi = nbk;  // triB is sorted ascending
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (s.triB[mid] < sg) lo = mid + 1;
+          else hi = mid;
+        }
+        if (lo < nbk && s.triB[lo] == sg) {
+          *s_nonfar = 1;
+          break;
+        }
       }
     }
+    __syncthreads();
+    check = *s_nonfar != 0;
   }
-  // fixed roles of this thread: pair (ti0 + k * tstep, si) of a chunk; gather row m, groups gq + k * gstep
+  // fixed roles of this thread: pairs (ti0 + k * tstep, si) of a chunk; gather row m, groups gq + k * gstep
   const int tstep = kThreads / SC, ti0 = tid / SC, si = tid - ti0 * SC;
   // gather rows in whole warps (one group stream per warp) when that keeps the groups in flight
   const int FM32 = (p.FM + 31) & ~31;
   const int FMb = kThreads / FM32 == kThreads / p.FM ? FM32 : p.FM;
   const int gstep = kThreads / FMb, gq = tid / FMb, m = tid - gq * FMb;
   const bool gather_on = m < fm && gq < gstep;
-  __syncthreads();
-  const bool check = *s_nonfar != 0;
-
-  for (int c = c0; c < c1; ++c) {
-    const int sbase = (c - c0) * SC;
-    const int scn = min(SC, nbk - sbase);
-    const R* __restrict__ recb = s.recB;  // this chunk's trial records (kChunkB: one of two buffers)
-    if constexpr (kChunkB) {
-      constexpr int RB4 = RB / 4;
-      recb = s.recB + ((c - c0) & 1) * SC * RB;
-      const int nn = c + 1 < c1 ? min(SC, nbk - sbase - SC) : 0;  // the next chunk's records
-      if (tid < nn * RB4) {
-        const int r = tid / RB4, k = tid - r * RB4;
-        cp_async16(s.recB + ((((c + 1 - c0) & 1) * SC + r) * RB + 4 * k),
-                   (const float4*)gRB + (int64_t)s.triB[sbase + SC + r] * RB4 + k);
+  // this row's test supports: two (RWG) in registers
+  int cnt = 0, fcA = 0, fcB = 0;
+  R fwA = 0, fwB = 0;
+  if (gather_on) {
+    cnt = s.fcnt[m];
+    if (MAXS <= 2) {
+      if (cnt > 0) {
+        fcA = s.fcode[m * MAXS];
+        fwA = s.fcoef[m * MAXS];
       }
-      cp_async_commit();
+      if (cnt > 1) {
+        fcB = s.fcode[m * MAXS + 1];
+        fwB = s.fcoef[m * MAXS + 1];
+      }
     }
-    if (si < scn) {
-      const int sb = sbase + si;
-      for (int ti = ti0; ti < tm; ti += tstep) {
-        C L[9];
-        bool done = false;
-        if (check && sphere_candidate(s.bndT[ti], s.bndB[sb])) {
-          const int64_t e = find_sigma(p.sing_off, p.sing_sigma, s.triT[ti], s.triB[sb]);
-          if (e >= 0) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-              const double2 v = p.sing_L[e * 9 + k];
-              L[k] = P::mk(v.x, v.y);
-            }
-            done = true;
-          }
+  }
+
+  for (int c = 0; c < nch; ++c) {
+    {
+      const int sbase = c * SC;
+      const int scn = min(SC, nbk - sbase);
+      C* __restrict__ Lb = s.Lbuf;
+      const R* __restrict__ recb = s.recB + (kChunkB ? (c & 1) * SC * RB : sbase * RB);  // this chunk's trial records
+      if constexpr (kChunkB) {
+        constexpr int RB4 = RB / 4;
+        const int nn = c + 1 < nch ? min(SC, nbk - sbase - SC) : 0;  // the next chunk's records
+        for (int i = tid; i < nn * RB4; i += kThreads) {
+          const int r = i / RB4, k = i - r * RB4;
+          cp_async16(s.recB + ((((c + 1) & 1) * SC + r) * RB + 4 * k),
+                     (const float4*)gRB + (int64_t)s.triB[sbase + SC + r] * RB4 + k);
         }
-        if (!done)
-          far_pair<P, OP, QT, QB>(S, K, s.recT + ti * RT, kChunkB ? recb + si * RB : s.recB + sb * RB, L);
-        const int li = ti * SC + si;
+        cp_async_commit();
+      }
+      if (si < scn) {
+        const int sb = sbase + si;
+        for (int ti = ti0; ti < tm; ti += tstep) {
+          C L[9];
+          bool done = false;
+          if (check && sphere_candidate(s.bndT[ti], s.bndB[sb])) {
+            const int64_t e = find_sigma(p.sing_off, p.sing_sigma, s.triT[ti], s.triB[sb]);
+            if (e >= 0) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) s.Lbuf[k * LS + li] = L[k];
+              for (int k = 0; k < 9; ++k) {
+                const double2 v = p.sing_L[e * 9 + k];
+                L[k] = P::mk(v.x, v.y);
+              }
+              done = true;
+            }
+          }
+          if (!done) far_pair<P, OP, QT, QB>(S, K, s.recT + ti * RT, recb + si * RB, L);
+          const int li = ti * SC + si;
+#pragma unroll
+          for (int k = 0; k < 9; ++k) Lb[k * LS + li] = L[k];
+        }
       }
     }
     if constexpr (kChunkB) cp_async_wait_all();  // the next chunk's records, before the barrier
     __syncthreads();
     if (gather_on) {
-      const int gg0 = s.chGrp[c - c0], ng = s.chGrp[c - c0 + 1] - gg0;
-      // this row's test supports (two for RWG) in registers for the chunk
-      const int cnt = s.fcnt[m];
-      int fcA = 0, fcB = 0;
-      R fwA = 0, fwB = 0;
-      if (MAXS <= 2) {
-        fcA = s.fcode[m * MAXS];
-        fwA = s.fcoef[m * MAXS];
-        if (cnt > 1) {
-          fcB = s.fcode[m * MAXS + 1];
-          fwB = s.fcoef[m * MAXS + 1];
-        }
-      }
-      for (int g = gq; g < ng; g += gstep) {
-        const int gi = gg0 + g;
-        const int n = s.grpFn[gi];
-        C acc = s.Zs[n * fm + m];
-        const int q0 = s.grpOff[gi], q1 = s.grpOff[gi + 1];
-        for (int bsup = q0; bsup < q1; ++bsup) {
-          const int col = s.gsCode[bsup] - sbase;
-          const R cb = s.gsCoef[bsup];
+      const C* __restrict__ Lb = s.Lbuf;
+      const int gg1 = s.chGrp[c + 1];
+      for (int g = s.chGrp[c] + gq; g < gg1; g += gstep) {
+        const int2 G = s.grp[g];
+        C* z = s.Zs + G.x + m;
+        C acc = *z;
+        const Support<R>* __restrict__ q = s.gs + (G.y >> 5);
+        const Support<R>* __restrict__ q1 = q + (G.y & 31);
+        for (; q != q1; ++q) {
+          const Support<R> u = *q;
           if (MAXS <= 2) {
-            {
-              const R w = fwA * cb;
-              const C l = s.Lbuf[fcA + col];
+            if (cnt > 0) {
+              const R w = fwA * u.w;
+              const C l = Lb[fcA + u.col];
               acc.x = fma(w, l.x, acc.x);
               acc.y = fma(w, l.y, acc.y);
             }
             if (cnt > 1) {
-              const R w = fwB * cb;
-              const C l = s.Lbuf[fcB + col];
+              const R w = fwB * u.w;
+              const C l = Lb[fcB + u.col];
               acc.x = fma(w, l.x, acc.x);
               acc.y = fma(w, l.y, acc.y);
             }
           } else {
             for (int a = 0; a < cnt; ++a) {
-              const R w = s.fcoef[m * MAXS + a] * cb;
-              const C l = s.Lbuf[s.fcode[m * MAXS + a] + col];
+              const R w = s.fcoef[m * MAXS + a] * u.w;
+              const C l = Lb[s.fcode[m * MAXS + a] + u.col];
               acc.x = fma(w, l.x, acc.x);
               acc.y = fma(w, l.y, acc.y);
             }
           }
         }
-        s.Zs[n * fm + m] = acc;
+        *z = acc;
       }
     }
     __syncthreads();
   }
-  for (int i = tid; i < fm * fn; i += kThreads) {
-    const int n = i / fm, m = i - n * fm;
-    const int64_t idx = p.rows[f0 + m] + p.cols[g0 + n] * p.ld;
-    const C v = s.Zs[i];
-    if (p.out_c64) ((double2*)p.out)[idx] = make_double2(v.x, v.y);
-    else ((float2*)p.out)[idx] = make_float2((float)v.x, (float)v.y);
+  // output columns by warps, rows by lanes
+  for (int n = tid >> 5; n < fn; n += kThreads / 32) {
+    const int64_t col = p.cols[g0 + n] * p.ld;
+    for (int mm = tid & 31; mm < fm; mm += 32) {
+      const C v = s.Zs[n * fm + mm];
+      const int64_t idx = col + s.row[mm];
+      if (p.out_c64) ((double2*)p.out)[idx] = make_double2(v.x, v.y);
+      else ((float2*)p.out)[idx] = make_float2((float)v.x, (float)v.y);
+    }
   }
 }
 
@@ -1086,7 +1101,7 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
 // when a CTA's tile belongs to another problem than its previous one; each CTA claims its next
 // tile when it starts a tile.
 template <class P, int OP, int QT, int QB>
-__global__ void __launch_bounds__(kThreads, P::kMinBlocks) k_far_persistent(const FarConst* __restrict__ Ks,
+__global__ void __launch_bounds__(P::kThreads, P::kMinBlocks) k_far_persistent(const FarConst* __restrict__ Ks,
                                                              const TilePlan* __restrict__ plans,
                                                              const int4* __restrict__ items, int nitems,
                                                              int* __restrict__ counter,
@@ -1110,9 +1125,9 @@ __global__ void __launch_bounds__(kThreads, P::kMinBlocks) k_far_persistent(cons
       it = make_int4(0, t % ntb, t / ntb, 0);
     }
     if (it.x != cur) {
-      for (int i = threadIdx.x; i < (int)(sizeof(FarConst) / 4); i += kThreads)
+      for (int i = threadIdx.x; i < (int)(sizeof(FarConst) / 4); i += P::kThreads)
         ((int*)&sK)[i] = ((const int*)&Ks[it.x])[i];
-      for (int i = threadIdx.x; i < (int)(sizeof(TilePlan) / 4); i += kThreads)
+      for (int i = threadIdx.x; i < (int)(sizeof(TilePlan) / 4); i += P::kThreads)
         ((int*)&sP)[i] = ((const int*)&plans[it.x])[i];
       cur = it.x;
     }
@@ -1291,7 +1306,7 @@ int launch_persistent_t(const FarConst* Ks, const TilePlan* plans, const int4* i
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic_smem(kern));
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(far persistent)");
   if (nitems <= 0) return 0;
-  kern<<<ctas, kThreads, smem_bytes, st>>>(Ks, plans, items, nitems, counter, abort_flag);
+  kern<<<ctas, P::kThreads, smem_bytes, st>>>(Ks, plans, items, nitems, counter, abort_flag);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "k_far_persistent launch");
 }
@@ -1301,14 +1316,15 @@ int occupancy_t(size_t smem_bytes, int* per_sm) {
   cudaError_t e = cudaFuncSetAttribute(k_far_persistent<P, OP, QT, QB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        max_dynamic_smem(k_far_persistent<P, OP, QT, QB>));
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(far persistent)");
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_far_persistent<P, OP, QT, QB>, kThreads, smem_bytes);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_far_persistent<P, OP, QT, QB>, P::kThreads,
+                                                    smem_bytes);
   return e == cudaSuccess ? 0 : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
 }
 
 template <class P, int OP, int QT, int QB>
 size_t smem_t(const TilePlan& p) {
   return carve<P>(nullptr, p.tmax, p.nmax, P::template rec<QT>(), P::template rec<QB>(), p.FM, p.FN, p.MAXS, p.SC,
-                  p.gmax, p.gsmax, chunk_trial_records<P, OP>(), nullptr);
+                  p.gmax, p.gsmax, chunk_trial_records<P, OP, QB>(), nullptr);
 }
 
 template <class P, int OP, int QT, int QB>

@@ -118,6 +118,12 @@ struct HostPlan {
 struct TileCfg { int FM, FN, SC; };
 extern const TileCfg kTileCfgs[];
 extern const int kNumTileCfgs;
+// Drops the leading (widest) choices while they make fewer tiles than the chip has CTA slots: a small matrix
+// is bound by the time of one tile, which falls with the square of its width.
+template <class F>
+void narrow_for_size(std::vector<int>& prefs, int64_t slots, F tiles) {
+  while (prefs.size() > 1 && tiles(kTileCfgs[prefs[0]]) < slots) prefs.erase(prefs.begin());
+}
 extern const int kPrefMixed[];
 extern const int kNumPrefMixed;
 extern const int kPrefFp64[];
