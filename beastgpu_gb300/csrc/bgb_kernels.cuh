@@ -75,7 +75,7 @@ struct DfTables {
   int trig_off, total_floats;
   DfTrig trig;
   dfl gx[4][BGB_MAX_SS], gw[4][BGB_MAX_SS];
-  dfl ser[4][4][2 * BGB_SS_SERIES];
+  df2 ser[4][4][BGB_SS_SERIES];  // (cosine, sine) coefficients
 };
 void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M);
 // Per-triangle double-float geometry: vertices (df), area and 1 / area (df).

@@ -105,7 +105,9 @@ __global__ void k_chunk_bounds(const float4* __restrict__ b, int nb, float4* __r
 // vertex matching, pulledback_integrand_gpu.jl:41-51), and BGB_MASK_INEXACT.
 // ----------------------------------------------------------------------------------------
 __device__ int classify_exact(const Geo64& a, const Geo64& b, double k2, int* mask = nullptr) {
-  const double dtol = 2.220446049250313e-16 * 1.0e3;
+  // sqrt(d2) < dtol with dtol = 1000 eps: dtol^2 is exact (10^6 2^-104) and the least double whose rounded
+  // root reaches dtol, so the squares compare alike, without nine FP64 roots per pair
+  const double dtol = 2.220446049250313e-16 * 1.0e3, dtol2 = dtol * dtol;
   const double xtol2 = 0.2 * 0.2;
   int hits = 0, m = 0, inexact = 0;
   double dmin2 = 1.7976931348623157e308;  // floatmax(Float64)
@@ -117,7 +119,7 @@ __device__ int classify_exact(const Geo64& a, const Geo64& b, double k2, int* ma
       double dy = __dsub_rn(a.v[u1][1], b.v[u2][1]);
       double dz = __dsub_rn(a.v[u1][2], b.v[u2][2]);
       double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-      const bool hit = __dsqrt_rn(d2) < dtol;
+      const bool hit = d2 < dtol2;
       hits += hit;
       m |= (int)hit << (u1 * 3 + u2);
       inexact |= hit && __double_as_longlong(d2) != 0;  // an integer compare: the FP64 pipe is the bound

@@ -13,6 +13,7 @@
 // Bound by the FP32 pipe's issue.  One warp per pair; the per-lane sums are reduced through shared
 // memory (15 df additions per lane instead of 80), and nine lanes each form one entry in df.
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "bgb_df.cuh"
@@ -40,16 +41,6 @@ __device__ __forceinline__ dfl df_mulx(dfl a, dfl b) {
   float e = __fmaf_rn(a.hi, b.hi, -p);
   e = __fmaf_rn(a.hi, b.lo, e);
   return {p, __fmaf_rn(a.lo, b.hi, e)};
-}
-// a * b + c for |c| >= |a b|
-__device__ __forceinline__ dfl df_fma_big(dfl a, dfl b, dfl c) {
-  const dfl p = df_mulx(a, b);
-  float s, e;
-  df_fast_two_sum(c.hi, p.hi, s, e);
-  e = __fadd_rn(e, __fadd_rn(c.lo, p.lo));
-  dfl r;
-  df_fast_two_sum(s, e, r.hi, r.lo);
-  return r;
 }
 // c + a * b
 __device__ __forceinline__ dfl df_macc(dfl c, dfl a, dfl b) { return df_add(c, df_mulx(a, b)); }
@@ -181,23 +172,25 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
       J[k] = J[k] < 1 ? 1 : (J[k] > 3 ? 3 : J[k]);
     }
     dfl a1[3], a2[3], b1[3], b2[3];
-    float la = 0.f, lb = 0.f, l2 = 0.f, m2 = 0.f;
+    float dv[9] = {};  // squared distances between the ends of X and of Y
     for (int c = 0; c < 3; ++c) {
       a1[c] = df_sub(gdf(A.v[I[2] - 1][c]), gdf(A.v[I[0] - 1][c]));
       a2[c] = df_sub(gdf(A.v[I[1] - 1][c]), gdf(A.v[I[2] - 1][c]));
       b1[c] = df_sub(gdf(B.v[J[2] - 1][c]), gdf(B.v[J[0] - 1][c]));
       b2[c] = df_sub(gdf(B.v[J[1] - 1][c]), gdf(B.v[J[2] - 1][c]));
-      const float x = a1[c].hi, y = b1[c].hi, z = x + a2[c].hi, w = y + b2[c].hi;
-      la = fmaf(x, x, la);
-      lb = fmaf(y, y, lb);
-      l2 = fmaf(z, z, l2);
-      m2 = fmaf(w, w, m2);
+      const float u[3] = {0.f, a1[c].hi, a1[c].hi + a2[c].hi}, v[3] = {0.f, b1[c].hi, b1[c].hi + b2[c].hi};
+#pragma unroll
+      for (int q = 0; q < 9; ++q) dv[q] = fmaf(u[q / 3] - v[q % 3], u[q / 3] - v[q % 3], dv[q]);
     }
     const dfl kd = gdf(op.k);
-    // terms of the series (theta <= k (largest |X| + largest |Y|), on one face k times its edge): nd in df, then float ones to 2^-51
+    // terms of the series (theta <= k times the largest distance of two vertices): nd in df, then float ones
+    // to 2^-51
     int nd = 0, nj = 0;
     {
-      const float th = 1.0001f * fabsf(kd.hi) * (sqrtf(fmaxf(la, l2)) + (cls == BGB_CLASS_CF ? 0.f : sqrtf(fmaxf(lb, m2))));
+      float d2 = dv[0];
+#pragma unroll
+      for (int q = 1; q < 9; ++q) d2 = fmaxf(d2, dv[q]);
+      const float th = 1.0001f * fabsf(kd.hi) * sqrtf(d2);
       if (th <= 3.f) {
         float t = 1.f;
         do {
@@ -207,9 +200,9 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
         } while (t > 4e-16f && nj < BGB_SS_SERIES);
       }
     }
-    dfl acc[NV];
+    df2 acc[NA];  // (real, imaginary) moments
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = dfl{0.f, 0.f};
+    for (int k = 0; k < NA; ++k) acc[k] = df2{0ull, 0ull};
     const int cnt = M.cnt[cls];
     const float2* __restrict__ pt = (const float2*)(tab + M.ss_off[cls]);
     for (int idx = lane; idx < cnt; idx += 32) {
@@ -225,50 +218,41 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
       const dfl r2 = df_dot(d, d);
       const dfl rinv = df_rsqrt_step(r2);
       const dfl th = df_mul(kd, df_mulx(r2, rinv));
-      dfl C[3], S[3];  // T_m = C - i S, m = M0 .. M0 + 2
+      df2 T[3];  // (C, S) of T_m = C - i S, m = M0 .. M0 + 2
       if (nj > 0) {
-        const dfl th2 = df_mul(th, th);
-        const dfl(*__restrict__ ser)[2 * BGB_SS_SERIES] = M.ser[cls];
-        float c[3], s[3];
+        const dfl th2s = df_mul(th, th);
+        const df2 th2 = df2_both(th2s);
+        const df2(*__restrict__ ser)[BGB_SS_SERIES] = M.ser[cls];
+        unsigned long long t[3];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) c[q] = s[q] = 0.f;
+        for (int q = 0; q < 3; ++q) t[q] = 0ull;
         for (int k = nj - 1; k >= nd; --k) {
 #pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            c[q] = __fmaf_rn(c[q], th2.hi, ser[q + 1 + M0][2 * k].hi);
-            s[q] = __fmaf_rn(s[q], th2.hi, ser[q + 1 + M0][2 * k + 1].hi);
-          }
+          for (int q = 0; q < 3; ++q) t[q] = fma2(t[q], th2.hi, ser[q + 1 + M0][k].hi);
         }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          C[q] = dfl{c[q], 0.f};
-          S[q] = dfl{s[q], 0.f};
-        }
+        for (int q = 0; q < 3; ++q) T[q] = df2{t[q], 0ull};
         for (int k = nd - 1; k >= 1; --k) {
 #pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            C[q] = df_fma_big(C[q], th2, ser[q + 1 + M0][2 * k]);
-            S[q] = df_fma_big(S[q], th2, ser[q + 1 + M0][2 * k + 1]);
-          }
+          for (int q = 0; q < 3; ++q) T[q] = df2_fma_big(T[q], th2, ser[q + 1 + M0][k]);
         }
+        const df2 one_th = df2_of(dfl{1.f, 0.f}, th);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {  // the first two terms may be of either order
-          C[q] = df_macc(ser[q + 1 + M0][0], C[q], th2);
-          S[q] = df_mul(df_macc(ser[q + 1 + M0][1], S[q], th2), th);
-        }
+        for (int q = 0; q < 3; ++q)  // the first two terms may be of either order
+          T[q] = df2_mul(df2_macc(ser[q + 1 + M0][0], T[q], th2), one_th);
       } else {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) C[q] = S[q] = dfl{0.f, 0.f};
+        for (int q = 0; q < 3; ++q) T[q] = df2{0ull, 0ull};
         for (int l = 0; l < M.n[cls]; ++l) {
           dfl sn, cs;
           const dfl xi = M.gx[cls][l];
           df_sincos(df_mul(th, xi), trig, M.trig, sn, cs);
+          const df2 e2 = df2_of(cs, sn);
           dfl w = df_mul(M.gw[cls][l], xi);
           if (M0 == 0) w = df_mul(w, xi);
 #pragma unroll
           for (int q = 0; q < 3; ++q) {
-            C[q] = df_macc(C[q], w, cs);
-            S[q] = df_macc(S[q], w, sn);
+            T[q] = df2_macc(T[q], df2_both(w), e2);
             w = df_mul(w, xi);
           }
         }
@@ -277,42 +261,37 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
       if (OP == BGB_OP_MAXWELL3D_DL) {
         // (i k + 1/(xi R)) (C - i S): degree 2 (X x Y) from T_1, T_0 / R, degree 1 (X - Y) from T_0, T_-1 / R
         const dfl f = df_mul(g, rinv);
-        const dfl hr2 = df_mul(f, df_add(df_mulx(kd, S[2]), df_mulx(rinv, C[1])));
-        const dfl hi2 = df_mul(f, df_sub(df_mulx(kd, C[2]), df_mulx(rinv, S[1])));
-        const dfl hr1 = df_mul(f, df_add(df_mulx(kd, S[1]), df_mulx(rinv, C[0])));
-        const dfl hi1 = df_mul(f, df_sub(df_mulx(kd, C[1]), df_mulx(rinv, S[0])));
+        dfl c0, s0, c1, s1, c2, s2;
+        df2_parts(T[0], c0, s0);
+        df2_parts(T[1], c1, s1);
+        df2_parts(T[2], c2, s2);
+        const df2 kk = df2_both(kd), rr = df2_of(rinv, df_neg(rinv)), ff = df2_both(f);
+        const df2 h2 = df2_mul(ff, df2_add(df2_mulx(kk, df2_of(s2, c2)), df2_mulx(rr, T[1])));
+        const df2 h1 = df2_mul(ff, df2_add(df2_mulx(kk, df2_of(s1, c1)), df2_mulx(rr, T[0])));
         const dfl x[3] = {df_sub(df_mulx(X[1], Y[2]), df_mulx(X[2], Y[1])), df_sub(df_mulx(X[2], Y[0]), df_mulx(X[0], Y[2])),
                           df_sub(df_mulx(X[0], Y[1]), df_mulx(X[1], Y[0]))};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          acc[2 * c] = df_macc(acc[2 * c], hr2, x[c]);
-          acc[2 * c + 1] = df_macc(acc[2 * c + 1], hi2, x[c]);
-          acc[6 + 2 * c] = df_macc(acc[6 + 2 * c], hr1, d[c]);
-          acc[7 + 2 * c] = df_macc(acc[7 + 2 * c], hi1, d[c]);
+          acc[c] = df2_macc(acc[c], h2, df2_both(x[c]));
+          acc[3 + c] = df2_macc(acc[3 + c], h1, df2_both(d[c]));
         }
       } else if (OP == BGB_OP_MAXWELL3D_SL) {
-        const dfl xy = df_mul(g, df_dot(X, Y)), t1r = df_mul(g, C[1]), t1i = df_mul(df_neg(g), S[1]);
-        acc[0] = df_macc(acc[0], xy, C[2]);
-        acc[1] = df_macc(acc[1], xy, df_neg(S[2]));
+        const df2 gg = df2_of(g, df_neg(g)), t1 = df2_mul(gg, T[1]);
+        const dfl xy = df_mul(g, df_dot(X, Y));
+        acc[0] = df2_macc(acc[0], df2_of(xy, df_neg(xy)), T[2]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          acc[2 + 2 * c] = df_macc(acc[2 + 2 * c], t1r, X[c]);
-          acc[3 + 2 * c] = df_macc(acc[3 + 2 * c], t1i, X[c]);
-          acc[8 + 2 * c] = df_macc(acc[8 + 2 * c], t1r, Y[c]);
-          acc[9 + 2 * c] = df_macc(acc[9 + 2 * c], t1i, Y[c]);
+          acc[1 + c] = df2_macc(acc[1 + c], t1, df2_both(X[c]));
+          acc[4 + c] = df2_macc(acc[4 + c], t1, df2_both(Y[c]));
         }
-        acc[14] = df_macc(acc[14], g, C[0]);
-        acc[15] = df_macc(acc[15], g, df_neg(S[0]));
+        acc[7] = df2_macc(acc[7], gg, T[0]);
       } else {
-        dfl tr[3], ti[3];  // kernel sums of degree 0, 1, 2
+        const df2 gg = df2_of(g, df_neg(g));
+        df2 t[3];  // kernel sums of degree 0, 1, 2
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          tr[q] = df_mul(g, C[q]);
-          ti[q] = df_mul(df_neg(g), S[q]);
-        }
+        for (int q = 0; q < 3; ++q) t[q] = df2_mul(gg, T[q]);
         const dfl p[3] = {dfl{1.f, 0.f}, al, be}, q[3] = {dfl{1.f, 0.f}, ga, de};
-        acc[0] = df_add(acc[0], tr[0]);
-        acc[1] = df_add(acc[1], ti[0]);
+        acc[0] = df2_add(acc[0], t[0]);
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -320,14 +299,18 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
             if (a + b == 0) continue;
             const int deg = (a > 0) + (b > 0);
             const dfl pq = a == 0 ? q[b] : (b == 0 ? p[a] : df_mul(p[a], q[b]));
-            acc[2 * (3 * a + b)] = df_macc(acc[2 * (3 * a + b)], tr[deg], pq);
-            acc[2 * (3 * a + b) + 1] = df_macc(acc[2 * (3 * a + b) + 1], ti[deg], pq);
+            acc[3 * a + b] = df2_macc(acc[3 * a + b], t[deg], df2_both(pq));
           }
       }
     }
     // reduction: lane v (and v + 16 when 16 rows suffice) sums row v
 #pragma unroll
-    for (int k = 0; k < NV; ++k) part[wid][k][lane] = make_float2(acc[k].hi, acc[k].lo);
+    for (int k = 0; k < NA; ++k) {
+      dfl re, im;
+      df2_parts(acc[k], re, im);
+      part[wid][2 * k][lane] = make_float2(re.hi, re.lo);
+      part[wid][2 * k + 1][lane] = make_float2(im.hi, im.lo);
+    }
     __syncwarp();
     {
       const int v = lane & (NS - 1), h = NS == 16 ? (lane >> 4) * 16 : 0;
@@ -411,7 +394,12 @@ void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M) {
       M.gw[cls][l] = df(T.gw[cls][l]);
     }
     for (int m = 0; m < 4; ++m)
-      for (int k = 0; k < 2 * BGB_SS_SERIES; ++k) M.ser[cls][m][k] = df(T.ser[cls][m][k]);
+      for (int k = 0; k < BGB_SS_SERIES; ++k) {
+        const dfl c = df(T.ser[cls][m][2 * k]), s = df(T.ser[cls][m][2 * k + 1]);
+        const float hi[2] = {c.hi, s.hi}, lo[2] = {c.lo, s.lo};
+        std::memcpy(&M.ser[cls][m][k].hi, hi, sizeof(hi));
+        std::memcpy(&M.ser[cls][m][k].lo, lo, sizeof(lo));
+      }
   }
   align4();
   M.trig_off = (int)buf.size();

@@ -155,18 +155,19 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_ss64(OpParams op1, const OpP
     sub3(B.v[J[1] - 1], B.v[J[2] - 1], b2);
     if (OP == BGB_OP_HELMHOLTZ3D_DL) tri_unit_normal(B, nrm);
     if (OP == BGB_OP_HELMHOLTZ3D_DLT) tri_unit_normal(A, nrm);
-    // terms of the series: theta <= k (largest |X| + largest |Y|), on one face k times its edge; truncation below 2^-56
+    // terms of the series: theta <= k times the largest distance of two vertices, truncation below 2^-56
     int nj = 0;
     if (gre == 0.0) {
-      float la = 0.f, lb = 0.f, l2 = 0.f, m2 = 0.f;
+      float dv[9] = {};  // squared distances between the ends of X and of Y
       for (int c = 0; c < 3; ++c) {
-        const float x = (float)a1[c], y = (float)b1[c], z = x + (float)a2[c], w = y + (float)b2[c];
-        la = fmaf(x, x, la);
-        lb = fmaf(y, y, lb);
-        l2 = fmaf(z, z, l2);
-        m2 = fmaf(w, w, m2);
+        const float u[3] = {0.f, (float)a1[c], (float)(a1[c] + a2[c])}, v[3] = {0.f, (float)b1[c], (float)(b1[c] + b2[c])};
+#pragma unroll
+        for (int q = 0; q < 9; ++q) dv[q] = fmaf(u[q / 3] - v[q % 3], u[q / 3] - v[q % 3], dv[q]);
       }
-      const float th = 1.0001f * fabsf((float)gim) * (sqrtf(fmaxf(la, l2)) + (cls == BGB_CLASS_CF ? 0.f : sqrtf(fmaxf(lb, m2))));
+      float d2 = dv[0];
+#pragma unroll
+      for (int q = 1; q < 9; ++q) d2 = fmaxf(d2, dv[q]);
+      const float th = 1.0001f * fabsf((float)gim) * sqrtf(d2);
       if (th <= 3.f) {
         float t = 1.f;
         do {
