@@ -65,7 +65,7 @@ struct RulesDF {
   dfl gz[kMaxGraded], wcf[kMaxGraded], lnz[kMaxGraded];
   dfl gzc[kMaxGradedCv], wcv[kMaxGradedCv], lnzc[kMaxGradedCv];
   dfl sgx[kMaxSing], sgw[kMaxSing], gl2x[2], gl2w[2];
-  dfl sa[kSeries + 1], sb[kSeries];
+  df2 ab[kSeries + 1];  // (sa_m, sb_m), the last one (sa, 0)
   dfl inv2pi, two_over_pi;
 };
 
@@ -225,6 +225,39 @@ __device__ __forceinline__ void add_point(const Op& op, const SegGeo& A, const S
   accumulate<OP>(op, A, B, s, t, Kr, Ki, w, c);
 }
 
+// Sums of kernel x weight against 1, s, t, s t (real, imaginary), from which the shape products follow: 11
+// instead of 20 FP64 operations per point.
+struct Mom {
+  double r[4] = {0, 0, 0, 0}, i[4] = {0, 0, 0, 0};
+  __device__ __forceinline__ void add(double Kr, double Ki, double w, double s, double t) {
+    Kr *= w;
+    Ki *= w;
+    const double st = s * t;
+    r[0] += Kr;
+    i[0] += Ki;
+    r[1] = fma(Kr, s, r[1]);
+    i[1] = fma(Ki, s, i[1]);
+    r[2] = fma(Kr, t, r[2]);
+    i[2] = fma(Ki, t, i[2]);
+    r[3] = fma(Kr, st, r[3]);
+    i[3] = fma(Ki, st, i[3]);
+  }
+};
+// f = (1 - s, s) or 1, g = (1 - t, t) or 1; ll: the product of the lengths.
+__device__ __forceinline__ void moments_to_acc(const Op& op, const double r[4], const double i[4], double ll, Acc& c) {
+  const bool hA = op.nsA == 2, hB = op.nsB == 2;
+  c.pr[0] = ll * (r[0] - (hA ? r[1] : 0.0) - (hB ? r[2] : 0.0) + (hA && hB ? r[3] : 0.0));
+  c.pi[0] = ll * (i[0] - (hA ? i[1] : 0.0) - (hB ? i[2] : 0.0) + (hA && hB ? i[3] : 0.0));
+  c.pr[1] = ll * (r[2] - (hA ? r[3] : 0.0));
+  c.pi[1] = ll * (i[2] - (hA ? i[3] : 0.0));
+  c.pr[2] = ll * (r[1] - (hB ? r[3] : 0.0));
+  c.pi[2] = ll * (i[1] - (hB ? i[3] : 0.0));
+  c.pr[3] = ll * r[3];
+  c.pi[3] = ll * i[3];
+  c.mr = ll * r[0];
+  c.mi = ll * i[0];
+}
+
 // Adds kernel value K (times the rule weight and the lengths) times the shape products.
 template <int OP>
 __device__ __forceinline__ void accumulate(const Op& op, const SegGeo& A, const SegGeo& B, double s, double t,
@@ -300,6 +333,24 @@ __device__ __forceinline__ double point_seg_dist2(double px, double py, double a
 
 constexpr double kTwoOverPi = 0.6366197723675814, kEulerGamma = 0.5772156649015329;
 
+// Single-layer kernel from u = (k R / 2)^2 <= 4 (power series of J0, Y0 up to u^M; static for k = 0) and ln R.
+__device__ __forceinline__ void log_kernel(const Op& op, const Rules& Rl, double u, double lnR, int M, double& Kr, double& Ki) {
+  if (op.k == 0.0) {
+    Kr = -kInv2Pi * lnR;
+    Ki = 0.0;
+    return;
+  }
+  double j0 = Rl.sa[M], s0 = Rl.sb[M - 1];
+  j0 = fma(j0, u, Rl.sa[M - 1]);
+  for (int m = M - 2; m >= 0; --m) {
+    j0 = fma(j0, u, Rl.sa[m]);
+    s0 = fma(s0, u, Rl.sb[m]);
+  }
+  const double y0v = kTwoOverPi * fma(lnR + op.lnk2 + kEulerGamma, j0, s0 * u);
+  Kr = -0.25 * y0v;
+  Ki = -0.25 * j0;
+}
+
 // The kernel at distance R with ln R given, for the singular and near rules: power series of
 // J0, Y0 (J1, Y1) up to u^M for x = k R <= 4, CUDA's Bessel functions beyond; the static kernel
 // for k = 0.  The logarithm comes from the caller (for the graded rules it is a sum of tabulated
@@ -308,21 +359,9 @@ template <int OP>
 __device__ __forceinline__ void kernel_series(const Op& op, const Rules& Rl, double R, double lnR, int M, double rx,
                                               double ry, const SegGeo& A, const SegGeo& B, double& Kr, double& Ki) {
   if (OP == BGB_OP2D_SL || OP == BGB_OP2D_HS) {
-    if (op.k == 0.0) {
-      Kr = -kInv2Pi * lnR;
-      Ki = 0.0;
-      return;
-    }
     const double x = op.k * R;
     if (x <= 4.0) {
-      const double u = 0.25 * x * x;
-      double j0 = Rl.sa[M];
-      for (int m = M - 1; m >= 0; --m) j0 = fma(j0, u, Rl.sa[m]);
-      double s0 = Rl.sb[M - 1];
-      for (int m = M - 2; m >= 0; --m) s0 = fma(s0, u, Rl.sb[m]);
-      const double y0v = kTwoOverPi * fma(lnR + op.lnk2 + kEulerGamma, j0, s0 * u);
-      Kr = -0.25 * y0v;
-      Ki = -0.25 * j0;
+      log_kernel(op, Rl, 0.25 * x * x, lnR, M, Kr, Ki);
     } else {
       Kr = -0.25 * y0(x);
       Ki = -0.25 * j0(x);
@@ -393,6 +432,7 @@ __device__ void near_rule_warp(const Op& op, const Rules& R, const SegGeo& A, co
   stack[top++] = Box{0.0, 1.0, 0.0, 1.0, 0};
   const int n = R.nnear;
   const int M = series_order(op.k, max_vertex_distance(A, B));
+  Mom mo;
   while (top > 0) {
     const Box b = stack[--top];
     const double p0x = __dadd_rn(A.x0, __dmul_rn(b.s0, A.dx)), p0y = __dadd_rn(A.y0, __dmul_rn(b.s0, A.dy));
@@ -400,10 +440,14 @@ __device__ void near_rule_warp(const Op& op, const Rules& R, const SegGeo& A, co
     const double q0x = __dadd_rn(B.x0, __dmul_rn(b.t0, B.dx)), q0y = __dadd_rn(B.y0, __dmul_rn(b.t0, B.dy));
     const double q1x = __dadd_rn(B.x0, __dmul_rn(b.t1, B.dx)), q1y = __dadd_rn(B.y0, __dmul_rn(b.t1, B.dy));
     const double la = __dmul_rn(__dsub_rn(b.s1, b.s0), A.len), lb = __dmul_rn(__dsub_rn(b.t1, b.t0), B.len);
-    double d2 = point_seg_dist2(p0x, p0y, q0x, q0y, q1x, q1y);
-    d2 = fmin(d2, point_seg_dist2(p1x, p1y, q0x, q0y, q1x, q1y));
-    d2 = fmin(d2, point_seg_dist2(q0x, q0y, p0x, p0y, p1x, p1y));
-    d2 = fmin(d2, point_seg_dist2(q1x, q1y, p0x, p0y, p1x, p1y));
+    // the four end-to-piece distances, one per lane of each quad (an FP64 instruction costs the warp the same
+    // for one lane as for all)
+    const int e = lane & 3;
+    const bool ps = e < 2;
+    const double px = e == 0 ? p0x : (e == 1 ? p1x : (e == 2 ? q0x : q1x)), py = e == 0 ? p0y : (e == 1 ? p1y : (e == 2 ? q0y : q1y));
+    double d2 = point_seg_dist2(px, py, ps ? q0x : p0x, ps ? q0y : p0y, ps ? q1x : p1x, ps ? q1y : p1y);
+    d2 = fmin(d2, __shfl_xor_sync(0xffffffffu, d2, 1));
+    d2 = fmin(d2, __shfl_xor_sync(0xffffffffu, d2, 2));
     if (b.depth < kMaxDepth && __dsqrt_rn(d2) < fmax(la, lb)) {
       if (la >= lb) {
         const double sm = 0.5 * (b.s0 + b.s1);
@@ -421,12 +465,18 @@ __device__ void near_rule_warp(const Op& op, const Rules& R, const SegGeo& A, co
       const int p = k / n, q = k - p * n;
       const double s = b.s0 + hs * R.nr_x[p], t = b.t0 + ht * R.nr_x[q];
       const double rx = (A.x0 + s * A.dx) - (B.x0 + t * B.dx), ry = (A.y0 + s * A.dy) - (B.y0 + t * B.dy);
-      const double Rd = sqrt(rx * rx + ry * ry);
+      const double R2 = rx * rx + ry * ry;
       double Kr, Ki;
-      kernel_series<OP>(op, R, Rd, log(Rd), M, rx, ry, A, B, Kr, Ki);
-      accumulate<OP>(op, A, B, s, t, Kr, Ki, (hs * R.nr_w[p]) * (ht * R.nr_w[q]), c);
+      if ((OP == BGB_OP2D_SL || OP == BGB_OP2D_HS) && 0.25 * op.k2 * R2 <= 4.0) {
+        log_kernel(op, R, 0.25 * op.k2 * R2, 0.5 * log(R2), M, Kr, Ki);  // no root: the series is in R^2
+      } else {
+        const double Rd = sqrt(R2);
+        kernel_series<OP>(op, R, Rd, log(Rd), M, rx, ry, A, B, Kr, Ki);
+      }
+      mo.add(Kr, Ki, (hs * R.nr_w[p]) * (ht * R.nr_w[q]), s, t);
     }
   }
+  moments_to_acc(op, mo.r, mo.i, A.len * B.len, c);
 }
 
 // Coincident (match 0: same orientation, 1: reversed) and common-vertex rules: the chart square
@@ -436,6 +486,7 @@ __device__ void singular_rule_warp(const Op& op, const Rules& R, const SegGeo& A
                                    int match, int lane, double* __restrict__ wtab, Acc& c) {
   const int n = R.nsing, nz = R.ngraded;
   const int M = series_order(op.k, max_vertex_distance(A, B));
+  Mom mo;
   if (cls == 3) {
     if (OP == BGB_OP2D_DL || OP == BGB_OP2D_DLT) return;  // r lies along the segment
     const bool same = match == 0;
@@ -453,8 +504,9 @@ __device__ void singular_rule_warp(const Op& op, const Rules& R, const SegGeo& A
       const double wt = R.gwz[a] * R.gl2_w[b] * (1.0 - z);
       double Kr, Ki;
       kernel_series<OP>(op, R, z * A.len, R.lnz[a] + lnl, M, uv * A.dx, uv * A.dy, A, B, Kr, Ki);
-      accumulate<OP>(op, A, B, u, same ? v : 1.0 - v, Kr, Ki, wt, c);
+      mo.add(Kr, Ki, wt, u, same ? v : 1.0 - v);
     }
+    moments_to_acc(op, mo.r, mo.i, A.len * B.len, c);
     return;
   }
   const int ma = match >> 1, mb = match & 1;
@@ -485,8 +537,9 @@ __device__ void singular_rule_warp(const Op& op, const Rules& R, const SegGeo& A
     double Kr, Ki;
     kernel_series<OP>(op, R, z * tb[b], R.lnz_cv[a] + tb[kMaxSing + b], M, xi * ax - eta * bx, xi * ay - eta * by, A,
                       B, Kr, Ki);
-    accumulate<OP>(op, A, B, ma == 0 ? xi : 1.0 - xi, mb == 0 ? eta : 1.0 - eta, Kr, Ki, wt, c);
+    mo.add(Kr, Ki, wt, ma == 0 ? xi : 1.0 - xi, mb == 0 ? eta : 1.0 - eta);
   }
+  moments_to_acc(op, mo.r, mo.i, A.len * B.len, c);
   __syncwarp();
 }
 
@@ -513,14 +566,29 @@ __device__ __forceinline__ float horner(const float (&c)[N], float u) {
 
 constexpr float kTwoOverPiF = 0.636619772f, kInv2PiF = 0.159154943f, kTwoPiF = 6.28318531f;
 
-// sin / cos of an angle within a few multiples of pi, reduced to [-pi, pi] first.
-__device__ __forceinline__ void sincos_reduced(float th, float* s, float* c) {
-  th = fmaf(-kTwoPiF, rintf(th * kInv2PiF), th);
-  __sincosf(th, s, c);
+// Hardware approximations with flush-to-zero: their arguments here are normal numbers.
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
-// G = -(i/4) H0^(2)(x) with x = k R; phi equals x modulo 2 pi (carried in FP64 by the caller).
-__device__ __forceinline__ void hankel0_mixed(float x, float phi, float& Gr, float& Gi) {
+// sin / cos of an angle within a few multiples of pi, reduced to [-pi, pi] first.  The nearest integer by
+// adding and subtracting 1.5 2^23: FP32-pipe operations, where rintf takes the pipe of sin and cos.
+__device__ __forceinline__ void sincos_reduced(float th, float* s, float* c) {
+  const float n = __fsub_rn(__fmaf_rn(th, kInv2PiF, 12582912.f), 12582912.f);
+  th = __fmaf_rn(-kTwoPiF, n, th);
+  asm("sin.approx.ftz.f32 %0, %1;" : "=f"(*s) : "f"(th));
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(*c) : "f"(th));
+}
+
+// G = -(i/4) H0^(2)(x) with x = k R, t = 3 / x; phi equals x modulo 2 pi.
+__device__ __forceinline__ void hankel0_mixed(float x, float t, float phi, float& Gr, float& Gi) {
   if (x < 3.f) {
     const float u = x * x * (1.f / 9.f);
     const float j0 = horner(c_P0, u);
@@ -528,17 +596,16 @@ __device__ __forceinline__ void hankel0_mixed(float x, float phi, float& Gr, flo
     Gr = -0.25f * y0;
     Gi = -0.25f * j0;
   } else {
-    const float t = __fdividef(3.f, x);
-    const float amp = horner(c_F0, t) * rsqrtf(x);
+    const float amp = -0.25f * horner(c_F0, t) * rsqrt_ftz(x);
     float sn, cs;
     sincos_reduced(phi - 0.785398163f + horner(c_G0, t), &sn, &cs);
-    Gr = -0.25f * amp * sn;
-    Gi = -0.25f * amp * cs;
+    Gr = amp * sn;
+    Gi = amp * cs;
   }
 }
 
-// g1 = (i k / 4) H1^(2)(x) / R = (k / 4R) (Y1 + i J1); phi as for hankel0_mixed.
-__device__ __forceinline__ void hankel1_mixed(float x, float phi, float k_over_4R, float& gr, float& gi) {
+// g1 = (i k / 4) H1^(2)(x) / R = (k / 4R) (Y1 + i J1); t and phi as for hankel0_mixed.
+__device__ __forceinline__ void hankel1_mixed(float x, float t, float phi, float k_over_4R, float& gr, float& gi) {
   if (x < 3.f) {
     const float u = x * x * (1.f / 9.f);
     const float j1 = x * horner(c_P1, u);
@@ -546,8 +613,7 @@ __device__ __forceinline__ void hankel1_mixed(float x, float phi, float k_over_4
     gr = k_over_4R * y1;
     gi = k_over_4R * j1;
   } else {
-    const float t = __fdividef(3.f, x);
-    const float amp = horner(c_F1, t) * rsqrtf(x) * k_over_4R;
+    const float amp = horner(c_F1, t) * rsqrt_ftz(x) * k_over_4R;
     float sn, cs;
     sincos_reduced(phi - 2.35619449f + horner(c_G1, t), &sn, &cs);
     gr = amp * sn;
@@ -555,11 +621,6 @@ __device__ __forceinline__ void hankel1_mixed(float x, float phi, float k_over_4
   }
 }
 
-// Far pair in mixed precision.  Per pair in FP64: midpoint separation D, R0 = |D| and the phase
-// k R0 reduced modulo 2 pi.  Per point pair in FP32: w = (point offsets from the midpoints),
-// R = |D + w|, delta = R - R0 = (2 D.w + w.w) / (R + R0) without cancellation, x = k R and
-// phase phi0 + k delta.  The trial sums of each test point are formed first (moments S_j), then spread
-// over the test shapes.
 struct FAcc {
   float pr[4], pi[4], mr, mi;
 };
@@ -580,26 +641,35 @@ __device__ __forceinline__ float reduce_2pi(dfl K) {
 // w = point offsets from the midpoints, R = |D + w|, delta = R - R0 = (2 D.w + w.w) / (R + R0)
 // without cancellation, x = k R and phase phi0 + k delta.  The trial sums of each test point are
 // formed first (moments S_j), then spread over the test shapes.
-template <int OP>
-__device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, const float* fw, int nft,
-                                               const float* bx, const float* bw, int nfb, const SegF& A,
+// Bound by FP32 issue and the transcendental pipe (5 of its operations and ~42 others per point pair): the
+// default 4 x 4 rule is unrolled (NT, NB; 0: runtime counts), so nodes, weights and trial offsets stay in
+// registers, and 3 / x is a product with 1 / R.  8,192 segments: far stage 4.97 ms with runtime loops, divisions
+// and rintf.
+template <int OP, int NT, int NB>
+__device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, const float* fw, int nft_,
+                                               const float* bx, const float* bw, int nfb_, const SegF& A,
                                                const SegF& B, FAcc& c) {
+  const int nft = NT > 0 ? NT : nft_, nfb = NB > 0 ? NB : nfb_;
   const dfl Dx = df_sub(dfl{A.cxh, A.cxl}, dfl{B.cxh, B.cxl});
   const dfl Dy = df_sub(dfl{A.cyh, A.cyl}, dfl{B.cyh, B.cyl});
   const float dfx = Dx.hi + Dx.lo, dfy = Dy.hi + Dy.lo;
-  float r0 = 0.f, phi0 = 0.f;
+  float r0 = 0.f, phi0 = 0.f, k3 = 0.f;
   const float kf = op.khi;
   if (kf != 0.f) {
     const dfl R0sq = df_add(df_mul(Dx, Dx), df_mul(Dy, Dy));
     const dfl R0 = df_mul(R0sq, df_rsqrt(R0sq));
     r0 = R0.hi + R0.lo;
     phi0 = reduce_2pi(df_mul(R0, dfl{op.khi, op.klo}));
+    k3 = __fdiv_rn(3.f, kf);
   }
+  const float dfx2 = 2.f * dfx, dfy2 = 2.f * dfy;
   float pr[4] = {0.f, 0.f, 0.f, 0.f}, pi[4] = {0.f, 0.f, 0.f, 0.f}, mr = 0.f, mi = 0.f;
+#pragma unroll
   for (int p = 0; p < nft; ++p) {
     const float sp = fx[p];
     const float ox = (sp - 0.5f) * A.dx, oy = (sp - 0.5f) * A.dy;
     float s0r = 0.f, s0i = 0.f, s1r = 0.f, s1i = 0.f;
+#pragma unroll
     for (int q = 0; q < nfb; ++q) {
       const float tq = bx[q];
       const float wx = ox - (tq - 0.5f) * B.dx, wy = oy - (tq - 0.5f) * B.dy;
@@ -607,7 +677,7 @@ __device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, co
       // phase increment delta from q = 2 D.w + w.w, accurate in absolute terms
       const float rx = dfx + wx, ry = dfy + wy;
       const float R2 = fmaf(rx, rx, ry * ry);
-      const float invR = rsqrtf(R2);
+      const float invR = rsqrt_ftz(R2);
       const float R = R2 * invR;
       float Kr, Ki;
       if (OP == BGB_OP2D_SL || OP == BGB_OP2D_HS) {
@@ -615,9 +685,9 @@ __device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, co
           Kr = -kInv2PiF * __logf(R);
           Ki = 0.f;
         } else {
-          const float qv = fmaf(2.f * dfx + wx, wx, (2.f * dfy + wy) * wy);
-          const float delta = __fdividef(qv, R + r0);
-          hankel0_mixed(kf * R, fmaf(kf, delta, phi0), Kr, Ki);
+          const float qv = fmaf(dfx2 + wx, wx, (dfy2 + wy) * wy);
+          const float delta = qv * rcp_ftz(R + r0);
+          hankel0_mixed(kf * R, k3 * invR, fmaf(kf, delta, phi0), Kr, Ki);
         }
       } else {
         float gr, gi;
@@ -625,9 +695,9 @@ __device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, co
           gr = -kInv2PiF * invR * invR;
           gi = 0.f;
         } else {
-          const float qv = fmaf(2.f * dfx + wx, wx, (2.f * dfy + wy) * wy);
-          const float delta = __fdividef(qv, R + r0);
-          hankel1_mixed(kf * R, fmaf(kf, delta, phi0), 0.25f * kf * invR, gr, gi);
+          const float qv = fmaf(dfx2 + wx, wx, (dfy2 + wy) * wy);
+          const float delta = qv * rcp_ftz(R + r0);
+          hankel1_mixed(kf * R, k3 * invR, fmaf(kf, delta, phi0), 0.25f * kf * invR, gr, gi);
         }
         const float proj = OP == BGB_OP2D_DL ? -(rx * B.nx + ry * B.ny) : rx * A.nx + ry * A.ny;
         Kr = gr * proj;
@@ -671,11 +741,14 @@ __device__ __forceinline__ void finalize_mixed(const Op& op, const SegF& A, cons
                                                LT* __restrict__ out) {
   const float nn = A.nx * B.nx + A.ny * B.ny;
   const float ia = 1.f / A.len, ib = 1.f / B.len;
+  LT v[4];
   const float dA[2] = {op.nsA == 2 ? -ia : 0.f, op.nsA == 2 ? ia : 0.f};
   const float dB[2] = {op.nsB == 2 ? -ib : 0.f, op.nsB == 2 ? ib : 0.f};
   const float bmr = op.fbr * c.mr - op.fbi * c.mi, bmi = op.fbr * c.mi + op.fbi * c.mr;
-  for (int i = 0; i < op.nsA; ++i)
-    for (int j = 0; j < op.nsB; ++j) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
       const float pr = c.pr[2 * i + j], pi = c.pi[2 * i + j];
       float lr = op.far_ * pr - op.fai * pi, li = op.far_ * pi + op.fai * pr;
       if (OP == BGB_OP2D_HS) {
@@ -683,8 +756,18 @@ __device__ __forceinline__ void finalize_mixed(const Op& op, const SegF& A, cons
         lr = fmaf(lr, nn, bmr * d);
         li = fmaf(li, nn, bmi * d);
       }
-      out[i * op.nsB + j] = LT{lr, li};
+      v[2 * i + j] = LT{lr, li};
     }
+  if (sizeof(LT) == 8 && op.LS == 4) {  // 32 contiguous bytes
+    ((float4*)out)[0] = make_float4((float)v[0].x, (float)v[0].y, (float)v[1].x, (float)v[1].y);
+    ((float4*)out)[1] = make_float4((float)v[2].x, (float)v[2].y, (float)v[3].x, (float)v[3].y);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (i < op.nsA && j < op.nsB) out[i * op.nsB + j] = v[2 * i + j];
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -761,7 +844,7 @@ __global__ void __launch_bounds__(128) k_curve_far(Op op, const Rules* __restric
   }
 }
 
-template <int OP>
+template <int OP, int NT, int NB>
 __global__ void __launch_bounds__(128) k_curve_far_mixed(Op op, const Rules* __restrict__ rules,
                                                          const SegF* __restrict__ gT, const SegF* __restrict__ gB,
                                                          const int* __restrict__ T, int nT, const int* __restrict__ S,
@@ -783,7 +866,7 @@ __global__ void __launch_bounds__(128) k_curve_far_mixed(Op op, const Rules* __r
     if (nonfar_bit(mask, (int64_t)sl * nT + tl)) continue;
     const SegF B = gB[S[sl]];
     FAcc c;
-    far_pair_mixed<OP>(op, fx, fw, nft, bx, bw, nfb, A, B, c);
+    far_pair_mixed<OP, NT, NB>(op, fx, fw, nft, bx, bw, nfb, A, B, c);
     finalize_mixed<OP>(op, A, B, c, L + ((int64_t)sl * nT + tl) * op.LS);
   }
 }
@@ -824,10 +907,11 @@ __global__ void __launch_bounds__(256) k_curve_special(Op op, const Rules* __res
 // ---- Mixed path: coincident and common-vertex pairs in double-float ---------------------------
 // The FP64 rules and series of singular_rule_warp / kernel_series evaluated with double-float
 // arithmetic on the FP32 pipes (about 48 bits), single and hypersingular kernels (the double layers
-// keep the FP64 kernel).  Each lane sums the kernel times the weight into four moments
+// keep the FP64 kernel), in packed pairs (both series, real and imaginary sums).  Each lane sums the kernel times the
+// weight into four moments
 // (1, s, t, s t), from which the shape products follow.
 struct DfMom {
-  dfl r[4], i[4];  // sum of K w, K w s, K w t, K w s t
+  df2 v[4];  // (real, imaginary) sums of K w, K w s, K w t, K w s t
 };
 
 __device__ __forceinline__ dfl df_scale(dfl a, float f) { return dfl{a.hi * f, a.lo * f}; }  // f a power of 2
@@ -842,11 +926,13 @@ __device__ __forceinline__ void df_point(const Op& op, const RulesDF& R, dfl Rd,
   } else {
     const dfl x = df_mul(Rd, dfl{op.khi, op.klo});
     if (x.hi <= 4.f) {
+      // both series in packed operations
       const dfl u = df_scale(df_mul(x, x), 0.25f);
-      dfl j0 = R.sa[M];
-      for (int m = M - 1; m >= 0; --m) j0 = df_add(df_mul(j0, u), R.sa[m]);
-      dfl s0 = R.sb[M - 1];
-      for (int m = M - 2; m >= 0; --m) s0 = df_add(df_mul(s0, u), R.sb[m]);
+      const df2 uu = df2_both(u);
+      df2 v = M < kSeries ? df2{R.ab[M].hi & 0xffffffffull, R.ab[M].lo & 0xffffffffull} : R.ab[kSeries];
+      for (int m = M - 1; m >= 0; --m) v = df2_macc(R.ab[m], v, uu);
+      dfl j0, s0;
+      df2_parts(v, j0, s0);
       const dfl y0v = df_mul(R.two_over_pi, df_add(df_mul(df_add(lnR, lnk2g), j0), df_mul(s0, u)));
       Kr = df_scale(y0v, -0.25f);
       Ki = df_scale(j0, -0.25f);
@@ -859,16 +945,11 @@ __device__ __forceinline__ void df_point(const Op& op, const RulesDF& R, dfl Rd,
       Ki.lo = (float)(yi - (double)Ki.hi);
     }
   }
-  const dfl kwr = df_mul(Kr, wl), kwi = df_mul(Ki, wl);
-  const dfl st = df_mul(s, t);
-  mo.r[0] = df_add(mo.r[0], kwr);
-  mo.i[0] = df_add(mo.i[0], kwi);
-  mo.r[1] = df_add(mo.r[1], df_mul(kwr, s));
-  mo.i[1] = df_add(mo.i[1], df_mul(kwi, s));
-  mo.r[2] = df_add(mo.r[2], df_mul(kwr, t));
-  mo.i[2] = df_add(mo.i[2], df_mul(kwi, t));
-  mo.r[3] = df_add(mo.r[3], df_mul(kwr, st));
-  mo.i[3] = df_add(mo.i[3], df_mul(kwi, st));
+  const df2 kw = df2_mul(df2_of(Kr, Ki), df2_both(wl));
+  mo.v[0] = df2_add(mo.v[0], kw);
+  mo.v[1] = df2_macc(mo.v[1], kw, df2_both(s));
+  mo.v[2] = df2_macc(mo.v[2], kw, df2_both(t));
+  mo.v[3] = df2_macc(mo.v[3], kw, df2_both(df_mul(s, t)));
 }
 
 __device__ __forceinline__ dfl df_from_double(double v) {
@@ -926,11 +1007,11 @@ __device__ void singular_rule_warp_df(const Op& op, const RulesDF& R, const SegG
   __syncwarp();
 }
 
-__device__ __forceinline__ dfl warp_sum_df(dfl v) {
+__device__ __forceinline__ df2 warp_sum_df2(df2 v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    const dfl o{__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)};
-    v = df_add(v, o);
+    const df2 o{__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)};
+    v = df2_add(v, o);
   }
   return v;
 }
@@ -970,26 +1051,17 @@ __global__ void __launch_bounds__(256) k_curve_special_df(Op op, const Rules* __
     } else {
       DfMom mo;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) mo.r[k] = mo.i[k] = dfl{0.f, 0.f};
+      for (int k = 0; k < 4; ++k) mo.v[k] = df2{0ull, 0ull};
       singular_rule_warp_df<OP>(op, sR, A, B, sp.cls, sp.match, lane, wtab, mo);
       double mr[4], mi[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        mr[k] = df_to_double(warp_sum_df(mo.r[k]));
-        mi[k] = df_to_double(warp_sum_df(mo.i[k]));
+        dfl re, im;
+        df2_parts(warp_sum_df2(mo.v[k]), re, im);
+        mr[k] = df_to_double(re);
+        mi[k] = df_to_double(im);
       }
-      // shape products from the moments: f = (1 - s, s) or 1, g = (1 - t, t) or 1
-      const bool hA = op.nsA == 2, hB = op.nsB == 2;
-      c.pr[0] = mr[0] - (hA ? mr[1] : 0.0) - (hB ? mr[2] : 0.0) + (hA && hB ? mr[3] : 0.0);
-      c.pi[0] = mi[0] - (hA ? mi[1] : 0.0) - (hB ? mi[2] : 0.0) + (hA && hB ? mi[3] : 0.0);
-      c.pr[1] = mr[2] - (hA ? mr[3] : 0.0);
-      c.pi[1] = mi[2] - (hA ? mi[3] : 0.0);
-      c.pr[2] = mr[1] - (hB ? mr[3] : 0.0);
-      c.pi[2] = mi[1] - (hB ? mi[3] : 0.0);
-      c.pr[3] = mr[3];
-      c.pi[3] = mi[3];
-      c.mr = mr[0];
-      c.mi = mi[0];
+      moments_to_acc(op, mr, mi, 1.0, c);  // (the lengths are in the weights)
     }
     if (lane == 0) finalize<OP>(op, A, B, c, L + sp.slot);
   }
@@ -1028,7 +1100,7 @@ __global__ void __launch_bounds__(128) k_curve_pairs(Op op, const Rules* __restr
       }
       FAcc c;
       const SegF Af = gTf[pairs[p].x], Bf = gBf[pairs[p].y];
-      far_pair_mixed<OP>(op, fx, fw, rules->nft, bx, bw, rules->nfb, Af, Bf, c);
+      far_pair_mixed<OP, 0, 0>(op, fx, fw, rules->nft, bx, bw, rules->nfb, Af, Bf, c);
       finalize_mixed<OP>(op, Af, Bf, c, L + p * 4);
     } else {
       Acc c;
@@ -1229,18 +1301,28 @@ static int put(cudaStream_t st, DevBuf& buf, const std::vector<T>& v) {
   return 0;
 }
 
+// Threads over the test segments, a run of trial segments per CTA: about 64 CTAs per SM in all, so that a CTA's
+// rules and test segment are loaded once for tens of pairs per thread (with one trial segment per CTA the far
+// stage of 8,192 segments took 3.9 ms).
+static dim3 pair_grid(int nT, int nS, int threads, int num_sms) {
+  const int gx = (nT + threads - 1) / threads;
+  return dim3(gx, std::max(1, std::min(std::min(nS, 65535), (64 * num_sms + gx - 1) / gx)));
+}
+
 template <int OP>
 static void launch_far(const Op& op, const Rules* rules, const SegGeo* gT, const SegGeo* gB, const int* T, int nT,
-                       const int* S, int nS, const unsigned* mask, double2* L, cudaStream_t st) {
-  dim3 grid((nT + 127) / 128, std::min(nS, 65535));
+                       const int* S, int nS, const unsigned* mask, double2* L, int num_sms, cudaStream_t st) {
+  const dim3 grid = pair_grid(nT, nS, 128, num_sms);
   k_curve_far<OP><<<grid, 128, 0, st>>>(op, rules, gT, gB, T, nT, S, nS, mask, L);
 }
 
 template <int OP>
 static void launch_far_mixed(const Op& op, const Rules* rules, const SegF* gT, const SegF* gB, const int* T, int nT,
-                             const int* S, int nS, const unsigned* mask, float2* L, cudaStream_t st) {
-  dim3 grid((nT + 127) / 128, std::min(nS, 65535));
-  k_curve_far_mixed<OP><<<grid, 128, 0, st>>>(op, rules, gT, gB, T, nT, S, nS, mask, L);
+                             const int* S, int nS, const unsigned* mask, float2* L, bool rule44, int num_sms,
+                             cudaStream_t st) {
+  const dim3 grid = pair_grid(nT, nS, 128, num_sms);
+  if (rule44) k_curve_far_mixed<OP, 4, 4><<<grid, 128, 0, st>>>(op, rules, gT, gB, T, nT, S, nS, mask, L);
+  else k_curve_far_mixed<OP, 0, 0><<<grid, 128, 0, st>>>(op, rules, gT, gB, T, nT, S, nS, mask, L);
 }
 
 template <int OP, class LT>
@@ -1292,8 +1374,12 @@ static void make_rules_df(const Rules& R, RulesDF* D) {
     D->gl2x[b] = df(R.gl2_x[b]);
     D->gl2w[b] = df(R.gl2_w[b]);
   }
-  for (int m = 0; m <= kSeries; ++m) D->sa[m] = df(R.sa[m]);
-  for (int m = 0; m < kSeries; ++m) D->sb[m] = df(R.sb[m]);
+  for (int m = 0; m <= kSeries; ++m) {
+    const dfl a = df(R.sa[m]), b = df(m < kSeries ? R.sb[m] : 0.0);
+    const float hi[2] = {a.hi, b.hi}, lo[2] = {a.lo, b.lo};
+    std::memcpy(&D->ab[m].hi, hi, sizeof(hi));
+    std::memcpy(&D->ab[m].lo, lo, sizeof(lo));
+  }
   D->inv2pi = df(0.15915494309189535);
   D->two_over_pi = df(0.6366197723675814);
 }
@@ -1514,7 +1600,7 @@ int bgb_assemble_curve(bgb_handle* h, const bgb_operator2d* op, const bgb_curve_
         BGB_CUDA(cudaMemsetAsync(B.counts.p, 0, sizeof(int) * 8, s));
         BGB_CUDA(cudaMemsetAsync(B.mask.p, 0, mask_bytes, s));
         BGB_CUDA(cudaEventRecord(h->ev[0], s));
-        dim3 grid((nT + 255) / 256, std::min(nS, 65535));
+        const dim3 grid = pair_grid(nT, nS, 256, h->num_sms);
         k_curve_classify<<<grid, 256, 0, s>>>(B.geo_t.as<SegGeo>(), B.geo_b.as<SegGeo>(), B.geof_t.as<SegF>(),
                                               B.geof_b.as<SegF>(), B.T.as<int>(), nT, B.S.as<int>(),
                                               nS, B.own.as<unsigned char>(), o.k2, o.LS, B.list.as<Special>(), cap,
@@ -1537,10 +1623,11 @@ int bgb_assemble_curve(bgb_handle* h, const bgb_operator2d* op, const bgb_curve_
       BGB_CUDA(cudaEventRecord(h->ev[2], s));
       if (precision == BGB_PREC_MIXED) {
         BGB_CURVE_DISPATCH(o.kind, launch_far_mixed, o, B.rules.as<Rules>(), B.geof_t.as<SegF>(), B.geof_b.as<SegF>(),
-                           B.T.as<int>(), nT, B.S.as<int>(), nS, B.mask.as<unsigned>(), B.L.as<float2>(), s);
+                           B.T.as<int>(), nT, B.S.as<int>(), nS, B.mask.as<unsigned>(), B.L.as<float2>(),
+                           qs->far_test == 4 && qs->far_trial == 4, h->num_sms, s);
       } else {
         BGB_CURVE_DISPATCH(o.kind, launch_far, o, B.rules.as<Rules>(), B.geo_t.as<SegGeo>(), B.geo_b.as<SegGeo>(),
-                           B.T.as<int>(), nT, B.S.as<int>(), nS, B.mask.as<unsigned>(), B.L.as<double2>(), s);
+                           B.T.as<int>(), nT, B.S.as<int>(), nS, B.mask.as<unsigned>(), B.L.as<double2>(), h->num_sms, s);
       }
       BGB_CUDA(cudaGetLastError());
       BGB_CUDA(cudaEventRecord(h->ev[3], s));
