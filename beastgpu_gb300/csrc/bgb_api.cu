@@ -1010,33 +1010,57 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     size_t smem = 0;
     for (int id : prefs) {
       const TileCfg tc = kTileCfgs[id];
-      if (tc.FM != ord_fm) {
-        ord_t = order_functions(St, cent_t, (int)row0, (int)(row0 + nrows), tc.FM, nth);
-        // rows of a tile in ascending order: the tile's output stores of one column then fall in
-        // fewer 32-byte sectors (C2: 23 instead of 60 per column)
-        for (size_t b = 0; b < ord_t.size(); b += (size_t)tc.FM)
-          std::sort(ord_t.begin() + b, ord_t.begin() + std::min(ord_t.size(), b + (size_t)tc.FM));
-        ord_fm = tc.FM;
+      // the two sides beside each other: the first levels of a bisection are serial (level-5 EFIE: 4.6 ms one
+      // after the other, longer than the classification and the singular pairs that hide it)
+      auto test_side = [&] {
+        if (tc.FM != ord_fm) {
+          ord_t = order_functions(St, cent_t, (int)row0, (int)(row0 + nrows), tc.FM, nth);
+          // rows of a tile in ascending order: the tile's output stores of one column then fall in
+          // fewer 32-byte sectors (C2: 23 instead of 60 per column)
+          for (size_t b = 0; b < ord_t.size(); b += (size_t)tc.FM)
+            std::sort(ord_t.begin() + b, ord_t.begin() + std::min(ord_t.size(), b + (size_t)tc.FM));
+          ord_fm = tc.FM;
+        }
+        PL.test = HostPlan();
+        plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth);
+      };
+      auto trial_side = [&](bool same_order) {
+        if (tc.FN != ord_fn) {
+          if (same_order)
+            ord_b[0] = ord_t;  // the same functions and width: the same order
+          else
+            over_blocks([&](int b, int threads) {
+              ord_b[b] = order_functions(Sb, cent_b, (int)col_start[b], (int)col_start[b + 1], tc.FN, threads);
+            });
+          ord_fn = tc.FN;
+        }
+        PL.trial.assign(nblocks, HostPlan());
+        over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, tc.SC, PL.trial[b], threads); });
+      };
+      if (same && nblocks == 1 && row0 == 0 && nrows == ncols && tc.FN == tc.FM) {
+        test_side();
+        trial_side(true);
+      } else if (nrows + ncols < 2000) {  // a thread costs more than the overlap gives
+        test_side();
+        trial_side(false);
+      } else {
+        parallel_for(2, 2, [&](int side) {
+          if (side)
+            trial_side(false);
+          else
+            test_side();
+        });
       }
-      if (tc.FN != ord_fn) {
-        if (same && nblocks == 1 && row0 == 0 && nrows == ncols && tc.FN == tc.FM)
-          ord_b[0] = ord_t;  // the same functions and width: the same order
-        else
-          over_blocks([&](int b, int threads) {
-            ord_b[b] = order_functions(Sb, cent_b, (int)col_start[b], (int)col_start[b + 1], tc.FN, threads);
-          });
-        ord_fn = tc.FN;
-      }
-      PL.test = HostPlan();
-      plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth);
       // Chunks of tc.SC trial triangles; a tile pinned by the caller, and the last choice, also with
       // narrower chunks when the chunk buffers do not fit (the result does not depend on the chunks).
       for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
         TilePlan probe{};
         probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = sc; probe.MAXS = PL.test.MAXS;
         probe.tmax = std::max(1, PL.test.tmax);
-        PL.trial.assign(nblocks, HostPlan());
-        over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
+        if (sc != tc.SC) {
+          PL.trial.assign(nblocks, HostPlan());
+          over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
+        }
         for (int b = 0; b < nblocks; ++b) {
           probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
           probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);

@@ -3,7 +3,11 @@
 
 #include "bgb_kernels.cuh"
 
+#include <algorithm>
+#include <atomic>
+#include <exception>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 namespace bgb {
@@ -163,6 +167,31 @@ void plan_test_side_par(const Supports& S, const std::vector<int>& order, int FM
                         int tcap = 1 << 30);
 void plan_trial_side_par(const Supports& S, const std::vector<int>& order, int FN, int SC, HostPlan& P, int nth);
 int planner_threads();
+// fn(i) for i in [0, n), spread over up to nth threads (the calling one included). An exception of any of
+// them reaches the caller after all have ended; where no thread can be started, fewer share the work.
+template <class F>
+void parallel_for(int n, int nth, F fn) {
+  std::atomic<int> next{0};
+  std::exception_ptr failed;
+  std::mutex mu;
+  auto work = [&] {
+    try {
+      for (int i = next++; i < n; i = next++) fn(i);
+    } catch (...) {
+      next = n;
+      std::lock_guard<std::mutex> lk(mu);
+      failed = std::current_exception();
+    }
+  };
+  std::vector<std::thread> th;
+  try {
+    for (int t = 1; t < std::min(nth, n); ++t) th.emplace_back(work);
+  } catch (const std::exception&) {
+  }
+  work();
+  for (auto& x : th) x.join();
+  if (failed) std::rethrow_exception(failed);
+}
 bool same_space(const bgb_space* a, const bgb_space* b);
 // Largest triangle edge of a space (host), for the argument range of the double-float sincos.
 SpaceExtents space_extents(const bgb_space* s);
