@@ -1,12 +1,13 @@
 // C ABI of libbeastgb: handles, validation, host-side tile planning and the assembly pipeline
 //
 //   upload spaces -> k_prepare_geo64 -> k_prepare_bounds -> k_classify (count, scan, fill)
-//   -> k_singular (FP64 Sauter-Schwab / near pairs) -> k_prepare_rec -> k_far_persistent
-//   (FP64 or mixed) -> output on the device, or row blocks copied to the host.
+//   -> singular pairs (k_ss64, k_singular_df; near and inexactly matching pairs: k_singular)
+//   -> k_prepare_rec -> far pairs and gather (mixed: k_far_persistent; FP64: k_pair64 and
+//   k_gather64 per panel of pairs) -> output on the device, or column blocks copied to the host.
 //
 // The pipeline mirrors assemble_gpu (assamble_gpu.jl:25-137) and assemblechunk_body_gpu!
 // (assamble_chunk_gpu.jl:104-196): classify, singular pairs, far pairs, write-back.  Unlike the
-// reference, the write-back is a deterministic gather inside the far kernel (no FP64 atomics
+// reference, the write-back is a deterministic gather on the device (no FP64 atomics
 // into a 2 x N x N buffer, no make_complex pass) and non-far pairs of class "near" are integrated
 // (the reference drops them, quadrule_determine.jl:76 with doubleQuadRuleMainCase.jl:154).
 #include "bgb_host.h"
@@ -243,7 +244,7 @@ FarConst make_farconst(const OpParams& op, const RuleTable& R, const QuadSel& qs
   for (int J = 0; J < k.qb; ++J) {
     const double* p = R.uvw[R.offset[qs.far_b] + J];
     double h[3] = {p[0], p[1], 1.0 - p[0] - p[1]};
-    for (int i = 0; i < 3; ++i) { k.shpB64[J][i] = h[i]; k.shpB[J][i] = (float)h[i]; }
+    for (int i = 0; i < 3; ++i) { k.shpB64[J][i] = h[i]; k.shpB[i][J] = (float)h[i]; }
   }
   // plain FP64 kernel: series for exp(-i k (R - R0)) when |k (R - R0)| <= k (r_test + r_trial) is small
   k.tay_n = 0;

@@ -118,20 +118,18 @@ int far_target_ctas_per_sm(int precision) {
 }
 
 int rec_stride(int precision, int q, int generic) {
-  (void)q;
   if (!generic) return precision == BGB_PREC_MIXED ? kRec34F : kRec34D;
-  return precision == BGB_PREC_MIXED ? farimpl::off32_size(BGB_MAXQ) : 13 + 4 * BGB_MAXQ;
+  return precision == BGB_PREC_MIXED ? farimpl::off32_size(q) : 13 + 4 * BGB_MAXQ;
 }
 
 size_t far_smem_bytes(int precision, int op_kind, int qt, int qb, const TilePlan& p) {
   const bool gen = far_generic_q(qt, qb);
-  // the layout depends on the operator only through chunk_trial_records (Lagrange or RWG)
   const bool lag = is_lagrange_op(op_kind);
   if (precision == BGB_PREC_MIXED)
-    return gen ? (lag ? smem_t<PMixed, BGB_OP_HELMHOLTZ3D_SL, BGB_MAXQ, BGB_MAXQ>(p)
-                      : smem_t<PMixed, BGB_OP_MAXWELL3D_SL, BGB_MAXQ, BGB_MAXQ>(p))
-               : (lag ? smem_t<PMixed, BGB_OP_HELMHOLTZ3D_SL, 3, 4>(p) : smem_t<PMixed, BGB_OP_MAXWELL3D_SL, 3, 4>(p));
-  return gen ? smem_t<PFp64, 0, BGB_MAXQ, BGB_MAXQ>(p) : smem_t<PFp64, 0, 3, 4>(p);
+    return gen ? (lag ? smem_t<PMixed, BGB_OP_HELMHOLTZ3D_SL, BGB_MAXQ, BGB_MAXQ>(p, qt, qb)
+                      : smem_t<PMixed, BGB_OP_MAXWELL3D_SL, BGB_MAXQ, BGB_MAXQ>(p, qt, qb))
+               : (lag ? smem_t<PMixed, BGB_OP_HELMHOLTZ3D_SL, 3, 4>(p, qt, qb) : smem_t<PMixed, BGB_OP_MAXWELL3D_SL, 3, 4>(p, qt, qb));
+  return gen ? smem_t<PFp64, 0, BGB_MAXQ, BGB_MAXQ>(p, qt, qb) : smem_t<PFp64, 0, 3, 4>(p, qt, qb);
 }
 
 int launch_far_pairs_diag(int precision, const FarConst& k, const void* rt, const void* rb, const int* tau,

@@ -12,9 +12,13 @@
 // written exactly once.  Non-far pairs (singular or near, found by the classifier) are
 // taken from the FP64 singular-pair buffer instead of the far rule.
 //
-// Roofline: compute-bound on FP32 issue (mixed) or FP64 issue (plain), plus MUFU
-// (rsqrt, rcp, sin, cos).  Per point pair the mixed kernel spends ~23 FP32 ops + 4 MUFU on
-// the kernel value and 13 (Helmholtz / EFIE) or ~26 (MFIE) on accumulation.
+// The tile kernel serves the mixed path and FP64 batches; single FP64 assemblies compute the local matrices of
+// panels of pairs (k_pair64, below) and gather them in a second kernel: at 1/62 of the FP32 rate the halo's
+// FP64 work costs more than writing the matrices once (level-4 EFIE: 84.3 -> 46 ms).
+//
+// Roofline: compute-bound on FP32 issue (mixed) or FP64 issue (plain), plus MUFU (rsqrt, rcp, sin, cos: 4 per
+// point pair).  The default rule pair (3 x 4 points) has its own pair code (bgb_far_pair34.cuh); the other rules
+// take 21 packed FP32 operations per two point pairs (EFIE).
 //
 // Mixed precision (FP32) keeps the phase k R accurate without FP64: per pair, the centroid
 // distance D = c_tau - c_sigma is formed in double-float, R0 is any FP32 number close to |D|,
@@ -25,6 +29,7 @@
 // centroid, so the EFIE/MFIE bilinear forms carry no cancellation either.
 // Far-pair kernel templates; instantiated per precision and operator in bgb_far_*_op*.cu.
 #pragma once
+#include "bgb_df.cuh"
 #include "bgb_kernels.cuh"
 
 #include <algorithm>
@@ -93,15 +98,16 @@ namespace farimpl {
 
 // Records of the generic rules (the 3 x 4 rule pair has its own, bgb_far_pair34.cuh).
 // FP32 record of a triangle, in 16-byte groups read with 128-bit shared-memory loads:
-// [CH.xyz CL.x] [CL.yz - -] [x y z w] per quadrature point [VO (9) INV2A - -]; the stride is an odd
-// number of groups, so the records of different triangles start in different bank groups.
-template <int Q>
+// [CH.xyz CL.x] [CL.yz - -] [VO (9) INV2A - -], two groups [x0 x1 y0 y1] [z0 z1 w0 w1] per two quadrature points
+// (the operands of packed operations; a last odd point is paired with one of weight zero).  The stride follows
+// the rule's points (6 or 7: 52 floats) and is an odd number of groups, so the records of different triangles
+// start in different bank groups.
+__host__ __device__ constexpr int off32_size(int q) { return 4 * ((5 + q + (q & 1)) | 1); }
 struct Off32 {
-  static constexpr int CH = 0, CL = 3, X = 8, PS = 4, VO = 8 + 4 * Q, INV2A = VO + 9, SIZE = 4 * ((5 + Q) | 1);
-  static constexpr int px(int I) { return X + PS * I; }      // point I: x, y, z
-  static constexpr int pw(int I) { return X + PS * I + 3; }  // point I: weight
+  static constexpr int CH = 0, CL = 3, VO = 8, INV2A = VO + 9, X = 20;
+  static __host__ __device__ constexpr int px(int I) { return X + 8 * (I >> 1) + (I & 1); }  // x; y, z: 2, 4 on
+  static __host__ __device__ constexpr int pw(int I) { return px(I) + 6; }                  // weight
 };
-__host__ __device__ constexpr int off32_size(int Q) { return 4 * ((5 + Q) | 1); }
 template <int Q>
 struct Off64 {
   static constexpr int C = 0, X = 3, W = 3 + 3 * Q, VO = 3 + 4 * Q, INV2A = 12 + 4 * Q, SIZE = 13 + 4 * Q;
@@ -111,8 +117,8 @@ struct PMixed {
   using R = float;
   using C = float2;
   static constexpr int kThreads = 256, kMinBlocks = 3;  // 24 warps per SM (<= 85 registers)
-  template <int Q>
-  static constexpr int rec() { return Q <= 4 ? kRec34F : Off32<Q>::SIZE; }
+  template <int Q>  // stride of the records of a rule of q points (q <= Q)
+  static __host__ __device__ constexpr int rec(int q) { return Q <= 4 ? kRec34F : off32_size(q); }
   static __device__ __forceinline__ C mk(double a, double b) { return make_float2((float)a, (float)b); }
 };
 struct PFp64 {
@@ -120,7 +126,7 @@ struct PFp64 {
   using C = double2;
   static constexpr int kThreads = 256, kMinBlocks = 1;
   template <int Q>
-  static constexpr int rec() { return Q <= 4 ? kRec34D : Off64<Q>::SIZE; }
+  static __host__ __device__ constexpr int rec(int = 0) { return Q <= 4 ? kRec34D : Off64<Q>::SIZE; }
   static __device__ __forceinline__ C mk(double a, double b) { return make_double2(a, b); }
 };
 
@@ -135,12 +141,25 @@ __device__ __forceinline__ void load_vo(const float4* __restrict__ g, float V[3]
   V[2][0] = v1.z; V[2][1] = v1.w; V[2][2] = v2.x;
 }
 
+using f2x = unsigned long long;  // two FP32 numbers, the operand of packed operations
+__device__ __forceinline__ f2x both(float x) { return pk2(x, x); }
+__device__ __forceinline__ float half_sum(f2x a) {
+  float x, y;
+  upk2(a, x, y);
+  return x + y;
+}
+
+// Bound by FP32 issue and MUFU (4 per point pair).  Trial points two at a time in packed operations, loops rolled: the
+// scalar form, unrolled over 13 x 13 points with an exit per point, ran ~120 KB of code per pair.  The MFIE's
+// sums come from sum H and sum H y like the EFIE's from sum G and sum G y.  Level-4 EFIE, 6 x 7 points: far stage
+// 7.6 -> 3.9 ms with the per-chunk trial records and strides by the rule's points (60 x 80 tiles instead of
+// 60 x 64 cut to fit, 1.56 instead of 1.86 times the pairs); unrolled by two 4.7 ms, two CTAs per SM 4.4 - 4.8 ms.
 template <int OP, int QT, int QB>
 __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float (*__restrict__ shpT)[3],
-                                               const float (*__restrict__ shpB)[3], const float* __restrict__ a,
+                                               const float (*__restrict__ shpB)[BGB_MAXQ + 1], const float* __restrict__ a,
                                                const float* __restrict__ b, float2 L[9]) {
-  using OA = Off32<QT>;
-  using OB = Off32<QB>;
+  using OA = Off32;
+  using OB = Off32;
   const float4* __restrict__ a4 = reinterpret_cast<const float4*>(a);
   const float4* __restrict__ b4 = reinterpret_cast<const float4*>(b);
   float Dh[3], Dl[3];
@@ -177,16 +196,16 @@ __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float 
   phi0 = fmaf(-nq, kPiB, phi0);
   phi0 = fmaf(-nq, kPiC, phi0);
   phi0 = __fadd_rn(phi0, pl);
-  const float R0sq = R0 * R0;
   const float D2x = 2.f * Dh[0], D2y = 2.f * Dh[1], D2z = 2.f * Dh[2];
   const float kh = K.k_hi;
   const float amp0 = K.lossy ? exp_ftz(-K.gre * R0) : 1.f;
   constexpr bool kHH = is_lagrange_op(OP);
+  constexpr bool kGrad = OP == BGB_OP_HELMHOLTZ3D_DL || OP == BGB_OP_HELMHOLTZ3D_DLT || OP == BGB_OP_MAXWELL3D_DL;
   float nA[3] = {0.f, 0.f, 0.f}, nB[3] = {0.f, 0.f, 0.f};
   if (OP == BGB_OP_HELMHOLTZ3D_DLT || OP == BGB_OP_HELMHOLTZ3D_HS) tri_normal(a + OA::VO, a[OA::INV2A], nA);
   if (OP == BGB_OP_HELMHOLTZ3D_DL || OP == BGB_OP_HELMHOLTZ3D_HS) tri_normal(b + OB::VO, b[OB::INV2A], nB);
   const int qt = QT < BGB_MAXQ ? QT : K.qt;
-  const int qb = QB < BGB_MAXQ ? QB : K.qb;
+  const int qb2 = (QB < BGB_MAXQ ? QB + 1 : K.qb + 1) / 2;
 
   // accumulators
   float2 S = make_float2(0.f, 0.f), P0 = make_float2(0.f, 0.f);
@@ -196,195 +215,114 @@ __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float 
 #pragma unroll
   for (int k = 0; k < 9; ++k) L[k] = make_float2(0.f, 0.f);
 
-  if constexpr (OP != BGB_OP_MAXWELL3D_DL) {
-    // Helmholtz / EFIE: q = s.(2 D_hi + s) with s = a_I - y_J, a_I = D_lo + x_I, split as
-    //   q = [c0 + a_I.(a_I + 2 D_hi)] + [y_J.(y_J - 2 D_hi)] - 2 a_I.y_J
-    // (per test point, per trial point, per point pair): 5 operations per point pair.
-#pragma unroll
-    for (int I = 0; I < QT; ++I) {
-      if (I >= qt) break;
-      const float4 XI = a4[OA::px(I) / 4];
-      const float Xx = XI.x, Xy = XI.y, Xz = XI.z;
-      const float ax = Dl[0] + Xx, ay = Dl[1] + Xy, az = Dl[2] + Xz;
-      const float KI = fmaf(ax, ax + D2x, fmaf(ay, ay + D2y, fmaf(az, az + D2z, c0)));
-      const float wI = XI.w;
-      // double layer: (x - y) . n_y = (D + X_I) . n_y, constant over the trial points
-      const float cI = OP == BGB_OP_HELMHOLTZ3D_DL
-                           ? fmaf(Dh[0] + ax, nB[0], fmaf(Dh[1] + ay, nB[1], (Dh[2] + az) * nB[2]))
-                           : 1.f;
-      float2 TI = make_float2(0.f, 0.f);
-      float2 UI[3], M[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) UI[c] = M[c] = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int J = 0; J < QB; ++J) {
-        if (J >= qb) break;
-        const float4 YJ = b4[OB::px(J) / 4];
-        const float yx = YJ.x, yy = YJ.y, yz = YJ.z;
-        const float mj = fmaf(yx, yx - D2x, fmaf(yy, yy - D2y, yz * (yz - D2z)));
-        const float dot = fmaf(ax, yx, fmaf(ay, yy, az * yz));
-        const float q = fmaf(-2.f, dot, KI + mj);
-        const float R2 = R0sq + q;
-        const float rs = rsqrt_ftz(R2);
-        const float delta = q * rcp_ftz(fmaf(R2, rs, R0));
-        float psi = fmaf(kh, delta, phi0);
-        if (!K.phase_direct) {  // |psi| may exceed 2 pi: reduce again
-          const float nn = rintf(psi * kInv2Pi);
-          psi = fmaf(-nn, kPiA, psi);
-          psi = fmaf(-nn, kPiB, psi);
-        }
-        float sn, cs;
-        sincos_ftz(psi, &sn, &cs);
-        float amp = (wI * YJ.w) * rs;
-        if (K.lossy) amp *= amp0 * exp_ftz(-K.gre * delta);
-        const float gr = amp * cs, gi = -amp * sn;
-        if (kHH) {
-          float hr = gr, hi = gi;
-          if (OP == BGB_OP_HELMHOLTZ3D_DL || OP == BGB_OP_HELMHOLTZ3D_DLT) {
-            // (gamma + 1/R) G / R, times -(x - y) . n_x = -(D - y_J) . n_x for the transposed layer
-            const float t = (K.gre + rs) * rs, u = kh * rs;
-            hr = t * gr - u * gi;
-            hi = t * gi + u * gr;
-            if (OP == BGB_OP_HELMHOLTZ3D_DLT) {
-              const float e = -fmaf(Dh[0] + (Dl[0] - yx), nA[0], fmaf(Dh[1] + (Dl[1] - yy), nA[1], (Dh[2] + (Dl[2] - yz)) * nA[2]));
-              hr *= e;
-              hi *= e;
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            const float g = shpB[J][j];
-            M[j].x = fmaf(hr, g, M[j].x);
-            M[j].y = fmaf(hi, g, M[j].y);
-          }
-        } else {
-          TI.x += gr;
-          TI.y += gi;
-          UI[0].x = fmaf(gr, yx, UI[0].x); UI[0].y = fmaf(gi, yx, UI[0].y);
-          UI[1].x = fmaf(gr, yy, UI[1].x); UI[1].y = fmaf(gi, yy, UI[1].y);
-          UI[2].x = fmaf(gr, yz, UI[2].x); UI[2].y = fmaf(gi, yz, UI[2].y);
-        }
+  const f2x R0sq2 = both(R0 * R0), R02 = both(R0), kh2 = both(kh), phi2 = both(phi0);
+#pragma unroll 1
+  for (int I = 0; I < qt; ++I) {
+    const float* __restrict__ pi = a + OA::px(I);
+    const float Xx = pi[0], Xy = pi[2], Xz = pi[4], wI = pi[6];
+    const float ax = Dl[0] + Xx, ay = Dl[1] + Xy, az = Dl[2] + Xz;
+    // q = |D + X_I - y|^2 - R0^2 = KI + y . (y - 2 (D + X_I))
+    const f2x KI = both(fmaf(ax, ax + D2x, fmaf(ay, ay + D2y, fmaf(az, az + D2z, c0))));
+    const f2x ex = both(-fmaf(2.f, ax, D2x)), ey = both(-fmaf(2.f, ay, D2y)), ez = both(-fmaf(2.f, az, D2z));
+    // sums of G (or of its radial derivative over R) times the weights, points y and hats; halves: even and odd points
+    f2x Tr = 0, Ti = 0, Ur[3] = {0, 0, 0}, Ui[3] = {0, 0, 0};
+#pragma unroll 1
+    for (int J = 0; J < qb2; ++J) {
+      const ulonglong2 g0 = *reinterpret_cast<const ulonglong2*>(b + OB::X + 8 * J);
+      const ulonglong2 g1 = *reinterpret_cast<const ulonglong2*>(b + OB::X + 8 * J + 4);
+      const f2x yx = g0.x, yy = g0.y, yz = g1.x, w = g1.y;
+      const f2x q = fma2(add2(yx, ex), yx, fma2(add2(yy, ey), yy, fma2(add2(yz, ez), yz, KI)));
+      const f2x R2 = add2(R0sq2, q);
+      float u0, u1, s0, s1, k0, k1;
+      upk2(R2, u0, u1);
+      const f2x rs = pk2(rsqrt_ftz(u0), rsqrt_ftz(u1));
+      upk2(fma2(R2, rs, R02), u0, u1);
+      const f2x delta = mul2(q, pk2(rcp_ftz(u0), rcp_ftz(u1)));
+      f2x psi = fma2(kh2, delta, phi2);
+      if (!K.phase_direct) {  // |psi| may exceed 2 pi: reduce again (rounding by the 1.5 2^23 addend)
+        const f2x magic = both(12582912.f);
+        const f2x n = sub2(magic, fma2(psi, both(kInv2Pi), magic));
+        psi = fma2(n, both(kPiB), fma2(n, both(kPiA), psi));
+      }
+      upk2(psi, u0, u1);
+      sincos_ftz(u0, &s0, &k0);
+      sincos_ftz(u1, &s1, &k1);
+      f2x amp = mul2(w, rs);
+      if (K.lossy) {
+        upk2(mul2(both(-K.gre), delta), u0, u1);
+        amp = mul2(amp, mul2(both(amp0), pk2(exp_ftz(u0), exp_ftz(u1))));
+      }
+      f2x hr = mul2(amp, pk2(k0, k1)), hi = mul2(amp, pk2(-s0, -s1));  // G
+      if (kGrad) {  // (gamma + 1 / R) G / R
+        const f2x t = mul2(add2(both(K.gre), rs), rs), u = mul2(kh2, rs);
+        const f2x gr = hr, gi = hi;
+        hr = fma2(t, gr, neg2(mul2(u, gi)));
+        hi = fma2(t, gi, mul2(u, gr));
       }
       if (kHH) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const float f = shpT[I][i] * cI;
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            L[i * 3 + j].x = fmaf(f, M[j].x, L[i * 3 + j].x);
-            L[i * 3 + j].y = fmaf(f, M[j].y, L[i * 3 + j].y);
-          }
+        if (OP == BGB_OP_HELMHOLTZ3D_DLT) {  // times -(x - y) . n_x = -(D - y) . n_x
+          const f2x e = fma2(sub2(yx, both(Dl[0] + Dh[0])), both(nA[0]),
+                             fma2(sub2(yy, both(Dl[1] + Dh[1])), both(nA[1]), mul2(sub2(yz, both(Dl[2] + Dh[2])), both(nA[2]))));
+          hr = mul2(hr, e);
+          hi = mul2(hi, e);
         }
-      } else {
-        S.x = fmaf(Xx, UI[0].x, fmaf(Xy, UI[1].x, fmaf(Xz, UI[2].x, S.x)));
-        S.y = fmaf(Xx, UI[0].y, fmaf(Xy, UI[1].y, fmaf(Xz, UI[2].y, S.y)));
-        Px[0].x = fmaf(Xx, TI.x, Px[0].x); Px[0].y = fmaf(Xx, TI.y, Px[0].y);
-        Px[1].x = fmaf(Xy, TI.x, Px[1].x); Px[1].y = fmaf(Xy, TI.y, Px[1].y);
-        Px[2].x = fmaf(Xz, TI.x, Px[2].x); Px[2].y = fmaf(Xz, TI.y, Px[2].y);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) { Py[c].x += UI[c].x; Py[c].y += UI[c].y; }
-        P0.x += TI.x;
-        P0.y += TI.y;
-      }
-    }
-  } else {
-#pragma unroll
-  for (int I = 0; I < QT; ++I) {
-    if (I >= qt) break;
-    const float4 XI = a4[OA::px(I) / 4];
-    const float Xx = XI.x, Xy = XI.y, Xz = XI.z;
-    const float ax = Dl[0] + Xx, ay = Dl[1] + Xy, az = Dl[2] + Xz;
-    const float wI = XI.w;
-    float2 TI = make_float2(0.f, 0.f);
-    float2 UI[3], EI[3], BI[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) UI[c] = EI[c] = BI[c] = make_float2(0.f, 0.f);
-    float2 M[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) M[c] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int J = 0; J < QB; ++J) {
-      if (J >= qb) break;
-      const float4 YJ = b4[OB::px(J) / 4];
-      const float Yx = YJ.x, Yy = YJ.y, Yz = YJ.z;
-      const float sx = ax - Yx, sy = ay - Yy, sz = az - Yz;
-      const float q = fmaf(sx, D2x + sx, fmaf(sy, D2y + sy, fmaf(sz, D2z + sz, c0)));
-      const float R2 = R0sq + q;
-      const float rs = rsqrt_ftz(R2);
-      const float Rr = R2 * rs;
-      const float delta = q * rcp_ftz(Rr + R0);
-      float psi = fmaf(kh, delta, phi0);
-      const float nn = rintf(psi * kInv2Pi);
-      psi = fmaf(-nn, kPiA, psi);
-      psi = fmaf(-nn, kPiB, psi);
-      float sn, cs;
-      sincos_ftz(psi, &sn, &cs);
-      float amp = wI * YJ.w * rs;
-      if (K.lossy) amp *= amp0 * exp_ftz(-K.gre * delta);
-      const float gr = amp * cs, gi = -amp * sn;
-      if (OP == BGB_OP_HELMHOLTZ3D_SL) {
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          const float g = shpB[J][j];
-          M[j].x = fmaf(gr, g, M[j].x);
-          M[j].y = fmaf(gi, g, M[j].y);
+          const f2x g = *reinterpret_cast<const f2x*>(&shpB[j][2 * J]);
+          Ur[j] = fma2(hr, g, Ur[j]);
+          Ui[j] = fma2(hi, g, Ui[j]);
         }
-      } else if (OP == BGB_OP_MAXWELL3D_SL) {
-        TI.x += gr;
-        TI.y += gi;
-        UI[0].x = fmaf(gr, Yx, UI[0].x); UI[0].y = fmaf(gi, Yx, UI[0].y);
-        UI[1].x = fmaf(gr, Yy, UI[1].x); UI[1].y = fmaf(gi, Yy, UI[1].y);
-        UI[2].x = fmaf(gr, Yz, UI[2].x); UI[2].y = fmaf(gi, Yz, UI[2].y);
       } else {
-        // H = -(gamma + 1/R) G / R ; d = x - y
-        const float g2r = gr * rs, g2i = gi * rs;
-        const float re = K.gre + rs;
-        const float Hx = -(re * g2r - kh * g2i), Hy = -(re * g2i + kh * g2r);
-        const float dx = Dh[0] + sx, dy = Dh[1] + sy, dz = Dh[2] + sz;
-        EI[0].x = fmaf(Hx, dx, EI[0].x); EI[0].y = fmaf(Hy, dx, EI[0].y);
-        EI[1].x = fmaf(Hx, dy, EI[1].x); EI[1].y = fmaf(Hy, dy, EI[1].y);
-        EI[2].x = fmaf(Hx, dz, EI[2].x); EI[2].y = fmaf(Hy, dz, EI[2].y);
-        const float c0x = dy * Yz - dz * Yy, c0y = dz * Yx - dx * Yz, c0z = dx * Yy - dy * Yx;
-        BI[0].x = fmaf(Hx, c0x, BI[0].x); BI[0].y = fmaf(Hy, c0x, BI[0].y);
-        BI[1].x = fmaf(Hx, c0y, BI[1].x); BI[1].y = fmaf(Hy, c0y, BI[1].y);
-        BI[2].x = fmaf(Hx, c0z, BI[2].x); BI[2].y = fmaf(Hy, c0z, BI[2].y);
+        Tr = add2(Tr, hr);
+        Ti = add2(Ti, hi);
+        Ur[0] = fma2(hr, yx, Ur[0]); Ui[0] = fma2(hi, yx, Ui[0]);
+        Ur[1] = fma2(hr, yy, Ur[1]); Ui[1] = fma2(hi, yy, Ui[1]);
+        Ur[2] = fma2(hr, yz, Ur[2]); Ui[2] = fma2(hi, yz, Ui[2]);
       }
     }
-    if (OP == BGB_OP_HELMHOLTZ3D_SL) {
+    const float2 T = make_float2(half_sum(Tr), half_sum(Ti));
+    float2 U[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) U[c] = make_float2(half_sum(Ur[c]), half_sum(Ui[c]));
+    if (kHH) {
+      // double layer: (x - y) . n_y = (D + X_I) . n_y, constant over the trial points
+      const float cI = OP == BGB_OP_HELMHOLTZ3D_DL
+                           ? wI * fmaf(Dh[0] + ax, nB[0], fmaf(Dh[1] + ay, nB[1], (Dh[2] + az) * nB[2]))
+                           : wI;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        const float f = shpT[I][i];
+        const float f = shpT[I][i] * cI;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          L[i * 3 + j].x = fmaf(f, M[j].x, L[i * 3 + j].x);
-          L[i * 3 + j].y = fmaf(f, M[j].y, L[i * 3 + j].y);
-        }
+        for (int j = 0; j < 3; ++j) L[i * 3 + j] = cfm(U[j], f, L[i * 3 + j]);
       }
     } else if (OP == BGB_OP_MAXWELL3D_SL) {
-      S.x = fmaf(Xx, UI[0].x, fmaf(Xy, UI[1].x, fmaf(Xz, UI[2].x, S.x)));
-      S.y = fmaf(Xx, UI[0].y, fmaf(Xy, UI[1].y, fmaf(Xz, UI[2].y, S.y)));
-      Px[0].x = fmaf(Xx, TI.x, Px[0].x); Px[0].y = fmaf(Xx, TI.y, Px[0].y);
-      Px[1].x = fmaf(Xy, TI.x, Px[1].x); Px[1].y = fmaf(Xy, TI.y, Px[1].y);
-      Px[2].x = fmaf(Xz, TI.x, Px[2].x); Px[2].y = fmaf(Xz, TI.y, Px[2].y);
+      const float x = wI * Xx, y = wI * Xy, z = wI * Xz;
+      S = cfm(U[0], x, cfm(U[1], y, cfm(U[2], z, S)));
+      Px[0] = cfm(T, x, Px[0]);
+      Px[1] = cfm(T, y, Px[1]);
+      Px[2] = cfm(T, z, Px[2]);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) { Py[c].x += UI[c].x; Py[c].y += UI[c].y; }
-      P0.x += TI.x;
-      P0.y += TI.y;
+      for (int c = 0; c < 3; ++c) Py[c] = cfm(U[c], wI, Py[c]);
+      P0 = cfm(T, wI, P0);
     } else {
-      // C += X x E_I (stored in Px), A1 += X . B_I (stored in S), B += B_I (Py), E += E_I (stored via L[0..2])
-      Px[0].x += Xy * EI[2].x - Xz * EI[1].x; Px[0].y += Xy * EI[2].y - Xz * EI[1].y;
-      Px[1].x += Xz * EI[0].x - Xx * EI[2].x; Px[1].y += Xz * EI[0].y - Xx * EI[2].y;
-      Px[2].x += Xx * EI[1].x - Xy * EI[0].x; Px[2].y += Xx * EI[1].y - Xy * EI[0].y;
-      S.x = fmaf(Xx, BI[0].x, fmaf(Xy, BI[1].x, fmaf(Xz, BI[2].x, S.x)));
-      S.y = fmaf(Xx, BI[0].y, fmaf(Xy, BI[1].y, fmaf(Xz, BI[2].y, S.y)));
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        Py[c].x += BI[c].x; Py[c].y += BI[c].y;
-        L[c].x += EI[c].x; L[c].y += EI[c].y;
-      }
+      // H = -(gamma + 1 / R) G / R, d = x - y = e + (X_I - y), e = D: with T = -sum H, U = -sum H y,
+      // E = sum H d = U - (D + X_I) T and B = sum H d x y = U x (D + X_I)
+      const float dx = -wI * (Dh[0] + ax), dy = -wI * (Dh[1] + ay), dz = -wI * (Dh[2] + az);
+      const float2 E0 = cfm(T, dx, csc(U[0], wI)), E1 = cfm(T, dy, csc(U[1], wI)), E2 = cfm(T, dz, csc(U[2], wI));
+      const float2 B0 = cfm(U[2], dy, csc(U[1], -dz)), B1 = cfm(U[0], dz, csc(U[2], -dx)),
+                   B2 = cfm(U[1], dx, csc(U[0], -dy));
+      // C += X x E (Px), A1 += X . B (S), B (Py), E (L[0..2])
+      Px[0] = cfm(E2, Xy, cfm(E1, -Xz, Px[0]));
+      Px[1] = cfm(E0, Xz, cfm(E2, -Xx, Px[1]));
+      Px[2] = cfm(E1, Xx, cfm(E0, -Xy, Px[2]));
+      S = cfm(B0, Xx, cfm(B1, Xy, cfm(B2, Xz, S)));
+      Py[0] = cad(Py[0], B0);
+      Py[1] = cad(Py[1], B1);
+      Py[2] = cad(Py[2], B2);
+      L[0] = cad(L[0], E0);
+      L[1] = cad(L[1], E1);
+      L[2] = cad(L[2], E2);
     }
-  }
-
   }
   const float2 alpha = make_float2(K.alpha32[0], K.alpha32[1]);
   if (OP == BGB_OP_HELMHOLTZ3D_HS) {
@@ -779,11 +717,11 @@ struct Smem {
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Trial records staged per chunk (two chunk buffers, the next copied in while the current one is
-// computed) instead of per tile: for the large records of the generic FP32 rules on Lagrange spaces,
-// whose ~6-support hats make wide trial blocks.
+// computed) instead of per tile: for the large records of the generic FP32 rules, which would
+// otherwise bound the tile's width.
 template <class P, int OP, int QB>
 __host__ __device__ constexpr bool chunk_trial_records() {
-  return sizeof(typename P::R) == 4 && is_lagrange_op(OP) && QB > 4;
+  return sizeof(typename P::R) == 4 && QB > 4;
 }
 
 template <class P>
@@ -831,11 +769,10 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
                                           int* s_nonfar) {
   using R = typename P::R;
   using C = typename P::C;
-  constexpr int RT = P::template rec<QT>();
-  constexpr int RB = P::template rec<QB>();
   constexpr int kThreads = P::kThreads;
   const int tid = threadIdx.x;
   const FarScalars S = far_scalars(K);  // registers, not shared-memory loads in the pair loop
+  const int RT = P::template rec<QT>(S.qt), RB = P::template rec<QB>(S.qb);
   const int SC = p.SC, MAXS = p.MAXS;
   Smem<P> s;
   constexpr bool kChunkB = chunk_trial_records<P, OP, QB>();
@@ -859,7 +796,7 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
     s.bndB[i] = p.bnd_b[t];
   }
   if constexpr (sizeof(R) == 4) {  // FP32 records: whole 16-byte groups
-    constexpr int RT4 = RT / 4, RB4 = RB / 4;
+    const int RT4 = RT / 4, RB4 = RB / 4;
     const float4* __restrict__ gT4 = reinterpret_cast<const float4*>(gRT);
     const float4* __restrict__ gB4 = reinterpret_cast<const float4*>(gRB);
     for (int i = tid; i < tm * RT4; i += kThreads) {
@@ -1009,7 +946,7 @@ __device__ __forceinline__ void tile_body(const FarConst& K, const TilePlan& p, 
       C* __restrict__ Lb = s.Lbuf;
       const R* __restrict__ recb = s.recB + (kChunkB ? (c & 1) * SC * RB : sbase * RB);  // this chunk's trial records
       if constexpr (kChunkB) {
-        constexpr int RB4 = RB / 4;
+        const int RB4 = RB / 4;
         const int nn = c + 1 < nch ? min(SC, nbk - sbase - SC) : 0;  // the next chunk's records
         for (int i = tid; i < nn * RB4; i += kThreads) {
           const int r = i / RB4, k = i - r * RB4;
@@ -1204,26 +1141,26 @@ int launch_pair64_t(const FarConst* K, const void* rt, const void* rb, const int
 // ----------------------------------------------------------------------------------------
 // Records
 // ----------------------------------------------------------------------------------------
-template <int Q>
+template <int Q>  // rules of at most Q points
 __global__ void k_prepare_rec32(const Geo64* __restrict__ g, int nt, const __grid_constant__ RuleTable rules, int rule,
                                 double wscale, float* __restrict__ out) {
-  using O = Off32<Q>;
+  using O = Off32;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const Geo64& T = g[t];
-  float* r = out + (int64_t)t * O::SIZE;
+  const int q = rules.npoints[rule], stride = off32_size(q);
+  float* r = out + (int64_t)t * stride;
   double c[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) c[k] = (T.v[0][k] + T.v[1][k] + T.v[2][k]) / 3.0;
-  for (int k = 0; k < O::SIZE; ++k) r[k] = 0.f;  // spare slots
+  for (int k = 0; k < stride; ++k) r[k] = 0.f;  // spare slots
   for (int k = 0; k < 3; ++k) {
     const float hi = (float)c[k];
     r[O::CH + k] = hi;
     r[O::CL + k] = (float)(c[k] - (double)hi);
   }
   r[O::INV2A] = (float)(1.0 / (2.0 * T.area));
-  const int q = rules.npoints[rule];
-  for (int I = 0; I < Q; ++I) {
+  for (int I = 0; I < q + (q & 1); ++I) {
     double u = 0, v = 0, w = 0;
     if (I < q) {
       u = rules.uvw[rules.offset[rule] + I][0];
@@ -1232,7 +1169,7 @@ __global__ void k_prepare_rec32(const Geo64* __restrict__ g, int nt, const __gri
     }
     for (int k = 0; k < 3; ++k) {
       const double x = (T.v[2][k] + T.t[0][k] * u) + T.t[1][k] * v;
-      r[O::px(I) + k] = (float)(x - c[k]);
+      r[O::px(I) + 2 * k] = (float)(x - c[k]);
     }
     r[O::pw(I)] = (float)((w / 2.0) * (2.0 * T.area) * wscale);
   }
@@ -1276,8 +1213,7 @@ template <class P, int OP, int QT, int QB>
 __global__ void k_far_pairs_diag(const __grid_constant__ FarConst K, const typename P::R* __restrict__ rt,
                                  const typename P::R* __restrict__ rb, const int* __restrict__ tau,
                                  const int* __restrict__ sigma, int64_t n, double2* __restrict__ out) {
-  constexpr int RT = P::template rec<QT>();
-  constexpr int RB = P::template rec<QB>();
+  const int RT = P::template rec<QT>(K.qt), RB = P::template rec<QB>(K.qb);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     typename P::C L[9];
     far_pair<P, OP, QT, QB>(far_scalars(K), K, rt + (int64_t)tau[e] * RT, rb + (int64_t)sigma[e] * RB, L);
@@ -1322,8 +1258,8 @@ int occupancy_t(size_t smem_bytes, int* per_sm) {
 }
 
 template <class P, int OP, int QT, int QB>
-size_t smem_t(const TilePlan& p) {
-  return carve<P>(nullptr, p.tmax, p.nmax, P::template rec<QT>(), P::template rec<QB>(), p.FM, p.FN, p.MAXS, p.SC,
+size_t smem_t(const TilePlan& p, int qt, int qb) {
+  return carve<P>(nullptr, p.tmax, p.nmax, P::template rec<QT>(qt), P::template rec<QB>(qb), p.FM, p.FN, p.MAXS, p.SC,
                   p.gmax, p.gsmax, chunk_trial_records<P, OP, QB>(), nullptr);
 }
 

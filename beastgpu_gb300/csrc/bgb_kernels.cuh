@@ -108,12 +108,13 @@ struct FarConst {
   float alpha32[2], beta32[2];
   double far_a[2], far_b[2];   // 3 x 4 rule pair: alpha and beta times its constant factors
   float k_hi, k_lo, gre;       // gamma_im as double-float, gamma_re
-  float shpT[BGB_MAXQ][3], shpB[BGB_MAXQ][3];     // Lagrange hats at rule points
+  float shpT[BGB_MAXQ][3];                        // Lagrange hats at rule points
+  alignas(8) float shpB[3][BGB_MAXQ + 1];         // two points at a time; zero past the rule's
   double shpT64[BGB_MAXQ][3], shpB64[BGB_MAXQ][3];
   // Plain FP64 kernel: with tay_n > 0 the phase of a point pair is k R = k R0 + k (R - R0), R0 the
-  // centroid distance, and exp(-i k (R - R0)) comes from the first tay_n <= 6 terms of the series of
-  // sin and cos (|k (R - R0)| <= k (r_test + r_trial), truncation below 2^-55); tay_s[j] =
-  // (-1)^j / (2j + 1)!, tay_c[j] = (-1)^j / (2j)!.  tay_n = 0: sincos at every point pair.
+  // centroid distance, and exp(-i k (R - R0)) comes from the first tay_n terms (at most 11 for the 3 x 4 rule
+  // pair, 6 for others) of the series of sin and cos (|k (R - R0)| <= k (r_test + r_trial), truncation below
+  // 2^-55); tay_s[j] = (-1)^j / (2j + 1)!, tay_c[j] = (-1)^j / (2j)!.  tay_n = 0: sincos at every point pair.
   int tay_n;
   double tay_s[BGB_TAYLOR_MAX], tay_c[BGB_TAYLOR_MAX];
 };
