@@ -152,7 +152,7 @@ __device__ __forceinline__ float half_sum(f2x a) {
 // Bound by FP32 issue and MUFU (4 per point pair).  Trial points two at a time in packed operations, loops rolled: the
 // scalar form, unrolled over 13 x 13 points with an exit per point, ran ~120 KB of code per pair.  The MFIE's
 // sums come from sum H and sum H y like the EFIE's from sum G and sum G y.  Level-4 EFIE, 6 x 7 points: far stage
-// 7.6 -> 3.9 ms with the per-chunk trial records and strides by the rule's points (60 x 80 tiles instead of
+// 6.9 -> 3.9 ms with the per-chunk trial records and strides by the rule's points (60 x 80 tiles instead of
 // 60 x 64 cut to fit, 1.56 instead of 1.86 times the pairs); unrolled by two 4.7 ms, two CTAs per SM 4.4 - 4.8 ms.
 template <int OP, int QT, int QB>
 __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float (*__restrict__ shpT)[3],

@@ -12,7 +12,9 @@
 // k_gather64: one CTA per output tile.  The local matrices of the next chunk of trial triangles are
 // copied to shared memory (cp.async, 16 B) while the current chunk is added into the entries, in the
 // order of the fused kernel -- trial triangle ascending, then test triangle ascending -- so the result
-// does not depend on tiles or panels.  Bound by L2 / HBM reads.  An odd chunk width keeps the 16-byte
+// does not depend on tiles or panels.  Bound by its FP64 sums (half of the pipe's cycles) and the panel's reads.
+// The copies step through (row, column) without divisions and unit coefficients (hats) cost no product: far
+// stage 47.2 -> 44.9 ms (cube of 6,912 triangles, hats), 31.8 -> 30.4 ms (level-4 EFIE).  An odd chunk width keeps the 16-byte
 // shared-memory reads of consecutive rows free of bank conflicts (rows are SC * 144 B apart).
 #include "bgb_kernels.cuh"
 
@@ -21,14 +23,17 @@
 namespace bgb {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;  // 384 and 512 are within 0.5%
+constexpr int kFetch = kThreads / 9;  // pairs copied per step, nine threads each
+constexpr int kUnit = 1 << 30;        // in a support's code: its coefficient is 1
 
 struct GatherSmem {
   double2* L[2];
   double2* Zs;
   double* fcoef;
   double* gsCoef;
-  int *rowT, *colB, *fcnt, *fcode, *grpFn, *grpOff, *chGrp, *gsCode;
+  int64_t* rowT;  // workspace offset of a test triangle's row
+  int *colB, *fcnt, *fcode, *grpFn, *grpOff, *chGrp, *gsCode;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -49,7 +54,7 @@ __host__ __device__ inline size_t carve64(unsigned char* base, const TilePlan& p
   q = take(sizeof(double2) * (size_t)p.FM * p.FN); if (s) s->Zs = (double2*)q;
   q = take(sizeof(double) * (size_t)p.FM * p.MAXS); if (s) s->fcoef = (double*)q;
   q = take(sizeof(double) * (size_t)p.gsmax); if (s) s->gsCoef = (double*)q;
-  q = take(sizeof(int) * p.tmax); if (s) s->rowT = (int*)q;
+  q = take(sizeof(int64_t) * p.tmax); if (s) s->rowT = (int64_t*)q;
   q = take(sizeof(int) * p.nmax); if (s) s->colB = (int*)q;
   q = take(sizeof(int) * p.FM); if (s) s->fcnt = (int*)q;
   q = take(sizeof(int) * (size_t)p.FM * p.MAXS); if (s) s->fcode = (int*)q;
@@ -86,20 +91,29 @@ __global__ void __launch_bounds__(kThreads) k_gather64(const TilePlan* __restric
   const int b0 = p.bb_off[bn], nbk = p.bb_off[bn + 1] - b0;
   const int f0 = p.tb_fn_off[bm], fm = p.tb_fn_off[bm + 1] - f0;
   const int g0 = p.bb_fn_off[bn], fn = p.bb_fn_off[bn + 1] - g0;
-  for (int i = tid; i < tm; i += kThreads) s.rowT[i] = prow[p.tb_tris[t0 + i]];
-  for (int i = tid; i < nbk; i += kThreads) s.colB[i] = pcol[p.bb_tris[b0 + i]];
+  for (int i = tid; i < tm; i += kThreads) s.rowT[i] = (int64_t)prow[p.tb_tris[t0 + i]] * ncols * 9;
+  for (int i = tid; i < nbk; i += kThreads) s.colB[i] = pcol[p.bb_tris[b0 + i]] * 9;
   __syncthreads();
   // local matrices of chunk c: entry (i, j) of pair (ti, si) at L[(ti * SC + si) * 9 + i * 3 + j]
+  // (nine threads per pair, each stepping through the pairs without a division)
+  const int fp = tid / 9, fk = tid - 9 * fp, fti = fp / SC, fsi = fp - fti * SC, dti = kFetch / SC, dsi = kFetch - dti * SC;
   auto fetch = [&](int c, double2* dst) {
     const int base = c * SC, scn = min(SC, nbk - base);
-    for (int i = tid; i < tm * scn * 9; i += kThreads) {
-      const int pr = i / 9, k = i - 9 * pr, ti = pr / scn, si = pr - ti * scn;
-      cp_async16(dst + (ti * SC + si) * 9 + k, ws + ((int64_t)s.rowT[ti] * ncols + s.colB[base + si]) * 9 + k);
-    }
+    if (fp < kFetch)
+      for (int ti = fti, si = fsi; ti < tm; ti += dti) {
+        if (si < scn) cp_async16(dst + (ti * SC + si) * 9 + fk, ws + (s.rowT[ti] + s.colB[base + si] + fk));
+        si += dsi;
+        if (si >= SC) {
+          si -= SC;
+          ++ti;
+        }
+      }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   const int c0 = p.bb_chunk_off[bn], nch = p.bb_chunk_off[bn + 1] - c0;
-  if (nch > 0) fetch(0, s.L[0]);
+  double2* const L0 = s.L[0];
+  const int lstep = (int)(s.L[1] - L0);  // the two chunk buffers
+  if (nch > 0) fetch(0, L0);
   // supports as offsets into a chunk's matrices
   for (int m = tid; m < fm; m += kThreads) {
     const int a0 = p.fs_off[f0 + m], a1 = p.fs_off[f0 + m + 1];
@@ -122,8 +136,9 @@ __global__ void __launch_bounds__(kThreads) k_gather64(const TilePlan* __restric
   for (int i = tid; i < sb1 - sb0; i += kThreads) {
     const int code = p.gs_code[sb0 + i];  // trial slot << 2 | local
     const int slot = code >> 2;
-    s.gsCode[i] = (slot % SC) * 9 + (code & 3);
-    s.gsCoef[i] = p.gs_coef[sb0 + i];
+    const double cb = p.gs_coef[sb0 + i];
+    s.gsCode[i] = ((slot % SC) * 9 + (code & 3)) | (cb == 1.0 ? kUnit : 0);
+    s.gsCoef[i] = cb;
   }
   for (int i = tid; i < fm * fn; i += kThreads) s.Zs[i] = make_double2(0.0, 0.0);
   // gather roles: row m, groups gq + k * gstep (whole warps of rows when that keeps the groups in flight)
@@ -134,8 +149,8 @@ __global__ void __launch_bounds__(kThreads) k_gather64(const TilePlan* __restric
   for (int c = 0; c < nch; ++c) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();  // chunk c is in shared memory, and nobody reads the other buffer any more
-    const double2* __restrict__ L = s.L[c & 1];
-    if (c + 1 < nch) fetch(c + 1, s.L[(c + 1) & 1]);
+    const double2* __restrict__ L = L0 + (c & 1) * lstep;
+    if (c + 1 < nch) fetch(c + 1, L0 + ((c + 1) & 1) * lstep);
     if (on) {
       const int gg0 = s.chGrp[c], gg1 = s.chGrp[c + 1];
       const int cnt = s.fcnt[m];
@@ -144,13 +159,22 @@ __global__ void __launch_bounds__(kThreads) k_gather64(const TilePlan* __restric
         double2 acc = *z;
         const int q1 = s.grpOff[g + 1];
         for (int q = s.grpOff[g]; q < q1; ++q) {
-          const int col = s.gsCode[q];
-          const double cb = s.gsCoef[q];
-          for (int a = 0; a < cnt; ++a) {
-            const double w = __dmul_rn(s.fcoef[m * MAXS + a], cb);
-            const double2 l = L[s.fcode[m * MAXS + a] + col];
-            acc.x = __fma_rn(w, l.x, acc.x);
-            acc.y = __fma_rn(w, l.y, acc.y);
+          const int code = s.gsCode[q], col = code & (kUnit - 1);
+          if (code & kUnit) {  // hats: the product of the coefficients is the test side's, an FP64 operation less in three
+            for (int a = 0; a < cnt; ++a) {
+              const double w = s.fcoef[m * MAXS + a];
+              const double2 l = L[s.fcode[m * MAXS + a] + col];
+              acc.x = __fma_rn(w, l.x, acc.x);
+              acc.y = __fma_rn(w, l.y, acc.y);
+            }
+          } else {
+            const double cb = s.gsCoef[q];
+            for (int a = 0; a < cnt; ++a) {
+              const double w = __dmul_rn(s.fcoef[m * MAXS + a], cb);
+              const double2 l = L[s.fcode[m * MAXS + a] + col];
+              acc.x = __fma_rn(w, l.x, acc.x);
+              acc.y = __fma_rn(w, l.y, acc.y);
+            }
           }
         }
         *z = acc;
@@ -158,12 +182,14 @@ __global__ void __launch_bounds__(kThreads) k_gather64(const TilePlan* __restric
     }
   }
   __syncthreads();
-  for (int i = tid; i < fm * fn; i += kThreads) {
-    const int n = i / fm, mm = i - n * fm;
-    const int64_t idx = p.rows[f0 + mm] + p.cols[g0 + n] * p.ld;
-    const double2 v = s.Zs[i];
-    if (p.out_c64) ((double2*)p.out)[idx] = v;
-    else ((float2*)p.out)[idx] = make_float2((float)v.x, (float)v.y);
+  for (int n = tid >> 5; n < fn; n += kThreads / 32) {  // output columns by warps, rows by lanes
+    const int64_t col = p.cols[g0 + n] * p.ld;
+    for (int mm = tid & 31; mm < fm; mm += 32) {
+      const int64_t idx = p.rows[f0 + mm] + col;
+      const double2 v = s.Zs[n * fm + mm];
+      if (p.out_c64) ((double2*)p.out)[idx] = v;
+      else ((float2*)p.out)[idx] = make_float2((float)v.x, (float)v.y);
+    }
   }
 }
 
