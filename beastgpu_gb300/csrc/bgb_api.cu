@@ -948,11 +948,12 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     narrow_for_size(prefs, (two_phase ? 2 : far_target_ctas_per_sm(precision)) * (int64_t)h->num_sms, [&](const TileCfg& c) {
       return ((nrows + c.FM - 1) / c.FM) * ((ncols + c.FN - 1) / c.FN);
     });
-  // Bytes of one panel's local matrices: up to 2 GiB (a few hundred trial triangles at 20,000 test
-  // triangles, whose rims add 4 - 8% pairs), within the caller's budget and a quarter of free memory.
+  // Bytes of one panel's local matrices: up to 4 GiB, within the caller's budget and a quarter of free memory.  The
+  // panels' rims are computed twice: with 2 / 4 / 8 GiB the cube of 6,912 triangles takes 48.7 / 46.7 / 45.3 ms
+  // (8, 4 and 0% more pairs), the level-4 sphere 34.1 / 33.3 / 33.4 ms.
   int64_t panel_bytes = 0;
   if (two_phase) {
-    panel_bytes = (int64_t)2 << 30;
+    panel_bytes = (int64_t)4 << 30;
     if (h->cfg.hbm_budget_bytes > 0) panel_bytes = std::min(panel_bytes, h->cfg.hbm_budget_bytes);
     const int64_t all = 144 * (int64_t)test->nt * trial->nt;
     if ((int64_t)h->panel_L[0].cap < std::min(panel_bytes, all)) {
