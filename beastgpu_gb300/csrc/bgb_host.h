@@ -80,6 +80,7 @@ struct bgb_handle {
   // plain FP64 far stage: local matrices of a panel (one per compute stream), workspace row of each test
   // triangle, column of each trial triangle
   bgb::SsTab64 ss_tab{};  // Sauter-Schwab ray tables of the last rule orders (points in ss_pts)
+  bgb::DfTables dfm{};    // the same in double-float (points in df_tab)
   bgb::DevBuf ss_pts, near_list;
   bgb::DevBuf panel_L[2], prow, pcol[2];
   static constexpr int kSlots = 3;  // output-block slots in flight (staging, plan tables, events)
