@@ -110,7 +110,8 @@ std::vector<int> order_functions(const Supports& S, const std::vector<double>& c
       stack.push_back(b);
     }
   };
-  nth = std::max(1, nth);
+  // a thread per ~1000 functions: starting one takes about as long as ordering those
+  nth = std::max(1, std::min(nth, (int)(idx.size() / 1000)));
   std::vector<Range> level{{0, idx.size()}};
   while (nth > 1 && level.size() < 4 * (size_t)nth) {
     std::vector<Range> next;
