@@ -452,7 +452,8 @@ __device__ __forceinline__ void far_pair34_fp64(const FarScalars& K, const doubl
   double th0 = 0.0;
   double2 rot = make_double2(1.0, 0.0);
   if (tn > 0) {
-    th0 = ml(gim, ml(nD, rsqrt_newton(nD)));
+    // 0 for equal centroids (a triangle and the middle one of its refinement); an integer compare
+    if (__double2hiint(nD) >= 0x00100000) th0 = ml(gim, ml(nD, rsqrt_newton(nD)));
     double s0, c0;
     sincos(th0, &s0, &c0);
     rot = make_double2(c0, -s0);
