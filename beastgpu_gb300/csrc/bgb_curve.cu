@@ -697,9 +697,11 @@ __device__ __forceinline__ void far_pair_mixed(const Op& op, const float* fx, co
   const float kf = op.khi;
   if (kf != 0.f) {
     const dfl R0sq = df_add(df_mul(Dx, Dx), df_mul(Dy, Dy));
-    const dfl R0 = df_mul(R0sq, df_rsqrt(R0sq));
-    r0 = R0.hi + R0.lo;
-    phi0 = reduce_2pi(df_mul(R0, dfl{op.khi, op.klo}));
+    if (R0sq.hi >= 1.17549435e-38f) {  // 0 for equal midpoints (a segment and the middle one of its refinement)
+      const dfl R0 = df_mul(R0sq, df_rsqrt(R0sq));
+      r0 = R0.hi + R0.lo;
+      phi0 = reduce_2pi(df_mul(R0, dfl{op.khi, op.klo}));
+    }
     k3 = __fdiv_rn(3.f, kf);
   }
   const float dfx2 = 2.f * dfx, dfy2 = 2.f * dfy;

@@ -176,7 +176,7 @@ __device__ __forceinline__ void far_pair_mixed(const FarScalars& K, const float 
     }
   }
   const float n2 = fmaf(Dh[0], Dh[0], fmaf(Dh[1], Dh[1], Dh[2] * Dh[2]));
-  const float R0 = n2 * rsqrt_ftz(n2);
+  const float R0 = near_root(n2);
   // c0 = |D_hi|^2 - R0^2, exact to double-float accuracy
   float p0, e0, p1, e1, p2, e2, s1, f1, s2, f2, r2h, r2l;
   two_prod(Dh[0], Dh[0], p0, e0);

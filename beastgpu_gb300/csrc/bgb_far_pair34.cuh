@@ -252,6 +252,10 @@ __device__ __forceinline__ void normal34(const T V[3][3], T inv2a, T scale, T n[
   for (int k = 0; k < 3; ++k) n[k] = ml(n[k], s);
 }
 
+// An FP32 number near sqrt(x): 0 below the normal numbers (equal centroids: a triangle and the middle one of its
+// refinement), where the flushed reciprocal root is infinite.
+__device__ __forceinline__ float near_root(float x) { return x >= 1.17549435e-38f ? x * rsqrt_ftz(x) : 0.f; }
+
 // ---- mixed: FP32 with the double-float phase base of far_pair_mixed -------------------------------
 template <int OP>
 __device__ __forceinline__ void far_pair34_mixed(const FarScalars& K, const float* __restrict__ a,
@@ -277,7 +281,7 @@ __device__ __forceinline__ void far_pair34_mixed(const FarScalars& K, const floa
     Dl[1] = __fadd_rn(Dl[1], __fsub_rn(a1.y, b1.y));
     Dl[2] = __fadd_rn(Dl[2], __fsub_rn(a1.z, b1.z));
     const float n2 = fmaf(Dh[0], Dh[0], fmaf(Dh[1], Dh[1], Dh[2] * Dh[2]));
-    R0 = n2 * rsqrt_ftz(n2);
+    R0 = near_root(n2);
     float p0, e0, p1, e1, p2, e2, s1, f1, s2, f2, r2h, r2l;
     two_prod(Dh[0], Dh[0], p0, e0);
     two_prod(Dh[1], Dh[1], p1, e1);

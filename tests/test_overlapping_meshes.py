@@ -43,3 +43,51 @@ def test_equal_centroids_fp64(name, swap):
     got = b.outputs[0].cpu().numpy()
     b.close()
     np.testing.assert_array_equal(got, Z)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", [(3, 4), (4, 6)])
+@pytest.mark.parametrize("swap", [False, True])
+@pytest.mark.parametrize("name", sorted(OPS))
+def test_equal_centroids_mixed(name, swap, rule):
+    make_op, make_space = OPS[name]
+    X, Y = (make_space(m) for m in cubes(swap))
+    op, qs = make_op(wavenumber=1.0), bg.QuadStrat(far_test=rule[0], far_trial=rule[1])
+    ref = oracle.assemble(op, X, Y, qs)
+    # FP32 rounding (6e-8) of R^2 relative to R0^2, (R0 / R)^2 <= 16, in a few terms: below 1e-5
+    for shift in (0.0, 1e-9):  # the second: centroids that differ below FP32 only
+        T = make_space(bg.Mesh(X.mesh.vertices + shift, X.mesh.triangles))
+        Z = bg.assemble_gpu(op, T, Y, bg.GPUConfiguration(precision="mixed"), quadstrat=qs)
+        assert np.linalg.norm(Z - (ref if shift == 0.0 else oracle.assemble(op, T, Y, qs))) <= 1e-5 * np.linalg.norm(ref)
+
+
+def thirds(n):
+    """A square of n segments a side, and the same square with each segment cut in three."""
+    def square(m):
+        c = np.array([[0.0, 0.0], [3.0, 0.0], [3.0, 3.0], [0.0, 3.0]])
+        v = np.concatenate([c[i] + (c[(i + 1) % 4] - c[i]) * np.arange(m)[:, None] / m for i in range(4)])
+        i = np.arange(4 * m, dtype=np.int32)
+        return bg.CurveMesh(v, np.stack([i, (i + 1) % (4 * m)], axis=1))
+    return square(n), square(3 * n)
+
+
+def test_squares_have_far_pairs_with_equal_midpoints():
+    a, b = thirds(2)
+    mid = [m.vertices[m.segments].mean(axis=1) for m in (a, b)]
+    equal = (mid[0][:, None] == mid[1][None]).all(-1)
+    far = oracle.classify_block_curve(bg.curve_lagrangec0d1(a), bg.curve_lagrangec0d1(b), 4.0) == 0
+    assert (equal & far).sum() == 8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", [(4, 4), (4, 6)])
+@pytest.mark.parametrize("name", ["singlelayer", "doublelayer", "doublelayer_transposed", "hypersingular"])
+def test_equal_midpoints_curve(name, rule):
+    a, b = thirds(2)
+    op, qs = getattr(bg.Helmholtz2D, name)(wavenumber=2.0), bg.QuadStrat2D(far_test=rule[0], far_trial=rule[1])
+    for m, n in ((a, b), (b, a)):
+        X, Y = bg.curve_lagrangec0d1(m), bg.curve_lagrangec0d1(n)
+        ref = oracle.assemble_rows_curve(op, X, Y, qs, np.arange(X.nfun, dtype=np.int32))
+        for prec, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+            Z = bg.assemble_gpu(op, X, Y, bg.GPUConfiguration(precision=prec), quadstrat=qs)
+            assert np.linalg.norm(Z - ref) <= tol * np.linalg.norm(ref)
