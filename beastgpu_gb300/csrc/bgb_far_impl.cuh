@@ -99,7 +99,7 @@ namespace farimpl {
 // Records of the generic rules (the 3 x 4 rule pair has its own, bgb_far_pair34.cuh).
 // FP32 record of a triangle, in 16-byte groups read with 128-bit shared-memory loads:
 // [CH.xyz CL.x] [CL.yz - -] [VO (9) INV2A - -], two groups [x0 x1 y0 y1] [z0 z1 w0 w1] per two quadrature points
-// (the operands of packed operations; a last odd point is paired with one of weight zero).  The stride follows
+// (the operands of packed operations; a last odd point is paired with itself at weight zero).  The stride follows
 // the rule's points (6 or 7: 52 floats) and is an odd number of groups, so the records of different triangles
 // start in different bank groups.
 __host__ __device__ constexpr int off32_size(int q) { return 4 * ((5 + q + (q & 1)) | 1); }
@@ -1161,12 +1161,9 @@ __global__ void k_prepare_rec32(const Geo64* __restrict__ g, int nt, const __gri
   }
   r[O::INV2A] = (float)(1.0 / (2.0 * T.area));
   for (int I = 0; I < q + (q & 1); ++I) {
-    double u = 0, v = 0, w = 0;
-    if (I < q) {
-      u = rules.uvw[rules.offset[rule] + I][0];
-      v = rules.uvw[rules.offset[rule] + I][1];
-      w = rules.uvw[rules.offset[rule] + I][2];
-    }
+    // the pad of an odd rule is its last point with weight zero: another place (a vertex) may be a test point
+    const double* p = rules.uvw[rules.offset[rule] + min(I, q - 1)];
+    const double u = p[0], v = p[1], w = I < q ? p[2] : 0.0;
     for (int k = 0; k < 3; ++k) {
       const double x = (T.v[2][k] + T.t[0][k] * u) + T.t[1][k] * v;
       r[O::px(I) + 2 * k] = (float)(x - c[k]);

@@ -91,3 +91,25 @@ def test_equal_midpoints_curve(name, rule):
         for prec, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
             Z = bg.assemble_gpu(op, X, Y, bg.GPUConfiguration(precision=prec), quadstrat=qs)
             assert np.linalg.norm(Z - ref) <= tol * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", [(4, 3), (1, 1), (4, 1), (1, 3)])
+@pytest.mark.parametrize("name", sorted(OPS))
+def test_trial_vertex_in_a_test_point(name, rule):
+    """The centroid of a triangle, a test point of these rules, is a vertex of the mesh that cuts its edges in three:
+    no rule point lies there, so every entry is finite."""
+    make_op, make_space = OPS[name]
+    a, b = bg.plate(1, 0, 0), bg.plate(3, 0, 0)
+    d = np.linalg.norm(centroids(a)[:, None] - b.vertices[None], axis=-1)
+    assert (d < 1e-15).any(axis=1).all()
+    def every_shape(m):  # a function per local shape
+        s = make_space(m)
+        return bg.Space(m, s.refspace, np.arange(3 * m.nt, dtype=np.int32).reshape(-1, 3), np.ones((m.nt, 3)), 3 * m.nt)
+    X, Y = every_shape(a), every_shape(b)
+    op, qs = make_op(wavenumber=1.0), bg.QuadStrat(far_test=rule[0], far_trial=rule[1])
+    ref = oracle.assemble(op, X, Y, qs)
+    Z = bg.assemble_gpu(op, X, Y, bg.GPUConfiguration(precision="mixed"), quadstrat=qs)
+    assert np.isfinite(ref).all() and np.isfinite(Z).all()
+    if name in ("efie", "hh", "hs"):  # (the double layers vanish on a plane)
+        assert np.linalg.norm(Z - ref) <= 1e-5 * np.linalg.norm(ref)
