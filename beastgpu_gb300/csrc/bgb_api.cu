@@ -1544,7 +1544,8 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
         double2* ws = h->panel_L[w].as<double2>();
         int* pcol = h->pcol[w].as<int>();
         if ((rc2 = launch_index_of(cols, q.ncol, pcol, trial->nt, cst)) ||
-            (rc2 = launch_pair64(K.op_kind, gen, dK, T.rec_t, T.rec_b, ti + o_rows, nprow, cols, q.ncol, ws, h->abort_dev, cst)) ||
+            (rc2 = launch_pair64(K.op_kind, gen, dK, T.rec_t, T.rec_b, ti + o_rows, nprow, cols, q.ncol, T.sing_off,
+                                 T.sing_sigma, ws, h->abort_dev, cst)) ||
             (rc2 = launch_place_special(h->ent_tau.as<int>(), h->ent_sigma.as<int>(), nsing, h->prow.as<int>(), pcol,
                                         T.sing_L, q.ncol, ws, cst)) ||
             (rc2 = launch_gather64(dT, ntb * (q.bn1 - q.bn0), q.bn0, h->prow.as<int>(), pcol, ws, q.ncol, smem,

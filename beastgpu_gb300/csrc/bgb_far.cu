@@ -93,11 +93,13 @@ int far_persistent_occupancy(int precision, int op_kind, int generic, size_t sme
 }
 
 int launch_pair64(int op_kind, int generic, const FarConst* K, const void* rt, const void* rb, const int* rows, int nrows,
-                  const int* cols, int ncols, double2* ws, const volatile int* ab, cudaStream_t st) {
-#define BGB_PAIR64_CASE(OP)                                                                            \
-  case OP:                                                                                             \
-    return generic ? launch_pair64_t<OP, BGB_MAXQ, BGB_MAXQ>(K, rt, rb, rows, nrows, cols, ncols, ws, ab, st) \
-                   : launch_pair64_t<OP, 3, 4>(K, rt, rb, rows, nrows, cols, ncols, ws, ab, st)
+                  const int* cols, int ncols, const int64_t* sing_off, const int* sing_sigma, double2* ws,
+                  const volatile int* ab, cudaStream_t st) {
+#define BGB_PAIR64_CASE(OP)                                                                                   \
+  case OP:                                                                                                    \
+    return generic ? launch_pair64_t<OP, BGB_MAXQ, BGB_MAXQ>(K, rt, rb, rows, nrows, cols, ncols, sing_off,   \
+                                                             sing_sigma, ws, ab, st)                          \
+                   : launch_pair64_t<OP, 3, 4>(K, rt, rb, rows, nrows, cols, ncols, sing_off, sing_sigma, ws, ab, st)
   switch (op_kind) {
     BGB_PAIR64_CASE(BGB_OP_HELMHOLTZ3D_SL);
     BGB_PAIR64_CASE(BGB_OP_MAXWELL3D_SL);

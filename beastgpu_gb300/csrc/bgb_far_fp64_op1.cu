@@ -11,8 +11,9 @@ template int launch_persistent_t<PFp64, 1, BGB_MAXQ, BGB_MAXQ>(const FarConst*, 
 template int occupancy_t<PFp64, 1, 3, 4>(size_t, int*);
 template int occupancy_t<PFp64, 1, BGB_MAXQ, BGB_MAXQ>(size_t, int*);
 template int launch_pair64_t<1, 3, 4>(const FarConst*, const void*, const void*, const int*, int, const int*, int,
-                                       double2*, const volatile int*, cudaStream_t);
+                                       const int64_t*, const int*, double2*, const volatile int*, cudaStream_t);
 template int launch_pair64_t<1, BGB_MAXQ, BGB_MAXQ>(const FarConst*, const void*, const void*, const int*, int,
-                                                     const int*, int, double2*, const volatile int*, cudaStream_t);
+                                                     const int*, int, const int64_t*, const int*, double2*,
+                                                     const volatile int*, cudaStream_t);
 }  // namespace farimpl
 }  // namespace bgb

@@ -659,14 +659,47 @@ __device__ __forceinline__ FarScalars far_scalars(const FarConst& K) {
   return S;
 }
 
+// Points that lie close to each other against the centroid distance (a small triangle over the inside of a large one):
+// E + H + d, a sum of terms of size |D|^2, carries eps (R0 / R)^2 into R^2, the points' difference eps R0 / R, as far as
+// the points themselves are known.  A function of its own: as a branch inside the pair code it cost the level-4 EFIE 6%
+// (33.2 -> 35.4 ms), by the registers that stay live and the code that no longer overlaps.
+template <int OP>
+__device__ __noinline__ void far_pair34_fp64_close(const FarConst& K, const double* __restrict__ a,
+                                                   const double* __restrict__ b, double2* __restrict__ L) {
+  double2 t[9];
+  far_pair34_fp64<OP, true>(far_scalars(K), K.tay_s, K.tay_c, a, b, t);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) L[k] = t[k];
+}
+// True below R0 = 3.3 - 3.5 times the larger of the point radii (beyond, R > 0.38 R0): triangles next to each other.
+// By exponents (n < 10.7 - 12 times the radius squared), beside the FP64 pipe.  Pairs without common vertices reach it
+// on no mesh of even triangles; on the box of right triangles 3.7 would take in four per triangle, whose second pass
+// cost the 8 x 8 box 26 of 590 us.
+__device__ __forceinline__ bool far_pair34_is_close(const double* __restrict__ a, const double* __restrict__ b) {
+  double n = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) n = fm(sb(a[k], b[k]), sb(a[k], b[k]), n);
+  int top = max(__double2hiint(a[12]), __double2hiint(b[12]));
+#pragma unroll
+  for (int i = 1; i < 3; ++i) top = max(top, max(__double2hiint(a[12 + i]), __double2hiint(b[12 + i])));
+  return __double2hiint(n) < top + 0x00380000;
+}
+
 template <class P, int OP, int QT, int QB>
 __device__ __forceinline__ void far_pair(const FarScalars& S, const FarConst& K, const typename P::R* a,
                                          const typename P::R* b, typename P::C L[9]) {
   if constexpr (QT == 3 && QB == 4 && sizeof(typename P::R) == 4)
     far_pair34_mixed<OP>(S, a, b, L);
-  else if constexpr (QT == 3 && QB == 4)
-    far_pair34_fp64<OP>(S, K.tay_s, K.tay_c, a, b, L);
-  else if constexpr (sizeof(typename P::R) == 4)
+  else if constexpr (QT == 3 && QB == 4) {
+    if (far_pair34_is_close(a, b)) {
+      double2 t[9];
+      far_pair34_fp64_close<OP>(K, a, b, t);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) L[k] = t[k];
+    } else {
+      far_pair34_fp64<OP, false>(S, K.tay_s, K.tay_c, a, b, L);
+    }
+  } else if constexpr (sizeof(typename P::R) == 4)
     far_pair_mixed<OP, QT, QB>(S, K.shpT, K.shpB, a, b, L);
   else
     far_pair_fp64<OP, QT, QB>(S, K.shpT64, K.shpB64, K.tay_s, K.tay_c, a, b, L);
@@ -1092,6 +1125,8 @@ __global__ void __launch_bounds__(kPairSide * kPairSide, 2) k_pair64(const FarCo
                                                                      const double* __restrict__ rec_b,
                                                                      const int* __restrict__ rows, int nrows,
                                                                      const int* __restrict__ cols, int ncols,
+                                                                     const int64_t* __restrict__ sing_off,
+                                                                     const int* __restrict__ sing_sigma,
                                                                      double2* __restrict__ ws,
                                                                      const volatile int* abort_flag) {
   constexpr int RT = PFp64::rec<QT>(), RB = PFp64::rec<QB>();
@@ -1115,16 +1150,26 @@ __global__ void __launch_bounds__(kPairSide * kPairSide, 2) k_pair64(const FarCo
   if (stop) return;
   const int ti = tid / kPairSide, si = tid - ti * kPairSide;
   if (ti >= nr || si >= nc) return;
-  double2 L[9];
-  far_pair<PFp64, OP, QT, QB>(far_scalars(K), K, sT + ti * RT, sB + si * RB, L);
   double2* o = ws + ((int64_t)(r0 + ti) * ncols + c0 + si) * 9;
+  const double *a = sT + ti * RT, *b = sB + si * RB;
+  double2 L[9];
+  if constexpr (QT == 3 && QB == 4) {
+    if (far_pair34_is_close(a, b)) {  // singular and near pairs, whose matrices are placed afterwards, and a few others
+      if (find_sigma(sing_off, sing_sigma, rows[r0 + ti], cols[c0 + si]) < 0) far_pair34_fp64_close<OP>(K, a, b, o);
+      return;
+    }
+    far_pair34_fp64<OP, false>(far_scalars(K), K.tay_s, K.tay_c, a, b, L);
+  } else {
+    far_pair<PFp64, OP, QT, QB>(far_scalars(K), K, a, b, L);
+  }
 #pragma unroll
   for (int k = 0; k < 9; ++k) o[k] = L[k];
 }
 
 template <int OP, int QT, int QB>
 int launch_pair64_t(const FarConst* K, const void* rt, const void* rb, const int* rows, int nrows, const int* cols,
-                    int ncols, double2* ws, const volatile int* abort_flag, cudaStream_t st) {
+                    int ncols, const int64_t* sing_off, const int* sing_sigma, double2* ws, const volatile int* abort_flag,
+                    cudaStream_t st) {
   if (nrows <= 0 || ncols <= 0) return 0;
   // rows along y in runs of at most 65535 blocks (a grid's limit)
   const int step = 65535 * kPairSide;
@@ -1132,7 +1177,8 @@ int launch_pair64_t(const FarConst* K, const void* rt, const void* rb, const int
     const int n = std::min(step, nrows - r);
     const dim3 grid((ncols + kPairSide - 1) / kPairSide, (n + kPairSide - 1) / kPairSide);
     k_pair64<OP, QT, QB><<<grid, kPairSide * kPairSide, 0, st>>>(K, (const double*)rt, (const double*)rb, rows + r, n,
-                                                                 cols, ncols, ws + (int64_t)r * ncols * 9, abort_flag);
+                                                                 cols, ncols, sing_off, sing_sigma,
+                                                                 ws + (int64_t)r * ncols * 9, abort_flag);
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "k_pair64 launch");
@@ -1288,10 +1334,11 @@ int launch_diag_t(const FarConst& K, const void* rt, const void* rb, const int* 
 
 #define BGB_PAIR64_EXTERN(OP)                                                                                       \
   extern template int launch_pair64_t<OP, 3, 4>(const FarConst*, const void*, const void*, const int*, int,        \
-                                                const int*, int, double2*, const volatile int*, cudaStream_t);    \
+                                                const int*, int, const int64_t*, const int*, double2*,             \
+                                                const volatile int*, cudaStream_t);                                \
   extern template int launch_pair64_t<OP, BGB_MAXQ, BGB_MAXQ>(const FarConst*, const void*, const void*, const int*, \
-                                                              int, const int*, int, double2*, const volatile int*,   \
-                                                              cudaStream_t);
+                                                              int, const int*, int, const int64_t*, const int*,      \
+                                                              double2*, const volatile int*, cudaStream_t);
 
 }  // namespace farimpl
 }  // namespace bgb

@@ -397,7 +397,8 @@ __device__ __forceinline__ double rsqrt_newton(double x) {
 // The phase is k R = k R0 + k (R - R0) with R0 the centroid distance: exp(-i k R0) is a factor of the whole
 // local matrix, and cos / sin of the small k (R - R0) come from tay_n terms of their series for all
 // four trial points together (sincos of k R where the series would be long).
-template <int OP>
+// CLOSE: the points' differences are squared; otherwise R^2 = E + H + d.
+template <int OP, bool CLOSE>
 __device__ __forceinline__ void far_pair34_fp64(const FarScalars& K, const double* __restrict__ tay_s,
                                                 const double* __restrict__ tay_c, const double* __restrict__ a,
                                                 const double* __restrict__ b, double2 L[9]) {
@@ -469,7 +470,18 @@ __device__ __forceinline__ void far_pair34_fp64(const FarScalars& K, const doubl
     double2 g[4];
 #pragma unroll
     for (int J = 0; J < 4; ++J) {
-      const double R2 = J == 0 ? E[I] : ad(ad(E[I], H[J - 1]), d[I][J - 1]);
+      double R2;
+      if (CLOSE) {
+        double x[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          x[k] = fm(0.5, G.V[I][k], D[k]);
+          if (J > 0) x[k] = ad(x[k], G.W[J - 1][k]);
+        }
+        R2 = dot(x, x);
+      } else {
+        R2 = J == 0 ? E[I] : ad(ad(E[I], H[J - 1]), d[I][J - 1]);
+      }
       rinv[J] = rsqrt_newton(R2);
       R[J] = ml(R2, rinv[J]);
     }
