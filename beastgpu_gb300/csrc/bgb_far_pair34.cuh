@@ -29,8 +29,9 @@ namespace farimpl {
 
 // FP32 record: five 16-byte groups [CH.xyz area] [CL.xyz 1/(2A)] [V_i.xyz |x_i|^2] x 3, V_i scaled by -0.4
 // on the trial side (an odd number of groups: the records of different triangles start in different banks).
-// FP64 record: centroid, the three offsets, |x_i|^2, area, 1/(2A).
-constexpr int kRec34F = 20, kRec34D = 17;
+// FP64 record: centroid, the three offsets, |x_i|^2, area, 1/(2A), unit normal; an odd stride (the 8-byte reads of
+// different triangles start in different banks).
+constexpr int kRec34F = 20, kRec34D = 21;
 // Factor of the trial records' areas: the hats' constants (rule weights, 1/(4 pi), 1/5), in FP64 before
 // the FP32 records are rounded.
 constexpr double kHatScale34 = 0.2 * 25.0 / 144.0 * BGB_INV_4PI_D;
@@ -243,11 +244,12 @@ __device__ __forceinline__ void mfie_tables(PairGeo34<T>& G, const T D[3]) {
   }
 }
 
-// Unit normal V_0 x V_1 * 3 / (2A) (the trial side's offsets carry -0.4: scale 6.25).
-template <class T>
-__device__ __forceinline__ void normal34(const T V[3][3], T inv2a, T scale, T n[3]) {
+// FP32: unit normal V_0 x V_1 * 3 / (2A) (the trial side's offsets carry -0.4: scale 18.75).  It takes the offsets' sum
+// for zero, which holds to eps64 times the centroid's coordinates: below FP32, so the FP64 path has the normal in its
+// record instead, from edges (10 to 15 times the error at 1000 edges from the origin otherwise).
+__device__ __forceinline__ void normal34(const float V[3][3], float inv2a, float scale, float n[3]) {
   cross(V[0], V[1], n);
-  const T s = ml(inv2a, scale);
+  const float s = ml(inv2a, scale);
 #pragma unroll
   for (int k = 0; k < 3; ++k) n[k] = ml(n[k], s);
 }
@@ -430,9 +432,7 @@ __device__ __forceinline__ void far_pair34_fp64(const FarScalars& K, const doubl
     for (int q = 0; q < 3; ++q) d[I][q] = dot(G.V[I], G.W[q]);
   double eI[3] = {0, 0, 0}, eq[4] = {0, 0, 0, 0}, nn = 0.0;
   if (kDL || kDLT || kHS) {
-    double nt[3] = {0, 0, 0}, ns[3] = {0, 0, 0};
-    if (kDLT || kHS) normal34(G.V, a[16], 3.0, nt);
-    if (kDL || kHS) normal34(G.W, b[16], 18.75, ns);
+    const double nt[3] = {a[17], a[18], a[19]}, ns[3] = {b[17], b[18], b[19]};
     if (kDL) {
       const double e = dot(D, ns);
 #pragma unroll
@@ -563,6 +563,12 @@ __global__ void k_prepare_rec34(const Geo64* __restrict__ g, int nt, double scal
       r[(f32 ? 8 + 4 * i : 3 + 3 * i) + k] = (T)(scale * v);
     }
     r[f32 ? 11 + 4 * i : 12 + i] = (T)(x2 * s);
+  }
+  if (!f32) {
+    double n[3];
+    cross(S.t[0], S.t[1], n);
+    for (int k = 0; k < 3; ++k) r[17 + k] = (T)(n[k] * inv2a);
+    r[20] = (T)0;
   }
 }
 
