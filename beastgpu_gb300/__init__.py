@@ -4,6 +4,6 @@ from .spaces import Space, raviartthomas, lagrangec0d1, lagrangecxd0, REFSPACE_R
 from .operators import Helmholtz3D, Maxwell3D, Operator, QuadStrat, defaultquadstrat  # noqa: F401
 from .api import (assemble_gpu, assemble, classify, local_matrices, GPUConfiguration, row_shard,  # noqa: F401
                   GpuWriteBackTrueInstance, GpuWriteBackFalseInstance, measure_issue_peaks, Batch,
-                  assemble_batch, local_matrices_curve)
+                  assemble_batch, local_matrices_curve, release_memory)
 from .curves import (CurveMesh, CurveSpace, circle, ellipse, arc, union, curve_lagrangec0d1,  # noqa: F401
                      curve_lagrangecxd0, Helmholtz2D, Operator2D, QuadStrat2D, defaultquadstrat2d)

@@ -87,6 +87,7 @@ SIGNATURES = {
     "bgb_last_error": ([], C.c_char_p),
     "bgb_create": ([C.POINTER(C.c_void_p), C.POINTER(Config)], C.c_int),
     "bgb_destroy": ([C.c_void_p], C.c_int),
+    "bgb_trim": ([C.c_void_p], C.c_int),
     "bgb_abort": ([C.c_void_p], C.c_int),
     "bgb_tile_info": ([C.c_void_p, C.c_int32], C.c_int),
     "bgb_measure_issue_peaks": ([C.c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_double),

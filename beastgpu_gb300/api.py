@@ -60,8 +60,11 @@ class GPUConfiguration:
     precision: "fp64" (plain all-FP64 kernels, the drop-in) or "mixed" (FP32 far pairs with
     double-float phase base, FP64-accurate singular and near pairs).
     total_GPU_budget: HBM bytes the call may use for the output staging (0 = 90% of free);
-    host outputs are produced in blocks of columns of at most a quarter of it (two device
+    host outputs are produced in blocks of columns of at most a quarter of it (three device
     staging buffers), and large outputs in about 16 blocks so that copies overlap the fill.
+    What it leaves bounds the local matrices that an FP64 call keeps per panel of triangle pairs
+    (0: up to 4 GiB, two times that for host outputs in blocks, of a quarter of free memory each).
+    These buffers stay with the handle of the configuration: release_memory() gives them back.
     pinned_ring_bytes: size of each half of the pinned host ring that pageable host outputs
     are copied through when the device cannot write pageable memory directly (0 = 512 MiB).
     pageable_via_ring: use the ring even where the device writes pageable memory directly.
@@ -127,6 +130,14 @@ def get_handle(device: int = 0, hbm_budget: int = 0, tile_config: int = -1, pinn
             h = Handle(device, hbm_budget, tile_config, pinned_ring, flags)
             _handles[key] = h
         return h
+
+
+def release_memory():
+    """Give back the large device buffers that assembly calls keep for the next one (bgb_trim)."""
+    with _hlock:
+        handles = list(_handles.values())
+    for h in handles:
+        _lib.check(_lib.load().bgb_trim(h.ptr))
 
 
 class _Keep:

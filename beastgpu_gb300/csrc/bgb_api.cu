@@ -686,6 +686,18 @@ int bgb_create(bgb_handle** out, const bgb_config* cfg) {
   return 0;
 }
 
+int bgb_trim(bgb_handle* h) {
+  if (!h) { set_error("handle is NULL"); return BGB_ERR_INVALID; }
+  std::lock_guard<std::mutex> lk(h->mu);
+  BGB_CUDA(cudaSetDevice(h->device));
+  for (cudaStream_t s : {h->stream, h->copy_stream, h->stream2, h->stream_sing, h->stream_up})
+    if (s) BGB_CUDA(cudaStreamSynchronize(s));
+  for (DevBuf& b : h->panel_L) b.release();
+  for (DevBuf& b : h->stage) b.release();
+  h->sing_L.release();
+  return 0;
+}
+
 int bgb_destroy(bgb_handle* h) {
   if (!h) return 0;
   cudaSetDevice(h->device);
@@ -947,33 +959,50 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   // uploads, classifies and integrates the singular pairs.
   const bool pinned_cfg = h->cfg.tile_config >= 0;
   if (pinned_cfg && h->cfg.tile_config >= kNumTileCfgs) { set_error("tile_config %d out of range", h->cfg.tile_config); return BGB_ERR_INVALID; }
-  std::vector<int> prefs;
-  if (pinned_cfg) prefs.push_back(h->cfg.tile_config);
-  else if (test->refspace == BGB_REFSPACE_LAGRANGE_C0D1 && precision == BGB_PREC_MIXED)
-    prefs.assign(kPrefLagrange, kPrefLagrange + kNumPrefLagrange);
-  else if (test->refspace == BGB_REFSPACE_LAGRANGE_C0D1)
-    prefs.assign(kPrefGatherLagrange, kPrefGatherLagrange + kNumPrefGatherLagrange);
-  else if (precision == BGB_PREC_MIXED) prefs.assign(kPrefMixed, kPrefMixed + kNumPrefMixed);
-  else prefs.assign(kPrefGather, kPrefGather + kNumPrefGather);
   // The plain FP64 path computes the pairs of a panel once and gathers the tiles from them
-  // (bgb_gather64.cu); the mixed path computes them inside the tiles.
-  const bool two_phase = precision == BGB_PREC_FP64;
-  if (!pinned_cfg)
-    narrow_for_size(prefs, (two_phase ? 2 : far_target_ctas_per_sm(precision)) * (int64_t)h->num_sms, [&](const TileCfg& c) {
-      return ((nrows + c.FM - 1) / c.FM) * ((ncols + c.FN - 1) / c.FN);
-    });
-  // Bytes of one panel's local matrices: up to 4 GiB, within the caller's budget and a quarter of free memory.  The
-  // panels' rims are computed twice: with 2 / 4 / 8 GiB the cube of 6,912 triangles takes 48.7 / 46.7 / 45.3 ms
-  // (8, 4 and 0% more pairs), the level-4 sphere 34.1 / 33.3 / 33.4 ms.
+  // (bgb_gather64.cu); the mixed path computes them inside the tiles, and so does the FP64 path where no panel fits.
+  bool two_phase = precision == BGB_PREC_FP64;
+  std::vector<int> prefs;
+  auto choose_prefs = [&] {
+    const bool lagrange = test->refspace == BGB_REFSPACE_LAGRANGE_C0D1, mixed = precision == BGB_PREC_MIXED;
+    if (pinned_cfg) {
+      prefs.assign(1, h->cfg.tile_config);
+      return;
+    }
+    if (two_phase && lagrange) prefs.assign(kPrefGatherLagrange, kPrefGatherLagrange + kNumPrefGatherLagrange);
+    else if (two_phase) prefs.assign(kPrefGather, kPrefGather + kNumPrefGather);
+    else if (mixed && lagrange) prefs.assign(kPrefLagrange, kPrefLagrange + kNumPrefLagrange);
+    else if (mixed) prefs.assign(kPrefMixed, kPrefMixed + kNumPrefMixed);
+    else if (lagrange) prefs.assign(kPrefLagrangeFp64, kPrefLagrangeFp64 + kNumPrefLagrangeFp64);
+    else prefs.assign(kPrefFp64, kPrefFp64 + kNumPrefFp64);
+    if (two_phase || mixed)  // (the lists of the fused FP64 tiles are not in order of width)
+      narrow_for_size(prefs, (two_phase ? 2 : far_target_ctas_per_sm(precision)) * (int64_t)h->num_sms, [&](const TileCfg& c) {
+        return ((nrows + c.FM - 1) / c.FM) * ((ncols + c.FN - 1) / c.FN);
+      });
+  };
+  choose_prefs();
+  // Bytes of one panel's local matrices: up to 4 GiB, within what the caller's budget leaves beside the staging of
+  // host outputs, and a quarter of the memory that is free beside it; an even share each where two compute streams
+  // need one.  The panels' rims are computed twice: with 2 / 4 / 8 GiB the cube of 6,912 triangles takes
+  // 48.7 / 46.7 / 45.3 ms (8, 4 and 0% more pairs), the level-4 sphere 34.1 / 33.3 / 33.4 ms.
+  const int npanels = std::min(2, nblocks);
   int64_t panel_bytes = 0;
   if (two_phase) {
+    const int nstage = host_out ? std::min((int)bgb_handle::kSlots, nblocks) : 0;
+    const int64_t staged = cols_per_block * per_col;
     panel_bytes = (int64_t)4 << 30;
-    if (h->cfg.hbm_budget_bytes > 0) panel_bytes = std::min(panel_bytes, h->cfg.hbm_budget_bytes);
-    const int64_t all = 144 * (int64_t)test->nt * trial->nt;
-    if ((int64_t)h->panel_L[0].cap < std::min(panel_bytes, all)) {
+    if (h->cfg.hbm_budget_bytes > 0)
+      panel_bytes = std::min(panel_bytes, (h->cfg.hbm_budget_bytes - nstage * staged) / npanels);
+    const int64_t need = std::min(panel_bytes, 144 * (int64_t)test->nt * trial->nt);
+    bool held = true;
+    for (int k = 0; k < npanels; ++k) held = held && (int64_t)h->panel_L[k].cap >= need;
+    for (int k = 0; k < nstage; ++k) held = held && (int64_t)h->stage[k].cap >= staged;
+    if (!held) {
       size_t freeb = 0, totalb = 0;
       cudaMemGetInfo(&freeb, &totalb);
-      panel_bytes = std::min(panel_bytes, (int64_t)(freeb + h->panel_L[0].cap + h->panel_L[1].cap) / 4);
+      int64_t rest = (int64_t)(freeb + h->panel_L[0].cap + h->panel_L[1].cap);
+      for (int k = 0; k < nstage; ++k) rest -= std::max<int64_t>(0, staged - (int64_t)h->stage[k].cap);
+      panel_bytes = std::min(panel_bytes, rest / 4);
     }
   }
   int smem_max = 0;
@@ -997,6 +1026,7 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
   const int nth = planner_threads();
   const int target_occ = far_target_ctas_per_sm(precision);
   auto plan_all = [&]() {
+    PL = Plans();
     const auto t0 = clk::now();
     cudaSetDevice(h->device);  // occupancy queries from this thread
     const Supports St = build_supports(test);
@@ -1024,105 +1054,127 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
       for (auto& x : th) x.join();
     };
     size_t smem = 0;
-    for (int id : prefs) {
-      const TileCfg tc = kTileCfgs[id];
-      // the two sides beside each other: the first levels of a bisection are serial (level-5 EFIE: 4.6 ms one
-      // after the other, longer than the classification and the singular pairs that hide it)
-      auto test_side = [&] {
-        if (tc.FM != ord_fm) {
-          ord_t = order_functions(St, cent_t, (int)row0, (int)(row0 + nrows), tc.FM, nth);
-          // rows of a tile in ascending order: the tile's output stores of one column then fall in
-          // fewer 32-byte sectors (C2: 23 instead of 60 per column)
-          for (size_t b = 0; b < ord_t.size(); b += (size_t)tc.FM)
-            std::sort(ord_t.begin() + b, ord_t.begin() + std::min(ord_t.size(), b + (size_t)tc.FM));
-          ord_fm = tc.FM;
-        }
-        PL.test = HostPlan();
-        plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth);
-      };
-      auto trial_side = [&](bool same_order) {
-        if (tc.FN != ord_fn) {
-          if (same_order)
-            ord_b[0] = ord_t;  // the same functions and width: the same order
-          else
-            over_blocks([&](int b, int threads) {
-              ord_b[b] = order_functions(Sb, cent_b, (int)col_start[b], (int)col_start[b + 1], tc.FN, threads);
-            });
-          ord_fn = tc.FN;
-        }
-        PL.trial.assign(nblocks, HostPlan());
-        over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, tc.SC, PL.trial[b], threads); });
-      };
-      if (same && nblocks == 1 && row0 == 0 && nrows == ncols && tc.FN == tc.FM) {
-        test_side();
-        trial_side(true);
-      } else if (nrows + ncols < 2000) {  // a thread costs more than the overlap gives
-        test_side();
-        trial_side(false);
-      } else {
-        parallel_for(2, 2, [&](int side) {
-          if (side)
-            trial_side(false);
-          else
-            test_side();
-        });
-      }
-      // Chunks of tc.SC trial triangles; a tile pinned by the caller, and the last choice, also with
-      // narrower chunks when the chunk buffers do not fit (the result does not depend on the chunks).
-      for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
-        TilePlan probe{};
-        probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = sc; probe.MAXS = PL.test.MAXS;
-        probe.tmax = std::max(1, PL.test.tmax);
-        if (sc != tc.SC) {
+    auto plan_tiles = [&] {
+      for (int id : prefs) {
+        const TileCfg tc = kTileCfgs[id];
+        // the two sides beside each other: the first levels of a bisection are serial (level-5 EFIE: 4.6 ms one
+        // after the other, longer than the classification and the singular pairs that hide it)
+        auto test_side = [&] {
+          if (tc.FM != ord_fm) {
+            ord_t = order_functions(St, cent_t, (int)row0, (int)(row0 + nrows), tc.FM, nth);
+            // rows of a tile in ascending order: the tile's output stores of one column then fall in
+            // fewer 32-byte sectors (C2: 23 instead of 60 per column)
+            for (size_t b = 0; b < ord_t.size(); b += (size_t)tc.FM)
+              std::sort(ord_t.begin() + b, ord_t.begin() + std::min(ord_t.size(), b + (size_t)tc.FM));
+            ord_fm = tc.FM;
+          }
+          PL.test = HostPlan();
+          plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth);
+        };
+        auto trial_side = [&](bool same_order) {
+          if (tc.FN != ord_fn) {
+            if (same_order)
+              ord_b[0] = ord_t;  // the same functions and width: the same order
+            else
+              over_blocks([&](int b, int threads) {
+                ord_b[b] = order_functions(Sb, cent_b, (int)col_start[b], (int)col_start[b + 1], tc.FN, threads);
+              });
+            ord_fn = tc.FN;
+          }
           PL.trial.assign(nblocks, HostPlan());
-          over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
-        }
-        for (int b = 0; b < nblocks; ++b) {
-          probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
-          probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
-          probe.nmax = std::max(probe.nmax, std::max(1, PL.trial[b].nmax));
-        }
-        int occ = 0;
-        if (two_phase) {
-          smem = gather64_smem_bytes(probe);
-          if (gather64_occupancy(smem, &occ)) occ = 0;
+          over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, tc.SC, PL.trial[b], threads); });
+        };
+        if (same && nblocks == 1 && row0 == 0 && nrows == ncols && tc.FN == tc.FM) {
+          test_side();
+          trial_side(true);
+        } else if (nrows + ncols < 2000) {  // a thread costs more than the overlap gives
+          test_side();
+          trial_side(false);
         } else {
-          smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
-          // Occupancy: when the widest test tile pushes shared memory past what the kernel's
-          // CTAs per SM allow, cap the triangles per test tile at the largest count that fits.
-          if (smem <= (size_t)smem_max && far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ) == 0 &&
-              occ >= 1 && occ < target_occ) {
-            int cap = -1;
-            for (int t = probe.tmax - 1; t >= std::max(1, PL.test.MAXS); --t) {
-              TilePlan q = probe;
-              q.tmax = t;
-              const size_t sm = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, q);
-              int o = 0;
-              if (far_persistent_occupancy(precision, K.op_kind, gen, sm, &o) == 0 && o >= target_occ) {
-                cap = t;
-                break;
+          parallel_for(2, 2, [&](int side) {
+            if (side)
+              trial_side(false);
+            else
+              test_side();
+          });
+        }
+        // Chunks of tc.SC trial triangles; a tile pinned by the caller, and the last choice, also with
+        // narrower chunks when the chunk buffers do not fit (the result does not depend on the chunks).
+        for (int sc = tc.SC; sc >= 1 && PL.cfg_id < 0; sc /= 2) {
+          TilePlan probe{};
+          probe.FM = tc.FM; probe.FN = tc.FN; probe.SC = sc; probe.MAXS = PL.test.MAXS;
+          probe.tmax = std::max(1, PL.test.tmax);
+          if (sc != tc.SC) {
+            PL.trial.assign(nblocks, HostPlan());
+            over_blocks([&](int b, int threads) { plan_trial_side_par(Sb, ord_b[b], tc.FN, sc, PL.trial[b], threads); });
+          }
+          for (int b = 0; b < nblocks; ++b) {
+            probe.gmax = std::max(probe.gmax, PL.trial[b].gmax);
+            probe.gsmax = std::max(probe.gsmax, PL.trial[b].gsmax);
+            probe.nmax = std::max(probe.nmax, std::max(1, PL.trial[b].nmax));
+          }
+          int occ = 0;
+          if (two_phase) {
+            smem = gather64_smem_bytes(probe);
+            if (gather64_occupancy(smem, &occ)) occ = 0;
+          } else {
+            smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
+            // Occupancy: when the widest test tile pushes shared memory past what the kernel's
+            // CTAs per SM allow, cap the triangles per test tile at the largest count that fits.
+            if (smem <= (size_t)smem_max && far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ) == 0 &&
+                occ >= 1 && occ < target_occ) {
+              int cap = -1;
+              for (int t = probe.tmax - 1; t >= std::max(1, PL.test.MAXS); --t) {
+                TilePlan q = probe;
+                q.tmax = t;
+                const size_t sm = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, q);
+                int o = 0;
+                if (far_persistent_occupancy(precision, K.op_kind, gen, sm, &o) == 0 && o >= target_occ) {
+                  cap = t;
+                  break;
+                }
+              }
+              if (cap > 0) {
+                PL.test = HostPlan();
+                plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth, cap);
+                probe.MAXS = PL.test.MAXS;
+                probe.tmax = std::max(1, PL.test.tmax);
+                smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
               }
             }
-            if (cap > 0) {
-              PL.test = HostPlan();
-              plan_test_side_par(St, ord_t, tc.FM, row0, PL.test, nth, cap);
-              probe.MAXS = PL.test.MAXS;
-              probe.tmax = std::max(1, PL.test.tmax);
-              smem = far_smem_bytes(precision, K.op_kind, K.qt, K.qb, probe);
-            }
+            occ = 0;
+            if (smem > (size_t)smem_max || far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ)) occ = 0;
           }
-          occ = 0;
-          if (smem > (size_t)smem_max || far_persistent_occupancy(precision, K.op_kind, gen, smem, &occ)) occ = 0;
+          if (occ >= 1) {
+            PL.cfg_id = id;
+            PL.tc = {tc.FM, tc.FN, sc};
+            PL.smem = smem;
+          } else if (id != prefs.back()) {
+            break;
+          }
         }
-        if (occ >= 1) {
-          PL.cfg_id = id;
-          PL.tc = {tc.FM, tc.FN, sc};
-          PL.smem = smem;
-        } else if (id != prefs.back()) {
-          break;
+        if (PL.cfg_id >= 0) break;
+      }
+    };
+    plan_tiles();
+    if (PL.cfg_id >= 0 && two_phase) {
+      // a panel is at least one tile wide: where that is too much, the fused tiles compute the pairs themselves
+      PL.rows = PL.test.tb_tris;
+      std::sort(PL.rows.begin(), PL.rows.end());
+      PL.rows.erase(std::unique(PL.rows.begin(), PL.rows.end()), PL.rows.end());
+      int64_t widest = 1;
+      for (const HostPlan& P : PL.trial) widest = std::max<int64_t>(widest, P.nmax);
+      if (144 * widest * (int64_t)PL.rows.size() > panel_bytes) {
+        Plans narrow = std::move(PL);
+        PL = Plans();
+        two_phase = false;
+        choose_prefs();
+        plan_tiles();
+        if (PL.cfg_id < 0) {  // (functions of many triangles fit the gather only)
+          PL = std::move(narrow);
+          two_phase = true;
         }
       }
-      if (PL.cfg_id >= 0) break;
     }
     if (PL.cfg_id < 0) {
       char buf[160];
@@ -1130,9 +1182,6 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
                smem_max, smem);
       PL.err = buf;
     } else if (two_phase) {
-      PL.rows = PL.test.tb_tris;
-      std::sort(PL.rows.begin(), PL.rows.end());
-      PL.rows.erase(std::unique(PL.rows.begin(), PL.rows.end()), PL.rows.end());
       const int64_t cap = std::max<int64_t>(1, panel_bytes / (144 * std::max<int64_t>(1, (int64_t)PL.rows.size())));
       PL.panels.assign(nblocks, {});
       PL.pcols.assign(nblocks, {});
@@ -1359,6 +1408,21 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
 
   // 4. the host plan (joined here) and the test-side tables, uploaded once
   planner.join();
+  if (PL.cfg_id >= 0 && two_phase) {
+    // one panel workspace per compute stream in use (sized to the largest panel)
+    for (int k = 0; k < npanels && two_phase; ++k) {
+      int64_t ncol = 1;
+      for (int b = k; b < nblocks; b += 2)
+        for (const Panel& q : PL.panels[b]) ncol = std::max<int64_t>(ncol, q.ncol);
+      if (h->panel_L[k].ensure(144 * (size_t)ncol * std::max<size_t>(1, PL.rows.size()))) two_phase = false;
+    }
+    if (!two_phase) {  // the memory went elsewhere meanwhile: the fused tiles need none
+      cudaGetLastError();
+      for (DevBuf& w : h->panel_L) w.release();
+      choose_prefs();
+      plan_all();
+    }
+  }
   hm[3] = host_ms();
   st.ms_plan = PL.ms;
   if (PL.cfg_id < 0) {
@@ -1392,15 +1456,8 @@ int bgb_assemble(bgb_handle* h, const bgb_operator* op, const bgb_space* test, c
     if ((rc = h->prow.ensure(sizeof(int) * std::max(1, test->nt)))) return rc;
     if ((rc = launch_index_of(h->tplan_i.as<int>() + o_rows, nprow, h->prow.as<int>(), test->nt, h->stream_up))) return rc;
     ++launches;
-    // one panel workspace per compute stream in use (sized to the largest panel)
-    for (int k = 0; k < std::min(2, nblocks); ++k) {
-      int64_t ncol = 1;
-      for (int b = k; b < nblocks; b += 2)
-        for (const Panel& q : PL.panels[b]) ncol = std::max<int64_t>(ncol, q.ncol);
-      if ((rc = h->pcol[k].ensure(sizeof(int) * std::max(1, trial->nt))) ||
-          (rc = h->panel_L[k].ensure(144 * (size_t)ncol * std::max(1, nprow))))
-        return rc;
-    }
+    for (int k = 0; k < npanels; ++k)
+      if ((rc = h->pcol[k].ensure(sizeof(int) * std::max(1, trial->nt)))) return rc;
   }
   BGB_CUDA(cudaEventRecord(h->ev_up[bgb_handle::kSlots], h->stream_up));
   int per_sm = 0;

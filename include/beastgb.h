@@ -105,7 +105,10 @@ typedef struct {
  * GB300 needs).  Zero-initialised fields take defaults. */
 typedef struct {
   int32_t device;              /* CUDA device ordinal */
-  int64_t hbm_budget_bytes;    /* 0 = 90% of free device memory; bounds row blocks */
+  int64_t hbm_budget_bytes;    /* 0 = 90% of free device memory; bounds the staging of host outputs and, beside it,
+                                  the local matrices that an FP64 call keeps per panel of pairs (0: those take up to
+                                  4 GiB, two times that for a host output in blocks, of a quarter of free memory
+                                  each; a call computes its pairs inside the output tiles where no panel fits) */
   int64_t pinned_ring_bytes;   /* each half of the pinned ring that pageable host outputs are
                                   copied through (at least one column of the output); 0 = 512 MiB */
   int32_t tile_config;         /* -1 = first tile shape that fits shared memory, else a tile id (bgb_tile_info) */
@@ -138,6 +141,10 @@ typedef struct bgb_handle bgb_handle;
  * (utils/configuration.jl:29-50, assamble_gpu.jl:25-65). */
 int bgb_create(bgb_handle** out, const bgb_config* cfg);
 int bgb_destroy(bgb_handle* h);
+
+/* Give back the large device buffers that the handle keeps between calls (panels of local matrices, staging of host
+ * outputs, singular pairs' matrices); the next call allocates what it needs again. */
+int bgb_trim(bgb_handle* h);
 
 /* Assemble rows [row0, row0 + nrows) of Z (test functions) against all trial functions.
  * nrows < 0 means all rows.  Output is column-major (Julia layout): element (m, n) at
