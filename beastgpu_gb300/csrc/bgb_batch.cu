@@ -485,10 +485,14 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
   const bool mixed = precision == BGB_PREC_MIXED;
   const int* prefs = lagrange ? (mixed ? kPrefLagrange : kPrefLagrangeFp64) : mixed ? kPrefMixed : kPrefFp64;
   const int nprefs = lagrange ? (mixed ? kNumPrefLagrange : kNumPrefLagrangeFp64) : mixed ? kNumPrefMixed : kNumPrefFp64;
-  std::vector<int> cands;
-  if (h->cfg.tile_config >= 0) cands.push_back(h->cfg.tile_config);
+  std::vector<int> cands, tuned;  // tuned: what the autotuner times
+  if (h->cfg.tile_config >= 0) tuned = cands = {h->cfg.tile_config};
   else {
-    cands.assign(prefs, prefs + nprefs);
+    tuned = cands = std::vector<int>(prefs, prefs + nprefs);
+    // shapes that are the fastest of no single matrix, but of some batches (24 ellipsoids, hats of 42 - 2,562 functions:
+    // 32 x 32 x 4 19.0 ms, 48 x 48 x 5 18.2, the shapes of the single matrices 19.5)
+    if (mixed)
+      for (int c : lagrange ? std::vector<int>{6, 13, 15, 5, 19} : std::vector<int>{4, 8, 1, 5, 6}) tuned.push_back(c);
     if (mixed)  // (the FP64 lists are not in order of width)
       narrow_for_size(cands, far_target_ctas_per_sm(precision) * (int64_t)h->num_sms, [&](const TileCfg& c) {
         int64_t t = 0;
@@ -497,12 +501,13 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
         return t;
       });
   }
-  const bool autotune = (flags & 1) && cands.size() > 1;
+  const bool autotune = (flags & 1) && tuned.size() > 1;
+  const int last = cands.back();
   // first full run (records + singular) with the first fitting candidate
   int first = -1;
   size_t smem = 0;
   for (int c : cands) {
-    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, 1, c == cands.back(), &smem))) return fail(rc);
+    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, 1, c == last, &smem))) return fail(rc);
     if (smem <= (size_t)smem_max) { first = c; break; }
   }
   if (first < 0) { set_error("bgb_batch_create: no tile shape fits shared memory"); return fail(BGB_ERR_CAPACITY); }
@@ -526,9 +531,9 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
   if (autotune) {
     // time the far launch alone for every fitting (shape, schedule)
     best_ms = 1e30;
-    for (int c : cands)
+    for (int c : tuned)
       for (int sched = 0; sched < 2; ++sched) {
-        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, c == cands.back(), &smem))) return fail(rc);
+        if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, c, sched, c == last, &smem))) return fail(rc);
         if (smem > (size_t)smem_max) continue;
         if ((rc = set_cfg(c, smem))) return fail(rc);
         if ((rc = enqueue_device_work(B, st, true))) return fail(rc);  // warm-up
@@ -539,7 +544,7 @@ int bgb_batch_create(bgb_handle* h, int32_t n, const bgb_problem* problems, int3
         const double ms = event_ms(B->ev[0], B->ev[1]);
         if (ms < best_ms) { best_ms = ms; best_cfg = c; best_sched = sched; }
       }
-    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, best_cfg, best_sched, best_cfg == cands.back(), &smem)) ||
+    if ((rc = build_plans(B, problems, St, Sb, cent_t, cent_b, tbase, bbase, best_cfg, best_sched, best_cfg == last, &smem)) ||
         (rc = set_cfg(best_cfg, smem)))
       return fail(rc);
   }
