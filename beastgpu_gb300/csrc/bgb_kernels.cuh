@@ -76,6 +76,7 @@ struct DfTables {
   DfTrig trig;
   dfl gx[4][BGB_MAX_SS], gw[4][BGB_MAX_SS];
   df2 ser[4][4][BGB_SS_SERIES];  // (cosine, sine) coefficients
+  df2 hat[4][2][BGB_SS_SERIES];  // the hats' of lower degree, with powers of 1 - xi
 };
 void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M);
 // Per-triangle double-float geometry: vertices (df), area and 1 / area (df).

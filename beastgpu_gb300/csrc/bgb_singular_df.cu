@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kWarps = 8;
 
-// Moments (complex): hats 9 (p_a q_b, p = (1, alpha xi, beta xi)); EFIE S, Px, Py, P0; MFIE sum H X x Y, sum H (X - Y).
+// Moments (complex): hats 9 (their products); EFIE S, Px, Py, P0; MFIE sum H X x Y, sum H (X - Y).
 template <int OP>
 struct DfMoments {
   static constexpr int N = OP == BGB_OP_HELMHOLTZ3D_SL ? 9 : (OP == BGB_OP_MAXWELL3D_SL ? 8 : 6);
@@ -73,23 +73,10 @@ __device__ __forceinline__ double2 df_entry(const OpDf& op, const GeoDf& A, cons
   const dfl ar = gdf(op.alpha[0]), ai = gdf(op.alpha[1]);
   dfl tr{0.f, 0.f}, ti{0.f, 0.f};
   if (OP == BGB_OP_HELMHOLTZ3D_SL) {
-    // hats of the reordered vertices: 1 - p1, p2, p1 - p2
-    const int H[3][3] = {{1, -1, 0}, {0, 0, 1}, {0, 1, -1}};
     const int r = I[0] == i + 1 ? 0 : (I[1] == i + 1 ? 1 : 2), c = J[0] == j + 1 ? 0 : (J[1] == j + 1 ? 1 : 2);
-    for (int a = 0; a < 3; ++a)
-      for (int b = 0; b < 3; ++b) {
-        const int t = H[r][a] * H[c][b];
-        if (t > 0) {
-          tr = df_add(tr, m(2 * (a * 3 + b)));
-          ti = df_add(ti, m(2 * (a * 3 + b) + 1));
-        } else if (t < 0) {
-          tr = df_sub(tr, m(2 * (a * 3 + b)));
-          ti = df_sub(ti, m(2 * (a * 3 + b) + 1));
-        }
-      }
     const dfl w = df_mul(df_mulf(df_mul(gdf(A.area), gdf(B.area)), 4.f), inv4pi);
-    tr = df_mul(tr, w);
-    ti = df_mul(ti, w);
+    tr = df_mul(m(2 * (3 * r + c)), w);
+    ti = df_mul(m(2 * (3 * r + c) + 1), w);
     const dfl Lr = df_sub(df_mul(ar, tr), df_mul(ai, ti)), Li = df_add(df_mul(ar, ti), df_mul(ai, tr));
     return make_double2(df_to_double(Lr), df_to_double(Li));
   }
@@ -143,6 +130,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
                                                                 const int* __restrict__ perm,
                                                                 const int64_t* __restrict__ range) {
   constexpr int NA = DfMoments<OP>::N, NV = 2 * NA, M0 = DfMoments<OP>::M0;
+  constexpr bool kHat = OP == BGB_OP_HELMHOLTZ3D_SL;
   constexpr int NS = NV <= 16 ? 16 : 32;  // rows of the reduction (two lanes per row when 16 suffice)
   __shared__ float4 trig[128];
   __shared__ float2 part[kWarps][NV][33];
@@ -218,28 +206,28 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
       const dfl r2 = df_dot(d, d);
       const dfl rinv = df_rsqrt_step(r2);
       const dfl th = df_mul(kd, df_mulx(r2, rinv));
-      df2 T[3];  // (C, S) of T_m = C - i S, m = M0 .. M0 + 2
+      df2 T[3];  // (C, S) of T_m = C - i S, m = M0 .. M0 + 2; hats: T_m with (1 - xi)^2 / xi^2, (1 - xi) / xi, 1 in m = 2
       if (nj > 0) {
         const dfl th2s = df_mul(th, th);
         const df2 th2 = df2_both(th2s);
-        const df2(*__restrict__ ser)[BGB_SS_SERIES] = M.ser[cls];
+        auto ser = [&](int q, int k) { return kHat && q < 2 ? M.hat[cls][q][k] : M.ser[cls][q + 1 + M0][k]; };
         unsigned long long t[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) t[q] = 0ull;
         for (int k = nj - 1; k >= nd; --k) {
 #pragma unroll
-          for (int q = 0; q < 3; ++q) t[q] = fma2(t[q], th2.hi, ser[q + 1 + M0][k].hi);
+          for (int q = 0; q < 3; ++q) t[q] = fma2(t[q], th2.hi, ser(q, k).hi);
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) T[q] = df2{t[q], 0ull};
         for (int k = nd - 1; k >= 1; --k) {
 #pragma unroll
-          for (int q = 0; q < 3; ++q) T[q] = df2_fma_big(T[q], th2, ser[q + 1 + M0][k]);
+          for (int q = 0; q < 3; ++q) T[q] = df2_fma_big(T[q], th2, ser(q, k));
         }
         const df2 one_th = df2_of(dfl{1.f, 0.f}, th);
 #pragma unroll
         for (int q = 0; q < 3; ++q)  // the first two terms may be of either order
-          T[q] = df2_mul(df2_macc(ser[q + 1 + M0][0], T[q], th2), one_th);
+          T[q] = df2_mul(df2_macc(ser(q, 0), T[q], th2), one_th);
       } else {
 #pragma unroll
         for (int q = 0; q < 3; ++q) T[q] = df2{0ull, 0ull};
@@ -250,9 +238,12 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
           const df2 e2 = df2_of(cs, sn);
           dfl w = df_mul(M.gw[cls][l], xi);
           if (M0 == 0) w = df_mul(w, xi);
+          const dfl om_xi = df_sub(dfl{1.f, 0.f}, xi);
 #pragma unroll
           for (int q = 0; q < 3; ++q) {
-            T[q] = df2_macc(T[q], df2_both(w), e2);
+            dfl wq = w;
+            for (int z = q; kHat && z < 2; ++z) wq = df_mul(wq, om_xi);
+            T[q] = df2_macc(T[q], df2_both(wq), e2);
             w = df_mul(w, xi);
           }
         }
@@ -287,20 +278,22 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_singular_df(OpDf op1, const 
         acc[7] = df2_macc(acc[7], gg, T[0]);
       } else {
         const df2 gg = df2_of(g, df_neg(g));
-        df2 t[3];  // kernel sums of degree 0, 1, 2
+        df2 t[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) t[q] = df2_mul(gg, T[q]);
-        const dfl p[3] = {dfl{1.f, 0.f}, al, be}, q[3] = {dfl{1.f, 0.f}, ga, de};
-        acc[0] = df2_add(acc[0], t[0]);
+        // hats of the reordered vertices: (1 - xi) + (1 - alpha) xi, beta xi, (alpha - beta) xi, every term positive:
+        // summed as the moments of 1, alpha xi, beta xi, a matrix loses a factor of 2 (1.0e-14 -> 2.0e-14 of its norm)
+        const dfl one{1.f, 0.f}, a0 = df_sub(one, al), c0 = df_sub(one, ga);
+        const dfl a[2] = {be, df_sub(al, be)}, c[2] = {de, df_sub(ga, de)};
+        const df2 v = df2_macc(t[1], t[2], df2_both(a0)), w = df2_macc(t[1], t[2], df2_both(c0));
+        acc[0] = df2_add(acc[0], df2_macc(df2_macc(t[0], t[1], df2_both(a0)), v, df2_both(c0)));
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int i = 0; i < 2; ++i) {
+          acc[1 + i] = df2_macc(acc[1 + i], v, df2_both(c[i]));
+          acc[3 + 3 * i] = df2_macc(acc[3 + 3 * i], w, df2_both(a[i]));
 #pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            if (a + b == 0) continue;
-            const int deg = (a > 0) + (b > 0);
-            const dfl pq = a == 0 ? q[b] : (b == 0 ? p[a] : df_mul(p[a], q[b]));
-            acc[3 * a + b] = df2_macc(acc[3 * a + b], t[deg], df2_both(pq));
-          }
+          for (int j = 0; j < 2; ++j) acc[4 + 3 * i + j] = df2_macc(acc[4 + 3 * i + j], t[2], df2_both(df_mul(a[i], c[j])));
+        }
       }
     }
     // reduction: lane v (and v + 16 when 16 rows suffice) sums row v
@@ -393,13 +386,28 @@ void build_df_tables(const QuadSel& qs, std::vector<float>& buf, DfTables& M) {
       M.gx[cls][l] = df(T.gx[cls][l]);
       M.gw[cls][l] = df(T.gw[cls][l]);
     }
+    auto put = [&](double cos_k, double sin_k, df2& out) {
+      const dfl c = df(cos_k), s = df(sin_k);
+      const float hi[2] = {c.hi, s.hi}, lo[2] = {c.lo, s.lo};
+      std::memcpy(&out.hi, hi, sizeof(hi));
+      std::memcpy(&out.lo, lo, sizeof(lo));
+    };
     for (int m = 0; m < 4; ++m)
-      for (int k = 0; k < BGB_SS_SERIES; ++k) {
-        const dfl c = df(T.ser[cls][m][2 * k]), s = df(T.ser[cls][m][2 * k + 1]);
-        const float hi[2] = {c.hi, s.hi}, lo[2] = {c.lo, s.lo};
-        std::memcpy(&M.ser[cls][m][k].hi, hi, sizeof(hi));
-        std::memcpy(&M.ser[cls][m][k].lo, lo, sizeof(lo));
+      for (int k = 0; k < BGB_SS_SERIES; ++k) put(T.ser[cls][m][2 * k], T.ser[cls][m][2 * k + 1], M.ser[cls][m][k]);
+    // as T_0 and T_1, with (1 - xi)^2 in the place of 1 and (1 - xi) in the place of xi
+    for (int q = 0; q < 2; ++q) {
+      long double f = 1.0L, term[2 * BGB_SS_SERIES];
+      for (int k = 0; k < 2 * BGB_SS_SERIES; ++k) {
+        if (k > 1) f *= k;
+        long double s = 0.0L;
+        for (int l = 0; l < T.n[cls]; ++l) {
+          const long double xi = T.gx[cls][l];
+          s += T.gw[cls][l] * powl(xi, 2 + q + k) * powl(1.0L - xi, 2 - q);
+        }
+        term[k] = ((k >> 1) & 1 ? -1 : 1) * s / f;
       }
+      for (int k = 0; k < BGB_SS_SERIES; ++k) put((double)term[2 * k], (double)term[2 * k + 1], M.hat[cls][q][k]);
+    }
   }
   align4();
   M.trig_off = (int)buf.size();
