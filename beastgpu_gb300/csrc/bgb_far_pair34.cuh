@@ -386,16 +386,6 @@ __device__ __forceinline__ void far_pair34_mixed(const FarScalars& K, const floa
 }
 
 // ---- plain FP64 -----------------------------------------------------------------------------------
-// 1 / sqrt(x) for a positive normal x: the hardware estimate (more than 20 bits, its square exact in
-// FP64) and one cubic Newton (Householder) step, y (1 + e (1/2 + 3 e / 8)) with e = 1 - x y^2; what is
-// dropped is below 2^-60.
-__device__ __forceinline__ double rsqrt_newton(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = __fma_rn(-x, __dmul_rn(y, y), 1.0);
-  return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
-}
-
 // The phase is k R = k R0 + k (R - R0) with R0 the centroid distance: exp(-i k R0) is a factor of the whole
 // local matrix, and cos / sin of the small k (R - R0) come from tay_n terms of their series for all
 // four trial points together (sincos of k R where the series would be long).

@@ -44,13 +44,6 @@ struct SsMoments {
   static constexpr int NT = OP == BGB_OP_HELMHOLTZ3D_DL || OP == BGB_OP_HELMHOLTZ3D_DLT ? 4 : 3;
 };
 
-__device__ __forceinline__ double rsqrt_step(double x) {  // as rsqrt_newton in bgb_far_pair34.cuh
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y * y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 __device__ __forceinline__ void sub3(const double* a, const double* b, double c[3]) {
   c[0] = a[0] - b[0];
   c[1] = a[1] - b[1];
@@ -192,7 +185,7 @@ __global__ void __launch_bounds__(32 * kWarps, 2) k_ss64(OpParams op1, const OpP
         d[c] = X[c] - Y[c];
       }
       const double r2 = fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]));
-      const double rinv = rsqrt_step(r2);
+      const double rinv = rsqrt_newton(r2);
       const double R = r2 * rinv;
       double C[NT], S[NT];  // T_m = C - i S, m = M0 ..
       if (nj > 0) {
