@@ -671,10 +671,11 @@ __device__ __noinline__ void far_pair34_fp64_close(const FarConst& K, const doub
 #pragma unroll
   for (int k = 0; k < 9; ++k) L[k] = t[k];
 }
-// True below R0 = 3.3 - 3.5 times the larger of the point radii (beyond, R > 0.38 R0): triangles next to each other.
-// By exponents (n < 10.7 - 12 times the radius squared), beside the FP64 pipe.  Pairs without common vertices reach it
-// on no mesh of even triangles; on the box of right triangles 3.7 would take in four per triangle, whose second pass
-// cost the 8 x 8 box 26 of 590 us.
+// True below R0 = 2.3 - 2.45 times the larger of the point radii, by exponents (n < 5.3 - 6 times the radius squared),
+// beside the FP64 pipe.  Beyond, points may still be as close as R0 / 6 where triangles of about one size overlap;
+// overlapping plates (8 x 8 on 8 x 8, 12 x 12) are within 1e-15 of a pair's matrix there, as below 3.4 radii before.
+// Triangles that do not overlap come this near on stretched meshes only; 3.4 radii took in pairs of every plate and box,
+// 25 of 700 us of a small call.
 __device__ __forceinline__ bool far_pair34_is_close(const double* __restrict__ a, const double* __restrict__ b) {
   double n = 0.0;
 #pragma unroll
@@ -682,7 +683,7 @@ __device__ __forceinline__ bool far_pair34_is_close(const double* __restrict__ a
   int top = max(__double2hiint(a[12]), __double2hiint(b[12]));
 #pragma unroll
   for (int i = 1; i < 3; ++i) top = max(top, max(__double2hiint(a[12 + i]), __double2hiint(b[12 + i])));
-  return __double2hiint(n) < top + 0x00380000;
+  return __double2hiint(n) < top + 0x00280000;
 }
 
 template <class P, int OP, int QT, int QB>
@@ -1132,7 +1133,8 @@ __global__ void __launch_bounds__(kPairSide * kPairSide, 2) k_pair64(const FarCo
   constexpr int RT = PFp64::rec<QT>(), RB = PFp64::rec<QB>();
   __shared__ FarConst K;
   __shared__ double sT[kPairSide * RT], sB[kPairSide * RB];
-  __shared__ int stop;
+  __shared__ int stop, nclose;
+  __shared__ unsigned char close[kPairSide * kPairSide];
   const int tid = threadIdx.x;
   const int r0 = blockIdx.y * kPairSide, c0 = blockIdx.x * kPairSide;
   const int nr = min(kPairSide, nrows - r0), nc = min(kPairSide, ncols - c0);
@@ -1145,25 +1147,40 @@ __global__ void __launch_bounds__(kPairSide * kPairSide, 2) k_pair64(const FarCo
     const int r = i / RB;
     sB[i] = rec_b[(int64_t)cols[c0 + r] * RB + (i - r * RB)];
   }
-  if (tid == 0) stop = abort_flag && *abort_flag;
+  if (tid == 0) {
+    stop = abort_flag && *abort_flag;
+    nclose = 0;
+  }
   __syncthreads();
   if (stop) return;
   const int ti = tid / kPairSide, si = tid - ti * kPairSide;
-  if (ti >= nr || si >= nc) return;
-  double2* o = ws + ((int64_t)(r0 + ti) * ncols + c0 + si) * 9;
+  auto out = [&](int t, int s) { return ws + ((int64_t)(r0 + t) * ncols + c0 + s) * 9; };
+  bool on = ti < nr && si < nc;
   const double *a = sT + ti * RT, *b = sB + si * RB;
-  double2 L[9];
   if constexpr (QT == 3 && QB == 4) {
-    if (far_pair34_is_close(a, b)) {  // singular and near pairs, whose matrices are placed afterwards, and a few others
-      if (find_sigma(sing_off, sing_sigma, rows[r0 + ti], cols[c0 + si]) < 0) far_pair34_fp64_close<OP>(K, a, b, o);
-      return;
+    // singular and near pairs, whose matrices are placed afterwards, and a few others: those are listed and computed
+    // by full warps at the end (a second pass of every warp that holds one: ellipsoid of 320 long triangles, far
+    // stage 156 -> 238 us)
+    if (on && far_pair34_is_close(a, b)) {
+      on = false;
+      if (find_sigma(sing_off, sing_sigma, rows[r0 + ti], cols[c0 + si]) < 0) close[atomicAdd(&nclose, 1)] = (unsigned char)tid;
     }
-    far_pair34_fp64<OP, false>(far_scalars(K), K.tay_s, K.tay_c, a, b, L);
-  } else {
-    far_pair<PFp64, OP, QT, QB>(far_scalars(K), K, a, b, L);
   }
+  if (on) {
+    double2 L[9];
+    if constexpr (QT == 3 && QB == 4) far_pair34_fp64<OP, false>(far_scalars(K), K.tay_s, K.tay_c, a, b, L);
+    else far_pair<PFp64, OP, QT, QB>(far_scalars(K), K, a, b, L);
+    double2* o = out(ti, si);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) o[k] = L[k];
+    for (int k = 0; k < 9; ++k) o[k] = L[k];
+  }
+  if constexpr (QT == 3 && QB == 4) {
+    __syncthreads();
+    if (tid < nclose) {  // at most one per thread
+      const int t = close[tid] / kPairSide, s = close[tid] % kPairSide;
+      far_pair34_fp64_close<OP>(K, sT + t * RT, sB + s * RB, out(t, s));
+    }
+  }
 }
 
 template <int OP, int QT, int QB>
