@@ -332,8 +332,8 @@ const int kNumPrefLagrange = sizeof(kPrefLagrange) / sizeof(int);
 // from full chunks: d = 24 cube 48 x 48 x 4 1,537 ms, 40 x 40 x 4 1,629 ms, 32 x 40 x 5 1,693 ms.
 const int kPrefLagrangeFp64[] = {9, 15, 18, 6, 13, 5, 7};
 const int kNumPrefLagrangeFp64 = sizeof(kPrefLagrangeFp64) / sizeof(int);
-// Output tiles of the FP64 gather (single assemblies; widest first): every pair is computed once
-// whatever the tile, so their width only trades L2 reads at the rims against CTAs per SM.
+// Output tiles of the FP64 gather (single assemblies; widest first): a panel's pairs are computed once (its rim again
+// in the next panel: 4% of the cube of 6,912 triangles) whatever the tile, so their width only trades L2 reads at the rims against CTAs per SM.
 const int kPrefGather[] = {19, 20, 21, 22};
 const int kNumPrefGather = sizeof(kPrefGather) / sizeof(int);
 const int kPrefGatherLagrange[] = {18, 21, 22};

@@ -14,7 +14,7 @@
 //
 // The tile kernel serves the mixed path and FP64 batches; single FP64 assemblies compute the local matrices of
 // panels of pairs (k_pair64, below) and gather them in a second kernel: at 1/62 of the FP32 rate the halo's
-// FP64 work costs more than writing the matrices once (level-4 EFIE: 84.3 -> 46 ms).
+// FP64 work costs more than writing the matrices once (level-4 EFIE: 84.3 -> 46 ms when it was split, 33 ms now).
 //
 // Roofline: compute-bound on FP32 issue (mixed) or FP64 issue (plain), plus MUFU (rsqrt, rcp, sin, cos: 4 per
 // point pair).  The default rule pair (3 x 4 points) has its own pair code (bgb_far_pair34.cuh); the other rules
@@ -1334,7 +1334,7 @@ int launch_diag_t(const FarConst& K, const void* rt, const void* rb, const int* 
   return e == cudaSuccess ? 0 : cuda_fail(e, "k_far_pairs_diag launch");
 }
 
-// Instances live in bgb_far_{mixed,fp64}_op{0,1,2}.cu.
+// Instances live in bgb_far_{mixed,fp64}_op{0,1,2,3,4,5}.cu.
 #define BGB_FAR_EXTERN(P, OP)                                                                                   \
   extern template int launch_diag_t<P, OP, 3, 4>(const FarConst&, const void*, const void*, const int*,        \
                                                  const int*, int64_t, double2*, cudaStream_t);                \

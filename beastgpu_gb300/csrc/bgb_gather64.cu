@@ -6,7 +6,7 @@
 // pairs, and k_gather64 adds them into the output entries.  The tiles of the fused kernel compute the
 // pairs at their rims again (1.5x the pairs for RWG functions in 64-wide tiles, 1.7x for hats in 48-wide
 // ones), which on an FP64 pipe at 1/62 of the FP32 rate costs far more than the workspace's traffic:
-// 144 B written and ~1.6 x 144 B read per pair, against the ~35 KB that HBM could move in the time the
+// 144 B written and ~1.6 x 144 B read per pair, against the ~8 KB that HBM could move in the ~1.1 ns that the
 // pipe needs for one pair.
 //
 // k_gather64: one CTA per output tile.  The local matrices of the next chunk of trial triangles are

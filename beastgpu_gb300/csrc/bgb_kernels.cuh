@@ -189,7 +189,8 @@ int far_generic_q(int qt, int qb);  // 1 when the (qt, qb) pair uses the generic
 int rec_stride(int precision, int q, int generic);
 
 // Plain FP64 far stage of a single assembly: the local matrices of a panel rows x cols (triangle lists,
-// device; those of the non-far pairs of the CSR sing_off, sing_sigma may stay unwritten), then the output tiles [bn0 * n_tblocks, + ntiles) from them.
+// device; those of the non-far pairs of the CSR sing_off, sing_sigma may stay unwritten), then the output tiles
+// [bn0 * n_tblocks, + ntiles) from them.
 int launch_pair64(int op_kind, int generic, const FarConst* K, const void* rec_t, const void* rec_b, const int* rows,
                   int nrows, const int* cols, int ncols, const int64_t* sing_off, const int* sing_sigma, double2* ws,
                   const volatile int* abort_flag, cudaStream_t st);

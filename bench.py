@@ -53,9 +53,9 @@ UNIT = "pair-interactions/s"
 LEVEL, KWAVE = 5, 2 * np.pi * 4
 ERR_ROWS, ERR_SEED = 1000, 0
 # DRAM bytes (read + write) of one far-kernel launch per triangle pair, from the ncu capture of
-# the level-4 case (0.462 GB for 5120^2 pairs); the traffic is the output written once, so it
+# the level-4 case (0.466 GB for 5120^2 pairs); the traffic is the output written once, so it
 # scales with the pairs.
-FAR_DRAM_BYTES_PER_PAIR = 0.462e9 / (5120 * 5120)
+FAR_DRAM_BYTES_PER_PAIR = 0.466e9 / (5120 * 5120)
 
 
 def workload():
@@ -214,9 +214,11 @@ CURVE_N, CURVE_K, CURVE_ROWS = 16384, 2 * np.pi * 100, 64
 # complex double local matrix written once).
 CURVE_FP64_FLOPS_PER_POINT_PAIR = 239.5
 CURVE_DRAM_BYTES_PER_PAIR = 1.040e9 / (4096 * 4096)
-# The same for the mixed far kernel: FP32 flops (2 FFMA + FADD + FMUL) per far point pair and DRAM
-# bytes per segment pair (the local matrix as 2x2 complex float), ncu on the 4,096-segment case.
-CURVE_MIXED_FP32_FLOPS_PER_POINT_PAIR = 97.2
+# The same for the mixed far kernel: FP32 flops per far point pair, counted in the source's loop over two trial points
+# (FMA = 2: 42 for distance and phase, 78 for the Hankel function, 16 for the four sums, halved; the transcendentals
+# and what is done once per test point or per pair not counted), and DRAM bytes per segment pair (the local matrix as
+# 2x2 complex float), ncu on the 4,096-segment case.
+CURVE_MIXED_FP32_FLOPS_PER_POINT_PAIR = 68.0
 CURVE_MIXED_DRAM_BYTES_PER_PAIR = 0.4755e9 / (4096 * 4096)
 
 
@@ -327,9 +329,8 @@ def run_curve(args):
             "unit": "TFLOP/s", "frac": tf / fp32_peak, "traffic": CURVE_MIXED_DRAM_BYTES_PER_PAIR * pairs,
             "traffic_source": "ncu dram__bytes of the 4,096-segment launch scaled by pairs (x16)",
             "peak_source": "measured live by bgb_measure_issue_peaks (FFMA chains)",
-            "flop_convention": f"{CURVE_MIXED_FP32_FLOPS_PER_POINT_PAIR} FP32 flops per far point pair (ncu count: "
-                               "2 FFMA + FADD + FMUL, per-pair double-float setup included)",
-            "note": "issue-bound: 89% of issue slots (FMA 46%, ALU 45%, MUFU 19% of peak), ncu on 4,096 segments"}
+            "flop_convention": f"{CURVE_MIXED_FP32_FLOPS_PER_POINT_PAIR} FP32 flops per far point pair (counted in the "
+                               "source's loop over the points, FMA = 2; setup per pair and transcendentals not counted)"}
     tf64 = point_pairs * CURVE_FP64_FLOPS_PER_POINT_PAIR / (kd["far_and_gather"] * 1e-3) / 1e12
     roof64 = {"kernel": "curve::k_curve_far<HS> (+ gather)", "bound": "fp64", "achieved": tf64, "peak": fp64_peak,
               "unit": "TFLOP/s", "frac": tf64 / fp64_peak,
@@ -864,7 +865,7 @@ def main():
     far_tf = flops_far / (far_ms * 1e-3) / 1e12
     sing_tf = flops_sing / (sing_ms * 1e-3) / 1e12
     if far_ms >= sing_ms:
-        roof = {"kernel": "k_far_tiles<PMixed, EFIE, 3, 4>", "bound": "fp32", "achieved": far_tf, "peak": fp32_peak,
+        roof = {"kernel": "k_far_persistent<PMixed, EFIE, 3, 4>", "bound": "fp32", "achieved": far_tf, "peak": fp32_peak,
                 "unit": "TFLOP/s", "frac": far_tf / fp32_peak}
     else:
         roof = {"kernel": "k_singular (FP64 Sauter-Schwab)", "bound": "fp64", "achieved": sing_tf, "peak": fp64_peak,
@@ -880,7 +881,8 @@ def main():
                  "hbm_gbs_far": out_gb / (far_ms * 1e-3), "hbm_frac_far_of_measured": (out_gb / (far_ms * 1e-3)) / hbm_peak
                  if hbm_peak else None,
                  "peak_source": "measured live by bgb_measure_issue_peaks (FMA chains)",
-                 "flop_convention": "per point pair: 15 (kernel) + 108 (EFIE 9-entry accumulation), FMA = 2",
+                 "flop_convention": "per point pair: 15 (kernel) + 108 (EFIE 9-entry accumulation from moments; the 3 x 4 code "
+                                    "forms the same sums with fewer operations), FMA = 2",
                  "kernels_ms": {"far": far_ms, "singular": sing_ms,
                                 "classify": float(np.mean([s["ms_classify"] for s in st_mixed]))},
                  "far_tflops": far_tf, "singular_tflops": sing_tf,
